@@ -104,6 +104,8 @@ struct Workspace {
     int* assoc_idx = nullptr;
     float* assoc_dist = nullptr;
     int* rho = nullptr;             // (h_max) niche counts of prior fronts
+    int* niche_last = nullptr;      // (h_max + 1) last-front members per direction, after rho
+    int* niche_start = nullptr;     // (h_max + 1) first position of each direction, after niche_last
     int* sel_vals[2] = {};          // niching sort values
     int* rank = nullptr;
     int* selected = nullptr;        // (n_max) selection before ordering

@@ -30,6 +30,7 @@
 #include <cooperative_groups.h>
 
 #include "internal.cuh"
+#include "niche_select.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -564,6 +565,57 @@ nich_cluster(const int* __restrict__ idx, const float* __restrict__ dist, const 
     nc_niching<false>(sm, cluster, c, idx, dist, np, nl, nrem, rho, H, seed, offset, nds_gidx, selected);
 }
 
+// Niche selection and the ascending survivor list of one generation: the
+// direction buckets of niche_select.cuh, else the three sorts above.
+union NcSelectShared {
+    NcShared sorts;
+    NicheShared<kNcThreads> buckets;
+};
+
+__global__ void __launch_bounds__(kNcThreads, 1)
+nich_select(const int* __restrict__ idx, const float* __restrict__ dist, const int* __restrict__ sizes, NicheScratch S,
+            int H, uint64_t seed, unsigned long long* __restrict__ offset, const int* __restrict__ nds_gidx,
+            int* __restrict__ selected, int n_mix, int N, int* __restrict__ survivors, int* __restrict__ status)
+{
+    extern __shared__ __align__(16) unsigned char nc_raw[];
+    NcSelectShared& sm = *reinterpret_cast<NcSelectShared*>(nc_raw);
+    NicheCluster grp{cg::this_cluster()};
+    const int c = grp.rank();
+    const int np = sizes[0], nl = sizes[1], nrem = sizes[2];
+    // every branch below is uniform over the cluster
+    if (nl > grp.count() * kNcSlice) {  // excluded by the host; reported, never indexed
+        if (c == 0 && threadIdx.x == 0) atomicExch(status, kDevNichingSize);
+        return;
+    }
+    const unsigned long long off = *offset;
+    if (niche_buckets<kNcThreads>(grp, sm.buckets, S, idx, dist, nds_gidx, np, nl, nrem, H, seed, off, n_mix)) {
+        if (c == 0 && threadIdx.x == 0) *offset = off + 2ull * (unsigned long long)nl;
+    } else {
+        if (nl > kNcSlice)
+            nc_niching<false>(sm.sorts, grp.g, c, idx, dist, np, nl, nrem, S.rho, H, seed, offset, nds_gidx, selected);
+        else if (c == 0)
+            nc_niching<true>(sm.sorts, grp.g, 0, idx, dist, np, nl, nrem, S.rho, H, seed, offset, nds_gidx, selected);
+        grp.sync();  // the selection is complete
+        const int take = min(nrem, nl);
+        for (int i = c * kNcThreads + (int)threadIdx.x; i < take; i += grp.count() * kNcThreads)
+            niche_mark(S.mask, __ldcg(selected + np + i));
+        grp.sync();
+    }
+    niche_survivors<kNcThreads>(grp, sm.buckets, S.mask, n_mix, survivors, N);
+}
+
+static_assert(kNsItems * kNcThreads == kNcSlice, "a CTA's members in registers");
+
+// CTAs of a selection: one per 1024 merged points up to 4096 (where one CTA
+// can also run the sorts), else the whole cluster.
+int nich_select_ctas(int n_mix, int H)
+{
+    if (n_mix > kNcSlice || H > 2 * kNcSlice) return kNcCtas;
+    int c = 1;
+    while (c * 1024 < n_mix) c *= 2;
+    return c;
+}
+
 }  // namespace
 
 int niching_cluster_capacity() { return kNcCtas * kNcSlice; }
@@ -598,6 +650,18 @@ bool niching_cluster_ready()
         cudaGetLastError();
         return false;
     }
+    if (clusters < 1) return false;
+    if (cudaFuncSetAttribute(nich_select, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(nich_select, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(NcSelectShared)) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cfg.dynamicSmemBytes = sizeof(NcSelectShared);
+    if (cudaOccupancyMaxActiveClusters(&clusters, (void*)nich_select, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
     state = clusters >= 1 ? 1 : 0;
     return state == 1;
 }
@@ -620,6 +684,28 @@ int launch_niching_cluster(const int* idx, const float* dist, const int* sizes, 
     cfg.numAttrs = 1;
     MOEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, nich_cluster, idx, dist, sizes, rho, H, seed, offset, nds_gidx,
                                      selected, status));
+    return MOEA_OK;
+}
+
+int launch_niche_select(const int* idx, const float* dist, const int* sizes, const NicheScratch& S, int H,
+                        uint64_t seed, unsigned long long* offset, const int* nds_gidx, int* selected, int n_mix, int N,
+                        int* survivors, int* status, cudaStream_t stream)
+{
+    const int ctas = nich_select_ctas(n_mix, H);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kNcThreads);
+    cfg.dynamicSmemBytes = sizeof(NcSelectShared);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    MOEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, nich_select, idx, dist, sizes, S, H, seed, offset, nds_gidx, selected, n_mix,
+                                     N, survivors, status));
     return MOEA_OK;
 }
 

@@ -18,6 +18,7 @@
 #include <cooperative_groups.h>
 
 #include "internal.cuh"
+#include "niche_select.cuh"
 #include "dirtree.h"
 
 namespace cg = cooperative_groups;
@@ -1640,6 +1641,12 @@ int run_order_selection(Workspace& ws, const int* selected, int count, int n_mix
                           stream);
 }
 
+NicheScratch niche_scratch(const Workspace& ws)
+{
+    return NicheScratch{ws.rho, ws.niche_last, ws.niche_start, ws.key64[0], ws.key64[1], ws.sel_vals[0],
+                        reinterpret_cast<uint32_t*>(ws.flags), ws.sizes + 5};
+}
+
 // One NSGA-III environmental selection on the split population.
 int run_nsga3_select(Workspace& ws, const SplitPop& pop, int M, int N, const float* refs, int H,
                      uint64_t seed, float* ideal_last, int* survivors, int* survivor_fronts,
@@ -1657,10 +1664,15 @@ int run_nsga3_select(Workspace& ws, const SplitPop& pop, int M, int N, const flo
     MOEA_TRY(run_associate(ws, ws.nds_objs, ws.n_max, ws.rcp_b, refs, M, ws.sizes + 3, n_mix, H,
                            ws.assoc_idx, ws.assoc_dist, assoc_mode, stream));
     stage_mark("select.associate", stream);
-    MOEA_TRY(run_niching(ws, seed, ws.nds_gidx, ws.assoc_dist, ws.assoc_idx, ws.sizes, H, N,
-                         ws.selected, stream));
+    if (n_mix <= niching_cluster_capacity() && niching_cluster_ready()) {
+        MOEA_TRY(launch_niche_select(ws.assoc_idx, ws.assoc_dist, ws.sizes, niche_scratch(ws), H, seed, ws.offset_dev,
+                                     ws.nds_gidx, ws.selected, n_mix, N, survivors, ws.counters + 6, stream));
+    } else {
+        MOEA_TRY(run_niching(ws, seed, ws.nds_gidx, ws.assoc_dist, ws.assoc_idx, ws.sizes, H, N,
+                             ws.selected, stream));
+        MOEA_TRY(run_order_selection(ws, ws.selected, N, n_mix, survivors, stream));
+    }
     stage_mark("select.niching", stream);
-    MOEA_TRY(run_order_selection(ws, ws.selected, N, n_mix, survivors, stream));
     if (survivor_fronts) {
         gather_fronts<<<ceil_div(N, 256), 256, 0, stream>>>(survivors, N, ws.fronts, survivor_fronts);
         MOEA_CUDA_TRY(cudaGetLastError());
