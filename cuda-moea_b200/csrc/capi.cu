@@ -4,6 +4,7 @@
 #include <new>
 
 #include "internal.cuh"
+#include "niche_select.cuh"
 
 namespace moea {
 
@@ -124,7 +125,7 @@ int workspace_init(Workspace& ws, int device, int n_max, int m_max, int h_max)
     A(ws.norm_part_idx, (size_t)nb * m_max);
     A(ws.rcp_b, m_max); A(ws.extreme, m_max); A(ws.ideal_tmp, m_max);
     A(ws.assoc_best, n); A(ws.assoc_idx, n); A(ws.assoc_dist, n);
-    A(ws.rho, 3 * (size_t)h_max + 2);  // and the two arrays below, h_max + 1 each
+    A(ws.rho, 3 * (size_t)h_max + 2 + kNsHistWords);  // and the three arrays below
     A(ws.sel_vals[0], n); A(ws.sel_vals[1], n);
     A(ws.rank, n); A(ws.selected, n); A(ws.flags, n);
     A(ws.offset_dev, 1);
@@ -134,6 +135,7 @@ int workspace_init(Workspace& ws, int device, int n_max, int m_max, int h_max)
     if (st == MOEA_OK) {
         ws.niche_last = ws.rho + h_max;
         ws.niche_start = ws.niche_last + h_max + 1;
+        ws.niche_hist = ws.niche_start + h_max + 1;
         ws.cub_bytes = cub_temp_bytes_needed(n_max);
         st = dalloc(ws, (char**)&ws.cub_tmp, ws.cub_bytes);
     }

@@ -106,6 +106,7 @@ struct Workspace {
     int* rho = nullptr;             // (h_max) niche counts of prior fronts
     int* niche_last = nullptr;      // (h_max + 1) last-front members per direction, after rho
     int* niche_start = nullptr;     // (h_max + 1) first position of each direction, after niche_last
+    int* niche_hist = nullptr;      // (kNsHistWords) after niche_start
     int* sel_vals[2] = {};          // niching sort values
     int* rank = nullptr;
     int* selected = nullptr;        // (n_max) selection before ordering

@@ -21,6 +21,13 @@
 // the sum of the squared bucket sizes: populations spread over the directions
 // have buckets of a few members.  Where a few directions hold most of the
 // front (the bounds below), the caller's sorts take over.
+//
+// Bound by the latency of its ten phases (each a global or distributed-memory
+// round trip and a barrier, 3,000-4,000 clocks): DTLZ1 M=3 N=32768 (31,000
+// prior and 2,000 last members, 32,640 directions) 21 us where the prior
+// counts, the three sorts and the survivor list took 95; DTLZ2 M=8 N=6436
+// (9,700 last members) 19 us against 125; 275 directions with buckets of up to
+// 458 of 7,900 members 30 us against 120.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -32,7 +39,6 @@ namespace moea {
 constexpr int kNsLevels = 1024;            // niche levels told apart; the last one also holds all above it
 constexpr int kNsBins = 1024;              // bins of the boundary level's random words
 constexpr int kNsWordStep = 512;           // survivor words written out per step (at most a block's threads)
-constexpr int kNsItems = 8;                // last-front members per thread, at most
 constexpr int kNsMaxBucket = 2048;         // largest direction bucket ranked by counting
 constexpr unsigned long long kNsMaxWork = 8ull << 20;  // largest sum of squared bucket sizes
 
@@ -45,8 +51,10 @@ struct NicheScratch {
     uint64_t* key_b;     // (nl)
     int* dir_of;         // (nl)
     uint32_t* mask;      // (ceil(n_mix / 32)) survivor bits
-    int* list_count;     // (1)
+    int* hist;           // (kNsLevels) members per niche level, then (kNsBins) members per bin, then
+                         // the length of the list of the boundary bin
 };
+constexpr int kNsHistWords = kNsLevels + kNsBins + 1;
 
 NicheScratch niche_scratch(const Workspace& ws);
 
@@ -56,10 +64,11 @@ int launch_niche_select(const int* idx, const float* dist, const int* sizes, con
                         uint64_t seed, unsigned long long* offset, const int* nds_gidx, int* selected, int n_mix, int N,
                         int* survivors, int* status, cudaStream_t stream);
 
-template <int THREADS>
+// ITEMS: last-front members per thread, at most.
+template <int THREADS, int ITEMS>
 struct NicheShared {
+    uint64_t stage[ITEMS * THREADS + 2 * kNsMaxBucket];  // the buckets that this CTA's members belong to
     int hist[kNsLevels];
-    int bins[kNsBins];
     int wsum[THREADS / 32];
     unsigned long long wsum64[THREADS / 32];
     int wmax[THREADS / 32];
@@ -67,6 +76,7 @@ struct NicheShared {
     int seg_max;                    // largest bucket of the segment
     unsigned long long seg_work;    // sum of squared bucket sizes of the segment
     int seg_off[16];                // first position of each CTA's segment
+    int max_bucket;
     int level, level_take, level_all, bin, bin_take;
     int word_off[kNsWordStep];
     int fallback;
@@ -74,7 +84,8 @@ struct NicheShared {
 
 // The CTAs that select together: a cluster, or one CTA.
 struct NicheCluster {
-    cooperative_groups::cluster_group g;
+    static constexpr bool kMany = true;
+    cooperative_groups::cluster_group g = cooperative_groups::this_cluster();
     __device__ __forceinline__ int rank() const { return (int)g.block_rank(); }
     __device__ __forceinline__ int count() const { return (int)g.num_blocks(); }
     __device__ __forceinline__ void sync() { g.sync(); }
@@ -82,6 +93,7 @@ struct NicheCluster {
     __device__ __forceinline__ T* map(T* p, int r) { return g.map_shared_rank(p, r); }
 };
 struct NicheSolo {
+    static constexpr bool kMany = false;
     __device__ __forceinline__ int rank() const { return 0; }
     __device__ __forceinline__ int count() const { return 1; }
     __device__ __forceinline__ void sync() { __syncthreads(); }
@@ -114,23 +126,18 @@ __device__ __forceinline__ int niche_scan(int v, int* wsum, int* total)
     return incl - v + (warp > 0 ? before : 0);
 }
 
-// The bin of a histogram held by every CTA of the group (summed over them)
-// where the running count reaches `want`: the bin, the members to take from it
-// and its size.  Every thread of every CTA calls; the result is in sm.
-template <int THREADS, class G>
-__device__ __forceinline__ void niche_threshold(G& grp, int* hist, int nbins, int want, int* wsum, int* out_bin,
-                                                int* out_take, int* out_size)
+// The bin of a histogram in device memory where the running count reaches
+// `want`: the bin, the members to take from it and its size.
+template <int THREADS>
+__device__ __forceinline__ void niche_threshold(const int* hist, int want, int* wsum, int* out_bin, int* out_take,
+                                                int* out_size)
 {
-    static_assert(kNsLevels % THREADS == 0 || THREADS % kNsLevels == 0, "bins per thread");
-    constexpr int kPer = kNsLevels > THREADS ? kNsLevels / THREADS : 1;
-    const int C = grp.count();
+    static_assert(kNsLevels == kNsBins && kNsLevels % THREADS == 0, "bins per thread");
+    constexpr int kPer = kNsLevels / THREADS;
     int v[kPer], sum = 0;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-        const int b = threadIdx.x * kPer + k;
-        v[k] = 0;
-        if (b < nbins)
-            for (int r = 0; r < C; ++r) v[k] += grp.map(hist, r)[b];
+        v[k] = __ldcg(hist + threadIdx.x * kPer + k);
         sum += v[k];
     }
     int total;
@@ -147,16 +154,30 @@ __device__ __forceinline__ void niche_threshold(G& grp, int* hist, int nbins, in
     __syncthreads();
 }
 
+// Keys of w[0, n) below k, eight loads in flight.
+__device__ __forceinline__ int niche_rank(const uint64_t* w, int n, uint64_t k)
+{
+    int rank = 0, u = 0;
+    for (; u + 8 <= n; u += 8) {
+        uint64_t a[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] = w[u + i];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) rank += a[i] < k ? 1 : 0;
+    }
+    for (; u < n; ++u) rank += w[u] < k ? 1 : 0;
+    return rank;
+}
+
 __device__ __forceinline__ void niche_mark(uint32_t* mask, int g) { atomicOr(mask + (g >> 5), 1u << (g & 31)); }
 
 // Marks the survivors of one selection in S.mask: every member of the prior
 // fronts and, unless it returns false, the nrem members of the last front
 // that the three orders above put first.  It returns false (in every thread
 // of the group, with S.rho and the prior members' bits complete) when the
-// buckets are too large to be ranked by counting.  nl <= kNsItems * THREADS *
-// CTAs.  Ends with the group in step.
-template <int THREADS, class G>
-__device__ bool niche_buckets(G& grp, NicheShared<THREADS>& sm, const NicheScratch& S, const int* __restrict__ idx,
+// buckets are too large to be ranked by counting.  nl <= ITEMS * THREADS * CTAs.  Ends with the group in step.
+template <int THREADS, int ITEMS, class G>
+__device__ bool niche_buckets(G& grp, NicheShared<THREADS, ITEMS>& sm, const NicheScratch& S, const int* __restrict__ idx,
                               const float* __restrict__ dist, const int* __restrict__ gidx, int np, int nl, int nrem,
                               int H, uint64_t seed, unsigned long long off, int n_mix)
 {
@@ -165,54 +186,66 @@ __device__ bool niche_buckets(G& grp, NicheShared<THREADS>& sm, const NicheScrat
     for (int i = gt; i < H; i += T) S.rho[i] = 0;
     for (int i = gt; i <= H; i += T) S.last[i] = 0;
     for (int i = gt; i < (n_mix + 31) >> 5; i += T) S.mask[i] = 0;
+    for (int i = gt; i < kNsHistWords; i += T) S.hist[i] = 0;
     for (int i = tid; i < kNsLevels; i += THREADS) sm.hist[i] = 0;
-    for (int i = tid; i < kNsBins; i += THREADS) sm.bins[i] = 0;
-    if (gt == 0) *S.list_count = 0;
     if (tid == 0) {
         sm.level = nrem > 0 ? 1 << 30 : -1;  // stays when all members of the last front are taken, or none
         sm.level_take = sm.level_all = 0;
         sm.bin = -1;
         sm.bin_take = 0;
     }
+    // this CTA's members, as well as its positions in the orders below: [lo, hi)
+    const int slice = (nl + C - 1) / C;
+    const int lo = min(nl, c * slice), hi = min(nl, lo + slice);
+    int dir[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const int p = lo + tid + j * THREADS;
+        dir[j] = -1;
+        if (p < hi) {
+            const int r = idx[np + p];
+            dir[j] = (r >= 0 && r < H) ? r : H;
+        }
+    }
     grp.sync();
     // direction counts; a member's slot in its direction comes from the count
-    for (int i = gt; i < np; i += T) {
-        const int r = idx[i];
-        niche_mark(S.mask, gidx[i]);
-        if (r >= 0 && r < H) atomicAdd(S.rho + r, 1);
-    }
-    int bucket[kNsItems], slot[kNsItems];
+    int slot[ITEMS];
 #pragma unroll
-    for (int j = 0; j < kNsItems; ++j) {
-        const int p = gt + j * T;
-        if (p - lane >= nl) break;  // warp-uniform
-        const bool valid = p < nl;
-        int b = -1;
-        if (valid) {
-            const int r = idx[np + p];
-            b = (r >= 0 && r < H) ? r : H;
-        }
-        const unsigned peers = __match_any_sync(0xFFFFFFFFu, b);
+    for (int j = 0; j < ITEMS; ++j) {
+        if (lo + warp * 32 + j * THREADS >= hi) break;  // warp-uniform
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, dir[j]);
         const int leader = __ffs(peers) - 1;
         int base = 0;
-        if (valid && lane == leader) base = atomicAdd(S.last + b, __popc(peers));
-        base = __shfl_sync(0xFFFFFFFFu, base, leader);
-        bucket[j] = b;
-        slot[j] = base + __popc(peers & ((1u << lane) - 1u));
+        if (dir[j] >= 0 && lane == leader) base = atomicAdd(S.last + dir[j], __popc(peers));
+        slot[j] = __shfl_sync(0xFFFFFFFFu, base, leader) + __popc(peers & ((1u << lane) - 1u));
+    }
+    for (int i = gt; i - lane < np; i += 4 * T) {  // warp-uniform
+        int r[4], g[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            r[k] = (i + k * T < np) ? idx[i + k * T] : -1;
+            g[k] = (i + k * T < np) ? gidx[i + k * T] : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (g[k] >= 0) niche_mark(S.mask, g[k]);
+            const unsigned peers = __match_any_sync(0xFFFFFFFFu, r[k]);
+            if (r[k] >= 0 && r[k] < H && lane == __ffs(peers) - 1) atomicAdd(S.rho + r[k], __popc(peers));
+        }
     }
     grp.sync();
     // first position of each direction: every CTA scans a segment of directions
     const int per = (((H + 1 + C - 1) / C) + 3) & ~3;
     {
-        const int lo = c * per, hi = min(H + 1, lo + per);
+        const int b_lo = c * per, b_hi = min(H + 1, b_lo + per);
         int carry = 0, big = 0;
         unsigned long long work = 0;
-        for (int b0 = lo; b0 < hi; b0 += 4 * THREADS) {
+        for (int b0 = b_lo; b0 < b_hi; b0 += 4 * THREADS) {
             const int b = b0 + 4 * tid;
             int v[4] = {0, 0, 0, 0};
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (b + k < hi) v[k] = __ldcg(S.last + b + k);
+                if (b + k < b_hi) v[k] = __ldcg(S.last + b + k);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 big = max(big, v[k]);
@@ -222,7 +255,7 @@ __device__ bool niche_buckets(G& grp, NicheShared<THREADS>& sm, const NicheScrat
             int at = carry + niche_scan<THREADS>(v[0] + v[1] + v[2] + v[3], sm.wsum, &total);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                if (b + k < hi) __stcg(S.start + b + k, at);
+                if (b + k < b_hi) __stcg(S.start + b + k, at);
                 at += v[k];
             }
             carry += total;
@@ -237,27 +270,43 @@ __device__ bool niche_buckets(G& grp, NicheShared<THREADS>& sm, const NicheScrat
             sm.wsum64[warp] = work;
         }
         __syncthreads();
-        if (tid == 0) {
-            for (int w = 1; w < THREADS / 32; ++w) {
-                big = max(big, sm.wmax[w]);
-                work += sm.wsum64[w];
+        if (warp == 0) {
+            big = lane < THREADS / 32 ? sm.wmax[lane] : 0;
+            work = lane < THREADS / 32 ? sm.wsum64[lane] : 0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                big = max(big, __shfl_xor_sync(0xFFFFFFFFu, big, o));
+                work += __shfl_xor_sync(0xFFFFFFFFu, work, o);
             }
-            sm.seg_total = carry;
-            sm.seg_max = big;
-            sm.seg_work = work;
+            if (lane == 0) {
+                sm.seg_total = carry;
+                sm.seg_max = big;
+                sm.seg_work = work;
+            }
         }
     }
     grp.sync();
-    if (tid == 0) {
+    if (warp == 0) {
         int at = 0, big = 0;
         unsigned long long work = 0;
-        for (int r = 0; r < C; ++r) {
-            sm.seg_off[r] = at;
-            at += *grp.map(&sm.seg_total, r);
-            big = max(big, *grp.map(&sm.seg_max, r));
-            work += *grp.map(&sm.seg_work, r);
+        if (lane < C) {
+            at = *grp.map(&sm.seg_total, lane);
+            big = *grp.map(&sm.seg_max, lane);
+            work = *grp.map(&sm.seg_work, lane);
         }
-        sm.fallback = (big > kNsMaxBucket || work > kNsMaxWork) ? 1 : 0;
+        int incl = at;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += y;
+            big = max(big, __shfl_xor_sync(0xFFFFFFFFu, big, o));
+            work += __shfl_xor_sync(0xFFFFFFFFu, work, o);
+        }
+        if (lane < C) sm.seg_off[lane] = incl - at;
+        if (lane == 0) {
+            sm.max_bucket = big;
+            sm.fallback = (big > kNsMaxBucket || work > kNsMaxWork) ? 1 : 0;
+        }
     }
     __syncthreads();
     if (sm.fallback) {  // the same in every CTA
@@ -266,95 +315,108 @@ __device__ bool niche_buckets(G& grp, NicheShared<THREADS>& sm, const NicheScrat
     }
     // members into their direction's bucket, keyed by (distance, member)
 #pragma unroll
-    for (int j = 0; j < kNsItems; ++j) {
-        const int p = gt + j * T;
-        if (p >= nl) break;
-        const int b = bucket[j];
+    for (int j = 0; j < ITEMS; ++j) {
+        const int p = lo + tid + j * THREADS;
+        if (p >= hi) break;
+        const int b = dir[j];
         const int pos = sm.seg_off[b / per] + __ldcg(S.start + b) + slot[j];
         __stcg(S.key_a + pos, ((uint64_t)__float_as_uint(dist[np + p]) << 32) | (uint32_t)p);
         __stcg(S.dir_of + pos, b);
     }
     grp.sync();
-    // order 1 inside the buckets, and the words of order 2
-    int first[kNsItems], size[kNsItems], prior[kNsItems], member[kNsItems];
+    // The buckets of this CTA's positions reach at most the largest bucket
+    // beyond them: they are ranked in shared memory.  Order 1 inside the
+    // buckets, and the words of order 2.
+    const int w_lo = max(0, lo - sm.max_bucket), w_hi = lo < hi ? min(nl, hi + sm.max_bucket) : w_lo;
+    int first[ITEMS], size[ITEMS], prior[ITEMS], member[ITEMS];
+    for (int u = w_lo + tid; u < w_hi; u += THREADS) sm.stage[u - w_lo] = __ldcg(S.key_a + u);
 #pragma unroll
-    for (int j = 0; j < kNsItems; ++j) {
-        const int q = gt + j * T;
-        if (q >= nl) break;
-        const int b = S.dir_of[q];
-        const int s = sm.seg_off[b / per] + S.start[b], n = S.last[b];
-        const uint64_t k = S.key_a[q];
-        const int pr = b < H ? S.rho[b] : 0;
-        int rank = 0;
-#pragma unroll 8
-        for (int u = 0; u < n; ++u) rank += S.key_a[s + u] < k ? 1 : 0;
-        const uint32_t rnd = splitmix_u32(off + (uint64_t)(s + rank), seed);
-        const uint32_t low = (pr == 0 && rank == 0) ? 0u : (rnd | 1u);
-        S.key_b[q] = ((uint64_t)low << 32) | (uint32_t)(s + rank);
-        first[j] = s;
-        size[j] = n;
-        prior[j] = pr;
+    for (int j = 0; j < ITEMS; ++j) {
+        const int q = lo + tid + j * THREADS;
+        first[j] = size[j] = prior[j] = member[j] = 0;
+        if (q >= hi) continue;
+        const int b = __ldcg(S.dir_of + q);
+        first[j] = sm.seg_off[b / per] + __ldcg(S.start + b);
+        size[j] = __ldcg(S.last + b);
+        prior[j] = b < H ? __ldcg(S.rho + b) : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const int q = lo + tid + j * THREADS;
+        if (q >= hi) break;
+        const uint64_t k = sm.stage[q - w_lo];
+        const int rank = niche_rank(sm.stage + (first[j] - w_lo), size[j], k);
+        const int at = first[j] + rank;
+        const uint32_t rnd = splitmix_u32(off + (uint64_t)at, seed);
+        const uint32_t low = (prior[j] == 0 && rank == 0) ? 0u : (rnd | 1u);
+        __stcg(S.key_b + q, ((uint64_t)low << 32) | (uint32_t)at);
         member[j] = (int)(uint32_t)k;
     }
     grp.sync();
     // order 2 inside the buckets; the levels and words of order 3
-    uint32_t word[kNsItems];
-    int at[kNsItems];
+    uint32_t word[ITEMS];
+    int pos2[ITEMS];
+    for (int u = w_lo + tid; u < w_hi; u += THREADS) sm.stage[u - w_lo] = __ldcg(S.key_b + u);
+    __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kNsItems; ++j) {
-        const int q = gt + j * T;
-        if (q >= nl) break;
-        const int s = first[j], n = size[j];
-        const uint64_t k = S.key_b[q];
-        int rank = 0;
-#pragma unroll 8
-        for (int u = 0; u < n; ++u) rank += S.key_b[s + u] < k ? 1 : 0;
-        at[j] = s + rank;
-        word[j] = splitmix_u32(off + (uint64_t)nl + (uint64_t)(s + rank), seed);
+    for (int j = 0; j < ITEMS; ++j) {
+        const int q = lo + tid + j * THREADS;
+        if (q >= hi) break;
+        const uint64_t k = sm.stage[q - w_lo];
+        const int rank = niche_rank(sm.stage + (first[j] - w_lo), size[j], k);
+        pos2[j] = first[j] + rank;
+        word[j] = splitmix_u32(off + (uint64_t)nl + (uint64_t)pos2[j], seed);
         prior[j] += rank;  // the level
         atomicAdd(sm.hist + min(prior[j], kNsLevels - 1), 1);
     }
-    grp.sync();
     const bool part = nrem > 0 && nrem < nl;
+    bool split = false;
     if (part) {
-        niche_threshold<THREADS>(grp, sm.hist, kNsLevels, nrem, sm.wsum, &sm.level, &sm.level_take, &sm.level_all);
+        __syncthreads();
+        for (int i = tid; i < kNsLevels; i += THREADS)
+            if (sm.hist[i]) atomicAdd(S.hist + i, sm.hist[i]);
+        grp.sync();
+        niche_threshold<THREADS>(S.hist, nrem, sm.wsum, &sm.level, &sm.level_take, &sm.level_all);
         if (sm.level == kNsLevels - 1 && sm.level_take < sm.level_all) {  // levels above are not told apart
             grp.sync();
             return false;
         }
-        if (sm.level_take < sm.level_all) {
-#pragma unroll
-            for (int j = 0; j < kNsItems; ++j) {
-                if (gt + j * T >= nl) break;
-                if (prior[j] == sm.level) atomicAdd(sm.bins + (word[j] >> 22), 1);
-            }
-        }
+        split = sm.level_take < sm.level_all;
     }
     const int level = sm.level;
-    const bool split = part && sm.level_take < sm.level_all;
-    grp.sync();  // bins complete; the level histograms were read
-    if (split) niche_threshold<THREADS>(grp, sm.bins, kNsBins, sm.level_take, sm.wsum, &sm.bin, &sm.bin_take, &sm.level_all);
-    const int bin = sm.bin, bin_take = sm.bin_take;
+    if (split) {
+        int* bins = S.hist + kNsLevels;
 #pragma unroll
-    for (int j = 0; j < kNsItems; ++j) {
-        if (gt + j * T >= nl) break;
+        for (int j = 0; j < ITEMS; ++j) {
+            if (lo + tid + j * THREADS >= hi) break;
+            if (prior[j] == level) atomicAdd(bins + (word[j] >> 22), 1);
+        }
+        grp.sync();
+        niche_threshold<THREADS>(bins, sm.level_take, sm.wsum, &sm.bin, &sm.bin_take, &sm.level_all);
+    }
+    const int bin = sm.bin, bin_take = sm.bin_take;
+    int* list_count = S.hist + kNsLevels + kNsBins;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        if (lo + tid + j * THREADS >= hi) break;
         bool take = prior[j] < level || (prior[j] == level && !split);
         if (split && prior[j] == level) {
             const int wb = (int)(word[j] >> 22);
             take = wb < bin;
             if (wb == bin)  // ranked below
-                S.key_a[atomicAdd(S.list_count, 1)] = ((uint64_t)word[j] << 32) | (uint32_t)at[j];
+                __stcg(S.key_a + atomicAdd(list_count, 1), ((uint64_t)word[j] << 32) | (uint32_t)pos2[j]);
         }
         if (take) niche_mark(S.mask, gidx[np + member[j]]);
     }
-    grp.sync();  // the list is complete; the bins were read
+    grp.sync();  // the list is complete
     if (split) {
-        const int ln = __ldcg(S.list_count);
+        const int ln = __ldcg(list_count);
 #pragma unroll
-        for (int j = 0; j < kNsItems; ++j) {
-            if (gt + j * T >= nl) break;
+        for (int j = 0; j < ITEMS; ++j) {
+            if (lo + tid + j * THREADS >= hi) break;
             if (prior[j] != level || (int)(word[j] >> 22) != bin) continue;
-            const uint64_t k = ((uint64_t)word[j] << 32) | (uint32_t)at[j];
+            const uint64_t k = ((uint64_t)word[j] << 32) | (uint32_t)pos2[j];
             int rank = 0;
             for (int u = 0; u < ln; ++u) rank += __ldcg(S.key_a + u) < k ? 1 : 0;
             if (rank < bin_take) niche_mark(S.mask, gidx[np + member[j]]);
@@ -366,8 +428,8 @@ __device__ bool niche_buckets(G& grp, NicheShared<THREADS>& sm, const NicheScrat
 
 // Survivors in ascending order from the bits of S.mask (complete, the group in
 // step).  Every CTA counts the words before its own and writes its own out.
-template <int THREADS, class G>
-__device__ void niche_survivors(G& grp, NicheShared<THREADS>& sm, const uint32_t* mask, int n_mix,
+template <int THREADS, int ITEMS, class G>
+__device__ void niche_survivors(G& grp, NicheShared<THREADS, ITEMS>& sm, const uint32_t* mask, int n_mix,
                                 int* __restrict__ survivors, int cap)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -38,7 +38,7 @@ namespace moea {
 namespace {
 
 constexpr int kNcCtas = 16;
-constexpr int kNcThreads = 512;
+constexpr int kNcThreads = 1024;
 constexpr int kNcWarps = kNcThreads / 32;
 constexpr int kNcSlice = 4096;                        // members per CTA
 constexpr int kNcSteps = kNcSlice / kNcWarps / 32;    // 32-member steps per warp segment
@@ -569,9 +569,10 @@ nich_cluster(const int* __restrict__ idx, const float* __restrict__ dist, const 
 // direction buckets of niche_select.cuh, else the three sorts above.
 union NcSelectShared {
     NcShared sorts;
-    NicheShared<kNcThreads> buckets;
+    NicheShared<kNcThreads, kNcPerThread> buckets;
 };
 
+template <class G>
 __global__ void __launch_bounds__(kNcThreads, 1)
 nich_select(const int* __restrict__ idx, const float* __restrict__ dist, const int* __restrict__ sizes, NicheScratch S,
             int H, uint64_t seed, unsigned long long* __restrict__ offset, const int* __restrict__ nds_gidx,
@@ -579,7 +580,7 @@ nich_select(const int* __restrict__ idx, const float* __restrict__ dist, const i
 {
     extern __shared__ __align__(16) unsigned char nc_raw[];
     NcSelectShared& sm = *reinterpret_cast<NcSelectShared*>(nc_raw);
-    NicheCluster grp{cg::this_cluster()};
+    G grp;
     const int c = grp.rank();
     const int np = sizes[0], nl = sizes[1], nrem = sizes[2];
     // every branch below is uniform over the cluster
@@ -588,33 +589,27 @@ nich_select(const int* __restrict__ idx, const float* __restrict__ dist, const i
         return;
     }
     const unsigned long long off = *offset;
-    if (niche_buckets<kNcThreads>(grp, sm.buckets, S, idx, dist, nds_gidx, np, nl, nrem, H, seed, off, n_mix)) {
+    if (niche_buckets<kNcThreads, kNcPerThread>(grp, sm.buckets, S, idx, dist, nds_gidx, np, nl, nrem, H, seed, off, n_mix)) {
         if (c == 0 && threadIdx.x == 0) *offset = off + 2ull * (unsigned long long)nl;
     } else {
-        if (nl > kNcSlice)
-            nc_niching<false>(sm.sorts, grp.g, c, idx, dist, np, nl, nrem, S.rho, H, seed, offset, nds_gidx, selected);
+        cg::cluster_group cluster = cg::this_cluster();
+        if (G::kMany && nl > kNcSlice)
+            nc_niching<false>(sm.sorts, cluster, c, idx, dist, np, nl, nrem, S.rho, H, seed, offset, nds_gidx, selected);
         else if (c == 0)
-            nc_niching<true>(sm.sorts, grp.g, 0, idx, dist, np, nl, nrem, S.rho, H, seed, offset, nds_gidx, selected);
+            nc_niching<true>(sm.sorts, cluster, 0, idx, dist, np, nl, nrem, S.rho, H, seed, offset, nds_gidx, selected);
         grp.sync();  // the selection is complete
         const int take = min(nrem, nl);
         for (int i = c * kNcThreads + (int)threadIdx.x; i < take; i += grp.count() * kNcThreads)
             niche_mark(S.mask, __ldcg(selected + np + i));
         grp.sync();
     }
-    niche_survivors<kNcThreads>(grp, sm.buckets, S.mask, n_mix, survivors, N);
+    niche_survivors<kNcThreads, kNcPerThread>(grp, sm.buckets, S.mask, n_mix, survivors, N);
 }
 
-static_assert(kNsItems * kNcThreads == kNcSlice, "a CTA's members in registers");
-
-// CTAs of a selection: one per 1024 merged points up to 4096 (where one CTA
-// can also run the sorts), else the whole cluster.
-int nich_select_ctas(int n_mix, int H)
-{
-    if (n_mix > kNcSlice || H > 2 * kNcSlice) return kNcCtas;
-    int c = 1;
-    while (c * 1024 < n_mix) c *= 2;
-    return c;
-}
+// One CTA for the merged populations whose last front it can hold and few
+// directions, where CTA barriers (about 1/10 of a cluster barrier with its
+// memory fence, of which a selection has eleven) outweigh the wider cluster.
+bool nich_select_solo(int n_mix, int H) { return n_mix <= kNcSlice && H <= 2 * kNcSlice; }
 
 }  // namespace
 
@@ -651,14 +646,16 @@ bool niching_cluster_ready()
         return false;
     }
     if (clusters < 1) return false;
-    if (cudaFuncSetAttribute(nich_select, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(nich_select, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(nich_select<NicheCluster>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(nich_select<NicheCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(NcSelectShared)) != cudaSuccess ||
+        cudaFuncSetAttribute(nich_select<NicheSolo>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(NcSelectShared)) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     cfg.dynamicSmemBytes = sizeof(NcSelectShared);
-    if (cudaOccupancyMaxActiveClusters(&clusters, (void*)nich_select, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, (void*)nich_select<NicheCluster>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -691,20 +688,25 @@ int launch_niche_select(const int* idx, const float* dist, const int* sizes, con
                         uint64_t seed, unsigned long long* offset, const int* nds_gidx, int* selected, int n_mix, int N,
                         int* survivors, int* status, cudaStream_t stream)
 {
-    const int ctas = nich_select_ctas(n_mix, H);
+    if (nich_select_solo(n_mix, H)) {
+        nich_select<NicheSolo><<<1, kNcThreads, sizeof(NcSelectShared), stream>>>(
+            idx, dist, sizes, S, H, seed, offset, nds_gidx, selected, n_mix, N, survivors, status);
+        MOEA_CUDA_TRY(cudaGetLastError());
+        return MOEA_OK;
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
+    cfg.gridDim = dim3(kNcCtas);
     cfg.blockDim = dim3(kNcThreads);
     cfg.dynamicSmemBytes = sizeof(NcSelectShared);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.x = kNcCtas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    MOEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, nich_select, idx, dist, sizes, S, H, seed, offset, nds_gidx, selected, n_mix,
+    MOEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, nich_select<NicheCluster>, idx, dist, sizes, S, H, seed, offset, nds_gidx, selected, n_mix,
                                      N, survivors, status));
     return MOEA_OK;
 }

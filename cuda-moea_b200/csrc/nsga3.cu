@@ -1644,7 +1644,7 @@ int run_order_selection(Workspace& ws, const int* selected, int count, int n_mix
 NicheScratch niche_scratch(const Workspace& ws)
 {
     return NicheScratch{ws.rho, ws.niche_last, ws.niche_start, ws.key64[0], ws.key64[1], ws.sel_vals[0],
-                        reinterpret_cast<uint32_t*>(ws.flags), ws.sizes + 5};
+                        reinterpret_cast<uint32_t*>(ws.flags), ws.niche_hist};
 }
 
 // One NSGA-III environmental selection on the split population.
