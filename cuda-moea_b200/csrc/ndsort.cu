@@ -5,13 +5,13 @@
 // Same result (front index per point, -1 past the stop rule, index of the last
 // front), different mechanism:
 //
-//  1. Sort of the points by (class, f0 | cv, S) with one 56-bit radix sort,
-//     S the top 22 bits of the order key of the FP32 sum f1 + ... + f_{M-1}.
+//  1. Sort of the points by (class, f0 | cv, S), a 56-bit key, in sorted tiles
+//     and rank merges (nds_sort_tiles, nds_sort_merge), S the top 22 bits of the order key of the FP32 sum f1 + ... + f_{M-1}.
 //     Class 0 = feasible, 1 = feasible with a NaN objective, 2 = infeasible,
 //     3 = infeasible with NaN violation.  FP32 addition rounds monotonically,
 //     so a feasible dominator p of q has f0(p) <= f0(q) and S(p) <= S(q); runs
 //     of equal keys in class 0 are then ordered lexicographically by
-//     (f1, ..., f_{M-1}, index) (nds_tie_fix, nds_tie_fix_long).  In this
+//     (f1, ..., f_{M-1}, index) (nds_tie_rank, nds_tie_fix_long).  In this
 //     order every dominator of a point lies strictly before it, identical
 //     vectors are adjacent, and a feasible dominator already satisfies
 //     f0 <= q0.
@@ -38,9 +38,12 @@
 //     reference's front propagation loops (:792-843, :1070-1279).
 #include <algorithm>
 
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include "internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace moea {
 namespace {
@@ -54,7 +57,8 @@ constexpr int kScanChunk = 512;    // words per chunk (16 per lane)
 constexpr uint32_t kInfeasibleBit = 0x80000000u;
 // Sort key: class (2 bits), the order key of f0 or of the violation (32
 // bits), the top kSortSBits bits of the order key of S.  22 bits of S keep
-// runs of equal keys as rare as 30 did while saving a radix pass; with 14
+// runs of equal keys as rare as 30 did and leave the eight bits that carry the
+// lane in a tile's first sort (seven radix passes in the fused sort); with 14
 // the runs grew and the tie fix-up cost more than the pass it saved.
 constexpr int kSortSBits = 22;
 constexpr int kSortKeyBits = 2 + 32 + kSortSBits;
@@ -65,8 +69,7 @@ constexpr int kSortClassShift = 32 + kSortSBits;
 // ---------------------------------------------------------------------------
 
 // Sort key of point i of class cls with key0 low word val: class << 54 |
-// val << 22 | S (class 0), kSortKeyBits bits (seven radix passes of 8 bits),
-// S the top 22 bits of the order key of the FP32 sum f1 + ... + f_{M-1}
+// val << 22 | S (class 0), kSortKeyBits bits, S the top 22 bits of the order key of the FP32 sum f1 + ... + f_{M-1}
 // (monotone in every f_m; +inf + -inf (NaN) sorts with +inf sums).
 __device__ __forceinline__ uint64_t sort_key(const SplitPop& pop, int M, int i, uint32_t cls, uint32_t val)
 {
@@ -79,40 +82,138 @@ __device__ __forceinline__ uint64_t sort_key(const SplitPop& pop, int M, int i, 
     return ((uint64_t)cls << kSortClassShift) | ((uint64_t)val << kSortSBits) | (s30 >> (30 - kSortSBits));
 }
 
-// key0[i] = class << 32 | order key of f0 (class 0) or cv (class 2);
-// skey[i] = sort_key(i).
-__global__ void nds_classify(SplitPop pop, int M, uint64_t* __restrict__ key0, uint64_t* __restrict__ skey,
-                             int* __restrict__ perm, int* __restrict__ feasible_count)
+// Class of point i, and its key0 low word: the order key of f0 (class 0) or of
+// the violation (class 2).
+__device__ __forceinline__ uint32_t classify_point(const SplitPop& pop, int M, int i, uint32_t* val)
+{
+    const float cv = pop.cvv(i);
+    *val = 0;
+    if (cv == 0.0f) {
+        bool nan = false;
+        for (int m = 0; m < M; ++m) nan |= isnan(pop.obj(m, i));
+        if (!nan) *val = float_order_key(pop.obj(0, i));
+        return nan ? 1u : 0u;
+    }
+    if (isnan(cv)) return 3u;
+    *val = float_order_key(cv);
+    return 2u;
+}
+
+// Count of the len ascending values a[] that are <= x, len <= L, L a power of two.
+__device__ __forceinline__ int count_le_step(const uint64_t* a, int len, int c, int s, uint64_t x)
+{
+    return (c + s <= len && a[c + s - 1] <= x) ? c + s : c;
+}
+
+// The sort of the keys, by rank instead of by digit.  A radix sort of the 56
+// key bits needs seven passes over all keys, each a launch bound by its
+// latency (9-10 us a pass at 4,000 to 65,536 points: 75 us with its histogram
+// and its classification).  Here tiles of 1024 keys are sorted in one CTA each
+// (a bitonic network per warp, then ranks by binary search in the CTA's other
+// runs: 8 x 32 -> 256, 4 x 256 -> 1024), and each merge pass places every key
+// by its rank in the seven other runs of its group: one pass up to 8192
+// points, two up to 65536, with the seven searches of a key side by side.
+// Equal keys keep their index order, as in the stable radix sort.
+constexpr int kSortTile = 1024;
+constexpr int kSortWays = 8;   // runs merged per pass
+
+// key0[i] = class << 32 | order key of f0 (class 0) or cv (class 2); sorted
+// tiles of (sort_key, index) into skey and perm.  Clears the sort's counters.
+__global__ void __launch_bounds__(kSortTile)
+nds_sort_tiles(SplitPop pop, int M, uint64_t* __restrict__ key0, uint64_t* __restrict__ skey, int* __restrict__ perm,
+               int* __restrict__ counters)
+{
+    __shared__ uint64_t s_a[kSortTile], s_b[kSortTile];
+    __shared__ unsigned short s_i[kSortTile];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int base = blockIdx.x * kSortTile, i = base + t;
+    if (blockIdx.x == 0 && t < 20 && (t < 5 || (t >= 10 && t <= 13) || t >= 16)) counters[t] = 0;
+    uint64_t key = (1ull << kSortKeyBits) - 1ull;  // padding: above every real key
+    if (i < pop.n) {
+        uint32_t val;
+        const uint32_t cls = classify_point(pop, M, i, &val);
+        key0[i] = ((uint64_t)cls << 32) | val;
+        key = sort_key(pop, M, i, cls, val);
+    }
+    uint64_t v = (key << 8) | (unsigned)lane;  // 56 + 8 bits; every real key is positive
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const uint64_t o = __shfl_xor_sync(0xFFFFFFFFu, v, j);
+            const bool take_min = ((lane & j) == 0) == ((lane & k) == 0);
+            v = take_min ? (o < v ? o : v) : (o > v ? o : v);
+        }
+    }
+    s_a[t] = v;
+    __syncthreads();
+    {
+        const uint64_t hi = v | 0xFFull, lo = (v & ~0xFFull) - 1ull;  // counts of <= key and < key
+        const int w0 = warp & ~7;
+        int c[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) c[r] = 0;
+#pragma unroll
+        for (int s = 16; s >= 1; s >>= 1)
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                c[r] = count_le_step(s_a + (w0 + r) * 32, 32, c[r], s, w0 + r < warp ? hi : lo);
+        int rank = lane;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            c[r] = count_le_step(s_a + (w0 + r) * 32, 32, c[r], 1, w0 + r < warp ? hi : lo);
+            if (w0 + r != warp) rank += c[r];
+        }
+        s_b[w0 * 32 + rank] = v & ~0xFFull;
+        s_i[w0 * 32 + rank] = (unsigned short)(warp * 32 + (int)(v & 31ull));
+    }
+    __syncthreads();
+    v = s_b[t];
+    const int g = t >> 8;
+    int c[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int s = 128; s >= 1; s >>= 1)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) c[r] = count_le_step(s_b + r * 256, 256, c[r], s, r < g ? v : v - 1ull);
+    int rank = t & 255;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        c[r] = count_le_step(s_b + r * 256, 256, c[r], 1, r < g ? v : v - 1ull);
+        if (r != g) rank += c[r];
+    }
+    if (base + rank < pop.n) {
+        skey[base + rank] = v >> 8;
+        perm[base + rank] = base + (int)s_i[t];
+    }
+}
+
+// Sorted runs of L keys (L a power of two) merged in groups of kSortWays.
+__global__ void __launch_bounds__(256)
+nds_sort_merge(const uint64_t* __restrict__ key_in, const int* __restrict__ perm_in, uint64_t* __restrict__ key_out,
+               int* __restrict__ perm_out, int n, int L)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool feasible_class = false, infeasible2 = false, infeasible3 = false;
-    if (i < pop.n) {
-        const float cv = pop.cvv(i);
-        uint32_t cls, val = 0;
-        if (cv == 0.0f) {
-            bool nan = false;
-            for (int m = 0; m < M; ++m) nan |= isnan(pop.obj(m, i));
-            cls = nan ? 1u : 0u;
-            if (!nan) val = float_order_key(pop.obj(0, i));
-        } else {
-            cls = isnan(cv) ? 3u : 2u;
-            if (cls == 2u) val = float_order_key(cv);
-        }
-        key0[i] = ((uint64_t)cls << 32) | val;
-        skey[i] = sort_key(pop, M, i, cls, val);
-        perm[i] = i;
-        feasible_class = cls <= 1u;
-        infeasible2 = cls == 2u;
-        infeasible3 = cls == 3u;
+    if (i >= n) return;
+    const uint64_t key = key_in[i];
+    const int run = i / L, r0 = run & ~(kSortWays - 1);
+    const long long first = (long long)r0 * L;
+    int c[kSortWays], len[kSortWays];
+#pragma unroll
+    for (int r = 0; r < kSortWays; ++r) {
+        const long long left = (long long)n - (first + (long long)r * L);
+        c[r] = 0;
+        len[r] = (r0 + r == run || left <= 0) ? 0 : (int)(left < L ? left : L);
     }
-    const unsigned fm = __ballot_sync(0xFFFFFFFFu, feasible_class);
-    const unsigned m2 = __ballot_sync(0xFFFFFFFFu, infeasible2);
-    const unsigned m3 = __ballot_sync(0xFFFFFFFFu, infeasible3);
-    if ((threadIdx.x & 31) == 0) {
-        if (fm) atomicAdd(feasible_count, __popc(fm));
-        if (m2) atomicAdd(feasible_count + 10, __popc(m2));
-        if (m3) atomicAdd(feasible_count + 11, __popc(m3));
-    }
+    for (int s = L >> 1; s >= 1; s >>= 1)
+#pragma unroll
+        for (int r = 0; r < kSortWays; ++r)
+            c[r] = count_le_step(key_in + first + (long long)r * L, len[r], c[r], s, r0 + r < run ? key : key - 1ull);
+    long long at = first + (i - (long long)run * L);
+#pragma unroll
+    for (int r = 0; r < kSortWays; ++r)
+        at += count_le_step(key_in + first + (long long)r * L, len[r], c[r], 1, r0 + r < run ? key : key - 1ull);
+    key_out[at] = key;
+    perm_out[at] = perm_in[i];
 }
 
 // Total order inside a run of equal sort keys of class 0: lexicographic on
@@ -131,34 +232,31 @@ constexpr int kTieLongThreads = 1024;
 constexpr int kTieLongCtas = 64;        // CTAs of nds_tie_fix_long, each taking runs in turn
 constexpr int kTieSmemSort = 4096;    // longer runs: bitonic in shared memory up to this size
 
-// One thread per run head of class 0: short runs are sorted in place, longer
-// ones are listed for nds_tie_fix_long.  Runs are disjoint, so the in-place
-// sorts do not race.
-__global__ void nds_tie_fix(SplitPop pop, int M, const uint64_t* __restrict__ skey, int* __restrict__ perm,
-                            int* __restrict__ long_runs, int* __restrict__ n_long)
+// Runs of equal keys in class 0 into lexicographic order: every member of a run
+// of at most kTieShort counts the members before it; longer runs are copied
+// and listed for nds_tie_fix_long.
+__global__ void nds_tie_rank(SplitPop pop, int M, const uint64_t* __restrict__ skey, const int* __restrict__ perm_in,
+                             int* __restrict__ perm_out, int* __restrict__ long_runs, int* __restrict__ n_long)
 {
     const int pos = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = pop.n;
     if (pos >= n) return;
     const uint64_t k = skey[pos];
-    if ((k >> kSortClassShift) != 0u || (pos > 0 && skey[pos - 1] == k)) return;
-    int L = 1;
-    while (L <= kTieShort && pos + L < n && skey[pos + L] == k) ++L;
-    if (L == 1) return;
-    if (L > kTieShort) {
-        long_runs[atomicAdd(n_long, 1)] = pos;
-        return;
-    }
-    int* a = perm + pos;
-    for (int x = 1; x < L; ++x) {
-        const int v = a[x];
-        int y = x - 1;
-        while (y >= 0 && tie_less(pop, M, v, a[y])) {
-            a[y + 1] = a[y];
-            --y;
+    const int pt = perm_in[pos];
+    int to = pos;
+    if ((k >> kSortClassShift) == 0u) {
+        int a = pos, b = pos + 1;  // the run, as far as kTieShort reaches
+        while (a > 0 && pos - a <= kTieShort && skey[a - 1] == k) --a;
+        while (b < n && b - a <= kTieShort && skey[b] == k) ++b;
+        if (b - a > kTieShort) {
+            if (a == pos) long_runs[atomicAdd(n_long, 1)] = pos;
+        } else if (b - a > 1) {
+            to = a;
+            for (int x = a; x < b; ++x)
+                if (x != pos && tie_less(pop, M, perm_in[x], pt)) ++to;
         }
-        a[y + 1] = v;
     }
+    perm_out[to] = pt;
 }
 
 // Ascending bitonic network over a[0, L) with virtual +inf padding to the
@@ -239,53 +337,77 @@ nds_tie_fix_long(SplitPop pop, int M, const uint64_t* __restrict__ skey, int* __
     }
 }
 
-// Sorted copy of objectives 1..M-1 and run heads for the dup computation.
-__global__ void nds_sorted_soa(SplitPop pop, int M, const uint64_t* __restrict__ key0,
-                               const int* __restrict__ perm, float* __restrict__ sf,
-                               int sf_stride, int* __restrict__ head)
+// Sorted copy of objectives 1..M-1, the dup positions, the peel's initial state
+// and the class counts.  The start of a run of identical vectors (class 0) or
+// violations (class 2) is found by doubling steps back and a binary search:
+// positions between two identical ones are identical, and nearly every run has
+// one member, so no scan over the positions is needed.
+__global__ void nds_finalize_rows(SplitPop pop, int M, const uint64_t* __restrict__ key0,
+                                  const uint64_t* __restrict__ skey, const int* __restrict__ perm,
+                                  float* __restrict__ sf, int sf_stride, int* __restrict__ counters,
+                                  int* __restrict__ qinfo, int* __restrict__ blocker, int* __restrict__ front_sorted,
+                                  uint32_t* __restrict__ fmask, int fmask_words)
 {
     const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos >= pop.n) return;
+    const int n = pop.n;
+    for (int w = pos; w < fmask_words; w += gridDim.x * blockDim.x) fmask[w] = 0u;
+    if (pos >= n) return;
     const int pt = perm[pos];
     const uint64_t k0 = key0[pt];
     const uint32_t cls = (uint32_t)(k0 >> 32);
     for (int m = 1; m < M; ++m) sf[(size_t)(m - 1) * sf_stride + pos] = pop.obj(m, pt);
-    bool is_head = true;
-    if (pos > 0) {
-        const int pp = perm[pos - 1];
-        const uint64_t k1 = key0[pp];
-        if (k1 == k0) {
-            if (cls == 0u) {
-                bool same = true;
-                for (int m = 1; m < M; ++m)
-                    same &= float_order_key(pop.obj(m, pt)) == float_order_key(pop.obj(m, pp));
-                is_head = !same;
-            } else {
-                is_head = false;
+    auto same = [&](int p) {
+        const int pp = perm[p];
+        if (key0[pp] != k0) return false;
+        bool eq = true;
+        if (cls == 0u)
+            for (int m = 1; m < M; ++m) eq &= float_order_key(pop.obj(m, pt)) == float_order_key(pop.obj(m, pp));
+        return eq;
+    };
+    uint32_t d = 0u;
+    if (cls == 0u || cls == 2u) {
+        int start = pos;
+        if (pos > 0 && same(pos - 1)) {
+            start = pos - 1;
+            int step = 2;
+            while (pos - step >= 0 && same(pos - step)) {
+                start = pos - step;
+                step *= 2;
+            }
+            int lo = max(-1, pos - step);  // differs (or before the first)
+            while (start - lo > 1) {
+                const int mid = (start + lo) >> 1;
+                if (same(mid)) start = mid;
+                else lo = mid;
             }
         }
-    }
-    head[pos] = is_head ? pos : 0;
-}
-
-__global__ void nds_finalize_rows(int n, const uint64_t* __restrict__ key0,
-                                  const int* __restrict__ perm, const int* __restrict__ run_start,
-                                  const int* __restrict__ feasible_count, int* __restrict__ qinfo,
-                                  int* __restrict__ blocker, int* __restrict__ front_sorted)
-{
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos >= n) return;
-    const uint32_t cls = (uint32_t)(key0[perm[pos]] >> 32);
-    uint32_t d;
-    switch (cls) {
-    case 0u: d = (uint32_t)run_start[pos]; break;
-    case 1u: d = 0u; break;
-    case 2u: d = (uint32_t)run_start[pos] | kInfeasibleBit; break;
-    default: d = (uint32_t)(*feasible_count) | kInfeasibleBit; break;
+        d = (uint32_t)start | (cls == 2u ? kInfeasibleBit : 0u);
+    } else if (cls == 3u) {
+        int lo = 0, hi = pos;  // first position of an infeasible class
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if ((skey[mid] >> kSortClassShift) >= 2u) hi = mid;
+            else lo = mid + 1;
+        }
+        d = (uint32_t)lo | kInfeasibleBit;
     }
     qinfo[pos] = (int)d;
     blocker[pos] = -1;
     front_sorted[pos] = -1;
+    // [0] feasible points, [10] class 2, [11] class 3, from the class boundaries
+    const uint32_t before = pos > 0 ? (uint32_t)(skey[pos - 1] >> kSortClassShift) : 0u;
+    if (cls >= 2u && before < 2u) {
+        counters[0] = pos;
+        atomicAdd(counters + 10, -pos);
+    }
+    if (cls == 3u && before < 3u) {
+        counters[11] = n - pos;
+        atomicAdd(counters + 10, pos);
+    }
+    if (pos == n - 1) {
+        if (cls < 2u) counters[0] = n;
+        if (cls == 2u) atomicAdd(counters + 10, n);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1165,60 +1287,76 @@ size_t peel_owned_smem(int W)
     return (size_t)((W + 3) & ~3) * sizeof(uint32_t) + (size_t)kWinChunks * kPeelThreads * sizeof(uint4);
 }
 
-// Run heads among the infeasible class-2 positions (sorted by violation).
-__global__ void nds_infeasible_heads(int n, const int* __restrict__ qinfo, const int* __restrict__ counters,
-                                     int target, int* __restrict__ flags)
+// Fronts in point order, and the closed-form fronts of the infeasible points
+// when the feasible ones number fewer than the target.  Every infeasible point
+// is dominated by all feasible points, a class-2 point also by every class-2
+// point of smaller violation, a class-3 point (NaN violation) by the feasible
+// points only.  With F the last feasible front (-1 without feasible points):
+// class 3 forms front F + 1 together with the first class-2 run of equal
+// violations, class-2 run j is front F + 1 + j.  The stop rule of the peel
+// keeps the fronts up to the first whose cumulative count reaches the target:
+// run j (j > 0) is kept when n3 + start_j < target.  One 8-CTA cluster: each
+// CTA numbers the runs of a segment, the segments' counts pass through the
+// cluster's shared memory (a launch instead of the head, scan and scatter
+// launches that it takes without).
+constexpr int kFrontCtas = 8, kFrontThreads = 1024;
+__global__ void __cluster_dims__(kFrontCtas, 1, 1) __launch_bounds__(kFrontThreads)
+nds_fronts(int n, const int* __restrict__ perm, const int* __restrict__ qinfo, const int* __restrict__ front_sorted,
+           int* counters, int target, int* __restrict__ fronts)
 {
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos >= n) return;
-    const int fc = counters[0], n2 = counters[10];
-    int f = 0;
-    if (fc < target && pos >= fc && pos < fc + n2)
-        f = ((uint32_t)qinfo[pos] & ~kInfeasibleBit) == (uint32_t)pos ? 1 : 0;
-    flags[pos] = f;
-}
-
-// Closed-form fronts of the infeasible points when the feasible ones number
-// fewer than the target.  Every infeasible point is dominated by all feasible
-// points, a class-2 point also by every class-2 point of smaller violation,
-// a class-3 point (NaN violation) by the feasible points only.  With F the
-// last feasible front (-1 without feasible points): class 3 forms front F + 1
-// together with the first class-2 run, class-2 run j is front F + 1 + j.  The
-// stop rule of the peel keeps the fronts up to the first whose cumulative
-// count reaches the target: run j (j > 0) is kept when n3 + start_j < target.
-// rank[pos] = inclusive count of run heads up to pos.
-__global__ void nds_infeasible_fronts(int n, const int* __restrict__ qinfo, const int* __restrict__ rank,
-                                      int* counters, int target, int* __restrict__ front_sorted)
-{
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    const int fc = counters[0], n2 = counters[10], n3 = counters[11];
-    if (fc >= target) return;
-    const int F1 = counters[12] + 1;
-    if (pos < n && pos >= fc) {
-        if (pos < fc + n2) {
-            const int j = rank[pos] - 1;
-            const int start = (int)((uint32_t)qinfo[pos] & ~kInfeasibleBit);
-            if (j == 0 || n3 + start < target) front_sorted[pos] = F1 + j;
-        } else {
-            front_sorted[pos] = F1;
-        }
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ int s_runs, s_w[kFrontThreads / 32];
+    const int c = (int)cluster.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int fc = counters[0], n2 = counters[10], n3 = counters[11], F1 = counters[12] + 1;
+    const bool closed = fc < target;  // uniform over the cluster
+    const int plain = closed ? fc : n;
+    for (int pos = c * kFrontThreads + tid; pos < n; pos += kFrontCtas * kFrontThreads)
+        if (pos < plain) fronts[perm[pos]] = front_sorted[pos];
+        else if (pos >= fc + n2) fronts[perm[pos]] = F1;
+    if (!closed) return;
+    if (n2 == 0) {
+        if (c == 0 && tid == 0) counters[2] = F1;
+        return;
     }
-    if (pos == 0) {
-        int last = F1;
-        if (n2 > 0) {
-            int p = target - n3 - 1;
-            p = p < fc ? fc : (p > fc + n2 - 1 ? fc + n2 - 1 : p);
-            last = F1 + rank[p] - 1;
-        }
-        counters[2] = last;
+    auto start_of = [&](int pos) { return (int)((uint32_t)qinfo[pos] & ~kInfeasibleBit); };
+    const int per = (n2 + kFrontCtas - 1) / kFrontCtas;
+    const int lo = fc + min(n2, c * per), hi = min(fc + n2, lo + per);
+    int runs = 0;
+    for (int pos = lo + tid; pos < hi; pos += kFrontThreads) runs += start_of(pos) == pos ? 1 : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) runs += __shfl_xor_sync(0xFFFFFFFFu, runs, o);
+    if (lane == 0) s_w[warp] = runs;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kFrontThreads / 32; ++w) runs += s_w[w];
+        s_runs = runs;
     }
-}
-
-__global__ void nds_scatter_fronts(int n, const int* __restrict__ perm,
-                                   const int* __restrict__ front_sorted, int* __restrict__ fronts)
-{
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos < n) fronts[perm[pos]] = front_sorted[pos];
+    cluster.sync();
+    int base = 0;
+    for (int r = 0; r < c; ++r) base += *cluster.map_shared_rank(&s_runs, r);
+    cluster.sync();  // the counts were read everywhere
+    // the position whose front is the last one kept
+    int p_last = target - n3 - 1;
+    p_last = p_last < fc ? fc : (p_last > fc + n2 - 1 ? fc + n2 - 1 : p_last);
+    for (int p0 = lo; p0 < hi; p0 += kFrontThreads) {
+        const int pos = p0 + tid;
+        const int start = pos < hi ? start_of(pos) : -1;
+        const unsigned heads = __ballot_sync(0xFFFFFFFFu, pos < hi && start == pos);
+        __syncthreads();  // s_w free
+        if (lane == 0) s_w[warp] = __popc(heads);
+        __syncthreads();
+        int before = base, total = base;
+        for (int w = 0; w < kFrontThreads / 32; ++w) {
+            before += w < warp ? s_w[w] : 0;
+            total += s_w[w];
+        }
+        if (pos < hi) {
+            const int j = before + __popc(heads & (0xFFFFFFFFu >> (31 - lane))) - 1;
+            fronts[perm[pos]] = (j == 0 || n3 + start < target) ? F1 + j : -1;
+            if (pos == p_last) counters[2] = F1 + j;
+        }
+        base = total;
+    }
 }
 
 __global__ void nds_reset_counters(int* counters)
@@ -2103,30 +2241,22 @@ int run_ndsort(Workspace& ws, const SplitPop& pop, int M, int target, int* out_f
     if (target > n) target = n;
     if (target < 1) target = 1;
     int* fronts = out_fronts ? out_fronts : ws.fronts;
-    int* feas = ws.counters;
     const int T = 256, G = ceil_div(n, T);
 
-    nds_reset_counters<<<1, 32, 0, stream>>>(ws.counters);
-    nds_classify<<<G, T, 0, stream>>>(pop, M, ws.key0, ws.key64[0], ws.perm[0], feas);
-    MOEA_CUDA_TRY(cudaGetLastError());
-    const uint64_t* key0 = ws.key0;
-    size_t tmp = ws.cub_bytes;
-    MOEA_CUDA_TRY(cub::DeviceRadixSort::SortPairs(ws.cub_tmp, tmp, ws.key64[0], ws.key64[1], ws.perm[0],
-                                                  ws.perm[1], n, 0, kSortKeyBits, stream));
+    nds_sort_tiles<<<ceil_div(n, kSortTile), kSortTile, 0, stream>>>(pop, M, ws.key0, ws.key64[0], ws.perm[0],
+                                                                     ws.counters);
+    int cur = 0;
+    for (long long L = kSortTile; L < n; L *= kSortWays, cur ^= 1)
+        nds_sort_merge<<<G, T, 0, stream>>>(ws.key64[cur], ws.perm[cur], ws.key64[cur ^ 1], ws.perm[cur ^ 1], n, (int)L);
+    const uint64_t* skey = ws.key64[cur];
+    int* perm = ws.perm[cur ^ 1];
     // runs of equal keys in class 0 into lexicographic order; ws.run_start
-    // holds the list of long runs until the dup scan below overwrites it
-    nds_tie_fix<<<G, T, 0, stream>>>(pop, M, ws.key64[1], ws.perm[1], ws.run_start, ws.counters + 13);
-    nds_tie_fix_long<<<kTieLongCtas, kTieLongThreads, 0, stream>>>(pop, M, ws.key64[1], ws.perm[1], ws.run_start,
-                                                               ws.counters + 13);
-    MOEA_CUDA_TRY(cudaGetLastError());
-    const int* perm = ws.perm[1];
-
-    nds_sorted_soa<<<G, T, 0, stream>>>(pop, M, key0, perm, ws.sorted_f, ws.n_max, ws.head);
-    MOEA_CUDA_TRY(cub::DeviceScan::InclusiveScan(ws.cub_tmp, tmp, ws.head, ws.run_start,
-                                                 cub::Max(), n, stream));
+    // holds the list of long runs
+    nds_tie_rank<<<G, T, 0, stream>>>(pop, M, skey, ws.perm[cur], perm, ws.run_start, ws.counters + 13);
+    nds_tie_fix_long<<<kTieLongCtas, kTieLongThreads, 0, stream>>>(pop, M, skey, perm, ws.run_start, ws.counters + 13);
     int* qinfo = ws.qinfo;
-    nds_finalize_rows<<<G, T, 0, stream>>>(n, key0, perm, ws.run_start, feas, qinfo, ws.blocker,
-                                           ws.front_sorted);
+    nds_finalize_rows<<<G, T, 0, stream>>>(pop, M, ws.key0, skey, perm, ws.sorted_f, ws.n_max, ws.counters, qinfo,
+                                           ws.blocker, ws.front_sorted, ws.peel_fmask, 3 * ws.words);
     MOEA_CUDA_TRY(cudaGetLastError());
     stage_mark("ndsort.lexsort", stream);
 
@@ -2152,8 +2282,7 @@ int run_ndsort(Workspace& ws, const SplitPop& pop, int M, int target, int* out_f
     MOEA_CUDA_TRY(cudaGetLastError());
     stage_mark("ndsort.dominance_tiles", stream);
 
-    // cooperative peel
-    const int W = ceil_div(n, 32);
+    // cooperative peel; nds_finalize_rows left its three front masks empty
     // every co-resident CTA with at least one group of 32 positions: each
     // CTA scans the rows of its own groups, so more CTAs mean fewer rows per
     // CTA and front (one CTA per group of 32 warps left half the SMs idle)
@@ -2168,9 +2297,6 @@ int run_ndsort(Workspace& ws, const SplitPop& pop, int M, int target, int* out_f
     int* fs = ws.front_sorted;
     uint32_t* fmask = ws.peel_fmask;
     int* ctr = ws.counters;
-    (void)W;
-    // the three front masks start empty
-    MOEA_CUDA_TRY(cudaMemsetAsync(fmask, 0, sizeof(uint32_t) * 3 * (size_t)Wp, stream));
     void* args[] = {(void*)&rows, (void*)&Wp, (void*)&nn, (void*)&tt, (void*)&qi,
                     (void*)&blk, (void*)&fs, (void*)&fmask, (void*)&ctr};
     cudaLaunchConfig_t cfg = {};
@@ -2209,11 +2335,7 @@ int run_ndsort(Workspace& ws, const SplitPop& pop, int M, int target, int* out_f
         MOEA_CUDA_TRY(cudaLaunchKernelExC(&cfg, (const void*)nds_peel, args));
     }
 
-    // infeasible fronts in closed form (no work when the feasible points suffice)
-    nds_infeasible_heads<<<G, T, 0, stream>>>(n, qinfo, ws.counters, target, ws.head);
-    MOEA_CUDA_TRY(cub::DeviceScan::InclusiveSum(ws.cub_tmp, tmp, ws.head, ws.run_start, n, stream));
-    nds_infeasible_fronts<<<G, T, 0, stream>>>(n, qinfo, ws.run_start, ws.counters, target, ws.front_sorted);
-    nds_scatter_fronts<<<G, T, 0, stream>>>(n, perm, ws.front_sorted, fronts);
+    nds_fronts<<<kFrontCtas, kFrontThreads, 0, stream>>>(n, perm, qinfo, ws.front_sorted, ws.counters, target, fronts);
     MOEA_CUDA_TRY(cudaGetLastError());
     stage_mark("ndsort.peel", stream);
     return MOEA_OK;
