@@ -250,16 +250,9 @@ struct moea_algorithm {
     cudaGraphExec_t graph[2] = {};
     bool graph_failed = false;
     int graph_kernels = 0;
-    // small populations: the generation as the fused kernels of a one-instance group
-    bool fused_single = false;
-    BatchInst* f_inst[2] = {};
-    FusedGroup f_group;
     // snapshots (data-recorder format) and their metadata
     std::string save_dir, problem_label;
     std::unique_ptr<SnapshotWriter> recorder;
-
-    int setup_single_fused();
-    int describe_single_fused();
 
     void drop_graphs()
     {
@@ -274,10 +267,6 @@ struct moea_algorithm {
         recorder.reset();  // waits for queued snapshots
         for (auto& g : graph)
             if (g) { cudaGraphExecDestroy(g); g = nullptr; }
-        for (auto& d : f_inst)
-            if (d) { cudaFree(d); d = nullptr; }
-        fused_free_group(f_group);
-        fused_single = false;
         void* ptrs[] = {vars[0], vars[1], vars[2], objs[0], objs[1], objs[2], cv[0], cv[1], cv[2],
                         rank[0], rank[1], rank[2], cv_sort[0], cv_sort[1], bounds, parent_idx, refs,
                         refs0, gamma, ideal_last, d_gen, d_active, ps_table, cv_table, t_buf, theta,
@@ -520,7 +509,6 @@ struct moea_algorithm {
         }
         MOEA_TRY(start_population());
         initialized = true;
-        if (cfg.fused_small && fused_eligible(this)) MOEA_TRY(setup_single_fused());
         if (!save_dir.empty()) {
             std::vector<float> lo(D), hi(D);
             for (int d = 0; d < D; ++d) {
@@ -613,7 +601,6 @@ struct moea_algorithm {
         frontzero_count = 0;
         MOEA_TRY(forget_nan_rows());
         drop_graphs();  // captured generations hold the seed of their epoch
-        if (fused_single) MOEA_TRY(describe_single_fused());
         return MOEA_OK;
     }
 
@@ -653,13 +640,6 @@ struct moea_algorithm {
     // is replayed from a CUDA graph.
     int generation_body()
     {
-        if (fused_single) {
-            const BatchInst* d = f_inst[P == 0 ? 0 : 1];
-            MOEA_TRY(fused_reproduce(d, f_group, stream));
-            MOEA_TRY(fused_evaluate(d, f_group, stream));
-            MOEA_TRY(fused_ndsort(d, f_group, stream));
-            return fused_select(d, f_group, stream);
-        }
         const uint64_t s = gen_seed();
         if (cfg.mating == MOEA_MATING_CALLBACK) {
             const int rc = cfg.mate(cfg.mate_user, vars[P], objs[P], cv[P], nsga3() ? rank[P] : nullptr,
@@ -856,8 +836,6 @@ struct moea_algorithm {
         frontzero_count = 0;
         if (cfg.problem_kind == 0 && cfg.problem_reset) cfg.problem_reset(cfg.evaluate_user);
         MOEA_TRY(start_population());
-        // the draws of the new epoch use another seed
-        if (fused_single) MOEA_TRY(describe_single_fused());
         return snapshot_now();
     }
 };
@@ -1206,28 +1184,6 @@ void fused_free_group(FusedGroup& g)
 }
 
 }  // namespace
-
-// One-instance fused plan: descriptors of both parities (instance index 0).
-int moea_algorithm::describe_single_fused()
-{
-    for (int parity = 0; parity < 2; ++parity) {
-        const BatchInst h = fused_describe(this, parity == 0 ? 0 : 2, parity == 0 ? 2 : 0);
-        if (!f_inst[parity]) MOEA_CUDA_TRY(cudaMalloc((void**)&f_inst[parity], sizeof(BatchInst)));
-        MOEA_CUDA_TRY(cudaMemcpy(f_inst[parity], &h, sizeof(BatchInst), cudaMemcpyHostToDevice));
-    }
-    return MOEA_OK;
-}
-
-int moea_algorithm::setup_single_fused()
-{
-    MOEA_TRY(fused_ndsort_configure());
-    MOEA_TRY(fused_select_configure());
-    MOEA_TRY(describe_single_fused());
-    std::vector<moea_algorithm*> self{this};
-    MOEA_TRY(fused_build_group(self, {0}, f_group));
-    fused_single = true;
-    return MOEA_OK;
-}
 
 struct moea_batch {
     std::vector<moea_algorithm*> inst;
@@ -1649,7 +1605,6 @@ moea_status moea_batch_create(const moea_algorithm_config* cfgs, int count, void
         moea_algorithm_config c = cfgs[i];
         c.stream = b->stream;
         c.use_graphs = 0;
-        c.fused_small = 0;  // the batch fuses its instances itself
         moea_algorithm* a = nullptr;
         st = moea_algorithm_create(&c, &a);
         if (st != MOEA_OK) break;

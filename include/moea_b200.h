@@ -468,9 +468,9 @@ typedef struct moea_algorithm_config {
     /* initial population (N,D) row-major on the host, or NULL */
     const float* h_initial_population;
     int use_graphs;           /* capture one generation into a CUDA graph when possible */
-    int fused_small;          /* run an eligible population with 2N <= 8192 (NSGA-III, built-in
-                                 unconstrained DTLZ, fixed directions) as the fused generation:
-                                 same results, about 20 launches instead of about 80 */
+    int fused_small;          /* accepted and without effect: a population alone runs the staged
+                                 generation at every size, which is the faster one (the fused
+                                 generation serves batches); the results are the same */
     /* Snapshots in the reference's data-recorder format
      * (nat/src/algorithm/data_recorder.cu:128-292): generation 0, every
      * save_interval-th generation and the last one, under save_directory
