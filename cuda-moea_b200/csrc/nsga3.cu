@@ -250,19 +250,136 @@ __device__ __forceinline__ double warp_sum_d(double v)
     return v;
 }
 
-// Reciprocal intercepts from the extreme points s_ext (and the per-objective
-// maxima s_max for the fallback), by all threads of a block; the Jacobi
-// sweeps run in warp 0 with lane r holding row r.
+// Lanes of the Jacobi sweeps: the columns of a pair are held by a group of S
+// lanes (S = M rounded up to a power of two, lane r of the group holding row
+// r), the disjoint pairs of a round side by side: one warp up to M = 8.
 template <int M>
-__device__ __forceinline__ void norm_solve(const float* __restrict__ nds, int nds_stride,
+struct JacobiCfg {
+    static constexpr int kCols = (M + 1) & ~1;
+    static constexpr int kPairs = kCols / 2;
+    static constexpr int kS = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
+    static constexpr int kWarps = (kPairs * kS + 31) / 32;
+};
+
+template <int M>
+__device__ __forceinline__ void jacobi_sync()
+{
+    if constexpr (JacobiCfg<M>::kWarps == 1) __syncwarp();
+    else asm volatile("bar.sync 1, %0;" ::"n"(JacobiCfg<M>::kWarps * 32) : "memory");
+}
+
+// Sum over the group of S lanes: the bits of a sum over the warp whose other
+// lanes hold zeros.
+template <int S>
+__device__ __forceinline__ double group_sum_d(double v)
+{
+#pragma unroll
+    for (int o = S / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    return v;
+}
+
+// One-sided Jacobi sweeps over the columns of A (and V) by the first
+// JacobiCfg<M>::kWarps warps of a block; returns whether the matrix is
+// ill-conditioned.  Sweeps in round-robin order (circle method over P = M
+// rounded up to even columns, column P - 1 a bye when M is odd): in round r
+// column P - 1 meets column r and, for k >= 1, (r + k) mod (P - 1) meets
+// (r - k) mod (P - 1).  The pairs of a round share no column and every pair
+// comes once per sweep.  A sweep is a chain of M - 1 (or M) dependent rounds,
+// each a chain of FP64 sums, divisions and roots: sums span S lanes, the test
+// takes no root, and up to M = 8 a round has no block barrier (whole intercept
+// solve at M = 3 / 5 / 8 / 10: 14 / 29 / 41 / 20 us with a warp and two block
+// barriers per round, 10 / 17 / 30 / 15 us now).
+template <int M>
+__device__ bool jacobi_sweeps(double (&sA)[M][M], double (&sV)[M][M], double* s_norm, int* s_flag)
+{
+    using C = JacobiCfg<M>;
+    const int tid = threadIdx.x, k = tid / C::kS, row = tid % C::kS;
+    const bool in = row < M;
+    for (int sweep = 0; sweep < 60; ++sweep) {
+        // A rotation leaves its two columns with the eigenvalues of their 2x2
+        // Gram matrix, so the smallest column norm never grows and the largest
+        // never shrinks: once the current norms fail the conditioning test,
+        // the converged ones fail it too, and the fallback (which ignores the
+        // rotations) is the result.  Degenerate extreme points (repeated rows)
+        // stop here instead of rotating rounding noise for all 60 sweeps.
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int col = 2 * k + h;
+            const double x = (in && col < M) ? sA[row][col] : 0.0;
+            const double sg = sqrt(group_sum_d<C::kS>(x * x));
+            if (row == 0 && col < M) s_norm[col] = sg;
+        }
+        if (tid == 0) *s_flag = 0;
+        jacobi_sync<M>();
+        double cmax = 0.0, cmin = INFINITY;
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+            cmax = fmax(cmax, s_norm[i]);
+            cmin = fmin(cmin, s_norm[i]);
+        }
+        if (cmin < 1e-10 || cmax / cmin > 1e6) return true;  // the same in every lane
+        bool rotated = false;
+        for (int r = 0; r < C::kCols - 1; ++r) {
+            int i = (k == 0) ? r : (r + k) % (C::kCols - 1);
+            int j = (k == 0) ? C::kCols - 1 : (r - k + (C::kCols - 1)) % (C::kCols - 1);
+            if (i > j) {
+                const int tmp = i;
+                i = j;
+                j = tmp;
+            }
+            const bool pair = k < C::kPairs && j < M;  // j == M is the bye
+            const double x = (pair && in) ? sA[row][i] : 0.0;
+            const double y = (pair && in) ? sA[row][j] : 0.0;
+            const double al = group_sum_d<C::kS>(x * x);
+            const double be = group_sum_d<C::kS>(y * y);
+            const double ga = group_sum_d<C::kS>(x * y);
+            // |ga| > 1e-15 sqrt(al be), decided without the root unless it is close
+            const double ab = al * be, g2 = ga * ga, lim = 1e-30 * ab;
+            bool rot;
+            if (ab > 1e-200 && g2 > lim * (1.0 + 1e-9)) rot = pair;
+            else if (ab > 1e-200 && g2 < lim * (1.0 - 1e-9)) rot = false;
+            else rot = pair && !(ga == 0.0 || fabs(ga) <= 1e-15 * sqrt(ab));
+            if (rot) {
+                const double zeta = (be - al) / (2.0 * ga);
+                const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+                const double c = 1.0 / sqrt(1.0 + t * t);
+                const double s = c * t;
+                if (in) {
+                    sA[row][i] = c * x - s * y;
+                    sA[row][j] = s * x + c * y;
+                    const double vx = sV[row][i], vy = sV[row][j];
+                    sV[row][i] = c * vx - s * vy;
+                    sV[row][j] = s * vx + c * vy;
+                }
+            }
+            rotated |= rot;
+            jacobi_sync<M>();
+        }
+        if constexpr (C::kWarps == 1) {
+            if (!__any_sync(0xFFFFFFFFu, rotated)) break;
+        } else {
+            if (rotated) *s_flag = 1;
+            jacobi_sync<M>();
+            const int any = *s_flag;
+            jacobi_sync<M>();  // read everywhere before it is cleared
+            if (!any) break;
+        }
+    }
+    return false;
+}
+
+// Reciprocal intercepts from the extreme points s_ext (and the per-objective
+// maxima s_max for the fallback), by all threads of a block.
+template <int M>
+__device__ __forceinline__ void norm_solve(const float* nds, int nds_stride,
                                            const int* s_ext, const float* s_max,
                                            float* __restrict__ rcp_out, int* __restrict__ extreme_out,
                                            int* __restrict__ ill_out)
 {
     __shared__ double sA[M][M];
     __shared__ double sV[M][M];
-    __shared__ double s_sigma[M];
-    __shared__ int s_bad;
+    __shared__ double s_norm[M];
+    __shared__ int s_bad, s_flag;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_bad = 0;
     __syncthreads();
@@ -275,116 +392,50 @@ __device__ __forceinline__ void norm_solve(const float* __restrict__ nds, int nd
         sV[r][m] = (r == m) ? 1.0 : 0.0;
     }
     __syncthreads();
-    // Sweeps in round-robin order (circle method over P = M rounded up to
-    // even columns, column P - 1 a bye when M is odd): in round r column
-    // P - 1 meets column r and, for k >= 1, (r + k) mod (P - 1) meets
-    // (r - k) mod (P - 1).  The pairs of a round share no column, so warp k
-    // rotates pair k; every pair comes once per sweep.
-    __shared__ int s_stop, s_rot;
-    constexpr int P = (M + 1) & ~1;
-    constexpr int kPairs = P / 2;
-    int bad = s_bad;
+    if (warp >= JacobiCfg<M>::kWarps) return;
+    bool bad = s_bad != 0;
+    if (!bad) bad = jacobi_sweeps<M>(sA, sV, s_norm, &s_flag);
+    if (warp != 0) return;
+    double sigma[M], smax = 0.0, smin = INFINITY;
     if (!bad) {
-        for (int sweep = 0; sweep < 60; ++sweep) {
-            // A rotation leaves its two columns with the eigenvalues of their
-            // 2x2 Gram matrix, so the smallest column norm never grows and the
-            // largest never shrinks: once the current norms fail the
-            // conditioning test below, the converged ones fail it too, and
-            // the fallback (which ignores the rotations) is the result.
-            // Degenerate extreme points (repeated rows) stop here instead of
-            // rotating rounding noise for all 60 sweeps.
-            if (warp == 0) {
-                double cmax = 0.0, cmin = INFINITY;
-                for (int i = 0; i < M; ++i) {
-                    const double x = (lane < M) ? sA[lane][i] : 0.0;
-                    const double sg = sqrt(warp_sum_d(x * x));
-                    cmax = fmax(cmax, sg);
-                    cmin = fmin(cmin, sg);
-                }
-                if (lane == 0) {
-                    s_stop = (cmin < 1e-10 || cmax / cmin > 1e6) ? 1 : 0;
-                    s_rot = 0;
-                }
-            }
-            __syncthreads();
-            if (s_stop) {  // uniform over the block
-                bad = 1;
-                break;
-            }
-            for (int r = 0; r < P - 1; ++r) {
-                if (warp < kPairs) {
-                    int i = (warp == 0) ? r : (r + warp) % (P - 1);
-                    int j = (warp == 0) ? P - 1 : (r - warp + (P - 1)) % (P - 1);
-                    if (i > j) {
-                        const int tmp = i;
-                        i = j;
-                        j = tmp;
-                    }
-                    if (j < M) {  // j == M is the bye
-                        const double x = (lane < M) ? sA[lane][i] : 0.0;
-                        const double y = (lane < M) ? sA[lane][j] : 0.0;
-                        const double al = warp_sum_d(x * x);
-                        const double be = warp_sum_d(y * y);
-                        const double ga = warp_sum_d(x * y);
-                        if (!(ga == 0.0 || fabs(ga) <= 1e-15 * sqrt(al * be))) {
-                            const double zeta = (be - al) / (2.0 * ga);
-                            const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-                            const double c = 1.0 / sqrt(1.0 + t * t);
-                            const double s = c * t;
-                            if (lane < M) {
-                                sA[lane][i] = c * x - s * y;
-                                sA[lane][j] = s * x + c * y;
-                                const double vx = sV[lane][i], vy = sV[lane][j];
-                                sV[lane][i] = c * vx - s * vy;
-                                sV[lane][j] = s * vx + c * vy;
-                            }
-                            if (lane == 0) s_rot = 1;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-            const int rotated = s_rot;
-            __syncthreads();  // every thread read s_rot before warp 0 clears it
-            if (!rotated) break;
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+            const double x = (lane < M) ? sA[lane][i] : 0.0;
+            sigma[i] = sqrt(warp_sum_d(x * x));
         }
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+            if (!isfinite(sigma[i])) bad = true;
+            smax = fmax(smax, sigma[i]);
+            smin = fmin(smin, sigma[i]);
+        }
+        if (smin < 1e-10 || smax / smin > 1e6) bad = true;
     }
-    if (warp == 0) {
-        {
-            double smax = 0.0, smin = INFINITY;
-            for (int i = 0; i < M && !bad; ++i) {
-                const double x = (lane < M) ? sA[lane][i] : 0.0;
-                const double sg = sqrt(warp_sum_d(x * x));
-                if (lane == 0) s_sigma[i] = sg;
-                if (!isfinite(sg)) bad = 1;
-                smax = fmax(smax, sg);
-                smin = fmin(smin, sg);
-            }
-            if (smin < 1e-10 || smax / smin > 1e6) bad = 1;
+    float r = 1.0f;
+    if (!bad) {
+        // lane i: the coefficient of column i
+        double sg = 1.0, ut1 = 0.0, acc = 0.0;
+#pragma unroll
+        for (int i = 0; i < M; ++i) sg = (lane == i) ? sigma[i] : sg;
+        if (lane < M)
+            for (int k = 0; k < M; ++k) ut1 += sA[k][lane];
+        const double mine = (sg > 1e-5) ? ut1 / (sg * sg) : 0.0;
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+            const double coef = __shfl_sync(0xFFFFFFFFu, mine, i);
+            if (lane < M) acc += sV[lane][i] * coef;
         }
-        __syncwarp();
-        float r = 1.0f;
-        if (lane < M) {
-            if (!bad) {
-                double acc = 0.0;
-                for (int i = 0; i < M; ++i) {
-                    double ut1 = 0.0;
-                    for (int k = 0; k < M; ++k) ut1 += sA[k][i];
-                    const double sg = s_sigma[i];
-                    const double coef = (sg > 1e-5) ? ut1 / (sg * sg) : 0.0;
-                    acc += sV[lane][i] * coef;
-                }
-                r = (float)acc;
-            } else {
-                const float mx = s_max[lane];
-                r = (mx > 1e-10f) ? 1.0f / fmaxf(mx, 1e-6f) : 1.0f;
-            }
-            if (!isfinite(r) || r <= 0.0f) r = 1.0f;
-            rcp_out[lane] = r;
-            if (extreme_out) extreme_out[lane] = s_ext[lane];
-        }
-        if (lane == 0 && ill_out) *ill_out = bad;
+        r = (float)acc;
+    } else if (lane < M) {
+        const float mx = s_max[lane];
+        r = (mx > 1e-10f) ? 1.0f / fmaxf(mx, 1e-6f) : 1.0f;
     }
+    if (lane < M) {
+        if (!isfinite(r) || r <= 0.0f) r = 1.0f;
+        rcp_out[lane] = r;
+        if (extreme_out) extreme_out[lane] = s_ext[lane];
+    }
+    if (lane == 0 && ill_out) *ill_out = bad;
 }
 
 // Intercepts from the extreme points: one-sided Jacobi SVD in FP64 of the
