@@ -130,7 +130,7 @@ int workspace_init(Workspace& ws, int device, int n_max, int m_max, int h_max)
     A(ws.rank, n); A(ws.selected, n); A(ws.flags, n);
     A(ws.offset_dev, 1);
     A(ws.dir_delta, 1);
-    A(ws.scalar_d, 1);
+    A(ws.scalar_d, 2);
 #undef A
     if (st == MOEA_OK) {
         ws.niche_last = ws.rho + h_max;

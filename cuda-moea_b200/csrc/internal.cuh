@@ -136,7 +136,7 @@ struct Workspace {
     float* tc_dirs = nullptr;       // tiles of 128 directions in the MMA's shared-memory image,
                                     // then one float: max | |r|^2 - 1 | of the directions
     unsigned* tc_rowmax = nullptr;  // (n_max) largest |x.r_j| estimate per point (FP32 bits)
-    double* scalar_d = nullptr;     // (1) FP64 result word (IGD mean)
+    double* scalar_d = nullptr;     // (2) FP64 result words (IGD mean and row count)
 
     // --- CUB temporary storage ---
     void* cub_tmp = nullptr;

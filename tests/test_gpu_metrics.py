@@ -69,3 +69,29 @@ def test_igd_equals_reference_metric_on_golden_cases():
         ref = metrics.pareto_front_points("DTLZ2", c["objectives"], c["front_count"], 2887).to(torch.float64)
         got = metrics.igd(x, ref, filter_nondominated=c["filter_nondominated"])
         assert abs(got - c["igd"]) <= 1e-12 * abs(c["igd"]), (c, got)
+
+
+@pytest.mark.parametrize("M,n,r", [(1, 1, 1), (2, 127, 513), (3, 129, 1), (4, 2049, 4097), (5, 8192, 300),
+                                   (9, 1000, 129), (16, 130, 700), (3, 8193, 5000)])
+@pytest.mark.parametrize("filt", [True, False])
+def test_igd_ranges_and_filters_at_their_edges(M, n, r, filt):
+    """Tiles, row ranges and points per thread at their remainders, and both
+    filters (pairs up to 8192 rows, the sort above): relative 1e-12, the bound
+    of an FP64 mean of r distances of 16 terms each."""
+    from cuda_moea import metrics
+    rng = np.random.default_rng(1000 * M + n)
+    approx = (1.0 + rng.integers(0, 40, (n, M)) / 40.0).astype(np.float32)   # ties and duplicates
+    if n > 100:
+        approx[5, 0] = np.inf
+        approx[6, M - 1] = -np.inf
+        approx[7, M // 2] = np.nan
+    ref = rng.random((r, M))
+    got = metrics.igd(torch.from_numpy(approx).cuda(), torch.from_numpy(ref), filter_nondominated=filt)
+    finite = approx[np.isfinite(approx).all(1)].astype(np.float64)
+    if filt:
+        rows = np.unique(finite, axis=0)
+        keep = [not ((rows <= q).all(1) & (rows < q).any(1)).any() for q in rows]
+        finite = rows[keep]
+    d = np.concatenate([np.sqrt(((q[:, None, :] - finite[None]) ** 2).sum(2)).min(1)
+                        for q in np.array_split(ref, max(1, r * len(finite) * M // 50_000_000))])
+    assert abs(got - d.mean()) <= 1e-12 * max(1.0, abs(d.mean()))
