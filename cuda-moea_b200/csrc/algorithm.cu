@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "offspring.cuh"
 #include "snapshot.h"
 
 namespace moea {
@@ -636,18 +637,53 @@ struct moea_algorithm {
         return nan_rows ? run_fill_int(nan_rows, 3, N, stream) : MOEA_OK;
     }
 
-    // Reproduction, evaluation and selection of one generation: the part that
-    // is replayed from a CUDA graph.
-    int generation_body()
+    // Mating, variation and evaluation of one generation.
+    int reproduce_evaluate()
     {
         const uint64_t s = gen_seed();
+        const bool tournament = cfg.mating == MOEA_MATING_TOURNAMENT;
+        if (cfg.mating != MOEA_MATING_CALLBACK && offspring_eligible(cfg.problem_kind, D, M)) {
+            OffspringArgs a{};
+            a.parents = vars[P];
+            a.cv = cv[P];
+            a.rank = tournament ? rank[P] : nullptr;
+            a.d_active = nsga3() ? nullptr : d_active;
+            a.active = N;
+            a.bounds = bounds;
+            a.off = vars[O];
+            a.pidx = parent_idx;
+            a.objs = objs[O];
+            a.cv_out = cv[O];
+            a.cv_table = constrained() ? cv_table : nullptr;
+            a.n_off = N;
+            a.D = D;
+            a.M = M;
+            a.kind = cfg.problem_kind;
+            a.mutate = cfg.mutation;
+            a.total = T;
+            a.sbx_eta0 = cfg.sbx_eta_initial;
+            a.sbx_eta1 = cfg.sbx_eta_final;
+            a.sbx_prob = cfg.sbx_probability;
+            a.copy_prob = cfg.sbx_copy_probability;
+            a.pm_eta0 = cfg.pm_eta_initial;
+            a.pm_eta1 = cfg.pm_eta_final;
+            a.pm_prob = cfg.pm_probability;
+            a.seed = s;
+            a.d_gen = d_gen;
+            MOEA_TRY(run_offspring(a, stream));
+            if (cfg.problem_kind == 0) {
+                stage_mark("variation", stream);
+                MOEA_TRY(evaluate(O, generation));
+            }
+            stage_mark("evaluate", stream);
+            return MOEA_OK;
+        }
         if (cfg.mating == MOEA_MATING_CALLBACK) {
             const int rc = cfg.mate(cfg.mate_user, vars[P], objs[P], cv[P], nsga3() ? rank[P] : nullptr,
                                     nsga3() ? N : active_count_sync(), parent_idx, N, D, M, generation,
                                     (void*)stream);
             if (rc != 0) return set_error(MOEA_ERR_CALLBACK, "mating callback failed (%d)", rc);
         } else {
-            const bool tournament = cfg.mating == MOEA_MATING_TOURNAMENT;
             MOEA_TRY(run_mating(cv[P], tournament ? rank[P] : nullptr, nsga3() ? nullptr : d_active, N, N,
                                 s, d_gen, 0, parent_idx, stream));
         }
@@ -665,6 +701,14 @@ struct moea_algorithm {
                 zero_cv_if_inactive<<<ceil_div(N, 256), 256, 0, stream>>>(cv[O], N, cv_table, d_gen);
         }
         stage_mark("evaluate", stream);
+        return MOEA_OK;
+    }
+
+    // Reproduction, evaluation and selection of one generation: the part that
+    // is replayed from a CUDA graph.
+    int generation_body()
+    {
+        MOEA_TRY(reproduce_evaluate());
         SplitPop pop{objs[P], objs[O], cv[P], cv[O], N, N, N, 2 * N};
         if (nsga3()) {
             SplitPop sort_pop = pop;
@@ -1346,7 +1390,6 @@ struct moea_batch {
             if (st != MOEA_OK) break;
             cudaEventRecord(e0, stream);
             st = fused_reproduce(d_inst[parity], g, stream);
-            if (st == MOEA_OK) st = fused_evaluate(d_inst[parity], g, stream);
             if (st == MOEA_OK) st = fused_ndsort(d_inst[parity], g, stream);
             if (st == MOEA_OK) st = fused_select(d_inst[parity], g, stream);
             cudaEventRecord(e1, stream);
@@ -1452,7 +1495,6 @@ struct moea_batch {
             cudaStream_t gs = gstream[gi];
             MOEA_CUDA_TRY(cudaStreamWaitEvent(gs, fork, 0));
             MOEA_TRY(fused_reproduce(d, g, gs));
-            MOEA_TRY(fused_evaluate(d, g, gs));
             MOEA_TRY(fused_ndsort(d, g, gs));
             MOEA_TRY(fused_select(d, g, gs));
             MOEA_CUDA_TRY(cudaEventRecord(gjoin[gi], gs));

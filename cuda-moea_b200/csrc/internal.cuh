@@ -308,7 +308,6 @@ struct FusedGroup {
 };
 
 int fused_reproduce(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s);
-int fused_evaluate(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s);
 int fused_ndsort(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s);
 int fused_select(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s);
 int fused_tile_blocks(int M, int n, int shape);  // tile CTAs of one instance in a tile shape (0, 1)
