@@ -1162,7 +1162,6 @@ BatchInst fused_describe(moea_algorithm* a, int P, int X)
     b.front_list = w.front_list; b.counters = w.counters; b.rows = w.rows; b.chunk_keys = w.chunk_keys;
     b.chunk_bits = w.chunk_bits; b.fronts = w.fronts; b.nds_gidx = w.nds_gidx; b.sizes = w.sizes;
     b.nds_objs = w.nds_objs; b.rcp_b = w.rcp_b; b.extreme = w.extreme; b.assoc_idx = w.assoc_idx;
-    b.assoc_best = w.assoc_best;
     b.assoc_dist = w.assoc_dist; b.rho = w.rho; b.selected = w.selected; b.flags = w.flags;
     b.survivors = a->survivors; b.offset = w.offset_dev;
     b.t_dirs_orig = a->refs;

@@ -282,7 +282,6 @@ struct BatchInst {
     uint32_t* rows; uint32_t* chunk_keys; uint32_t* chunk_bits;
     int* fronts; int* nds_gidx; int* sizes; float* nds_objs; float* rcp_b; int* extreme;
     int* assoc_idx; float* assoc_dist; int* rho; int* selected; int* flags; int* survivors;
-    unsigned long long* assoc_best;  // packed (d2 bits, index) minima of a direction-split scan
     unsigned long long* offset;
     const float* t_dirs_orig;  // (M, H) directions in their own order
     const float* t_dirs; const int* t_order; const float* t_center; const float* t_cos;

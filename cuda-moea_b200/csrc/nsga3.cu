@@ -17,6 +17,7 @@
 
 #include <cooperative_groups.h>
 
+#include "assoc_dense.cuh"
 #include "internal.cuh"
 #include "niche_select.cuh"
 #include "dirtree.h"
@@ -792,33 +793,25 @@ int dispatch_norm(Workspace& ws, const SplitPop& pop, const int* gidx, const int
 // ---------------------------------------------------------------------------
 // association
 // ---------------------------------------------------------------------------
-//
-// For unit directions r_j the perpendicular distance satisfies
-// d2_j = |x|^2 - (x.r_j)^2 up to rounding, so the reference argmin is found
-// among the directions whose dot^2 lies within a rounding margin of the
-// largest dot^2.  Each thread keeps a running max of dot^2 and evaluates the
-// reference's FP32 formula (association.cu:139-170: fmaf dot, contracted
-// residual, fmaf sum of squares) only for those candidates.  Ties keep the
-// smaller index within a thread (ascending j, strict <) and across direction
-// splits through a packed (d2 bits, j) atomicMin, so the result equals the
-// reference argmin exactly.  Margin: |d2_fp32(j) - (|x|^2 - dot_j^2)| is bounded
-// by about (4M+5) eps |x|^2; the kernel uses (16M+64) eps |x|^2.
+// The searches share one rule: the reference's argmin lies among the directions
+// whose dot^2 comes within a rounding margin of the largest (assoc_margin).
+// assoc_dense.cu visits every direction; the cone tree below skips most of a
+// large set; assoc_tc.cu forms the dots on the tensor cores.
 
-constexpr int kAssocThreads = 256;
-constexpr int kAssocTile = 1024;
-
-template <int M>
-struct DirTile {
-    static constexpr int kLen = (M <= 4) ? kAssocTile : 512;  // directions per smem tile
-};
-
-// delta = max_j | |r_j|^2 - 1 | in FP64, rounded up to FP32 (one block).
-__global__ void dir_delta_kernel(const float* __restrict__ refs, int M, int H, float* __restrict__ out)
+// delta = max_j | |r_j|^2 - 1 | in FP64, rounded up to FP32: one 8-CTA cluster
+// (one CTA took 11 us for 10,626 directions of five objectives).
+constexpr int kDeltaCtas = 8, kDeltaThreads = 512;
+__global__ void __cluster_dims__(kDeltaCtas, 1, 1) __launch_bounds__(kDeltaThreads)
+dir_delta_kernel(const float* __restrict__ refs, int M, int H, float* __restrict__ out)
 {
-    __shared__ double s_max[32];
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ double s_warp[kDeltaThreads / 32];
+    __shared__ double s_max[kDeltaCtas];
+    const int c = (int)cluster.block_rank(), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double d = 0.0;
-    for (int j = threadIdx.x; j < H; j += blockDim.x) {
+    for (int j = c * kDeltaThreads + threadIdx.x; j < H; j += kDeltaCtas * kDeltaThreads) {
         double rr = 0.0;
+#pragma unroll 8
         for (int m = 0; m < M; ++m) {
             const double v = refs[(size_t)m * H + j];
             rr += v * v;
@@ -827,126 +820,18 @@ __global__ void dir_delta_kernel(const float* __restrict__ refs, int M, int H, f
         d = (e == e) ? fmax(d, e) : INFINITY;
     }
     for (int o = 16; o; o >>= 1) d = fmax(d, __shfl_xor_sync(0xffffffffu, d, o));
-    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = d;
+    if (lane == 0) s_warp[warp] = d;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        d = threadIdx.x < (blockDim.x >> 5) ? s_max[threadIdx.x] : 0.0;
+    if (warp == 0) {
+        d = lane < kDeltaThreads / 32 ? s_warp[lane] : 0.0;
         for (int o = 16; o; o >>= 1) d = fmax(d, __shfl_xor_sync(0xffffffffu, d, o));
-        if (threadIdx.x == 0) out[0] = __double2float_ru(fmin(d, 1e30));
+        if (lane == 0) cluster.map_shared_rank(s_max, 0)[c] = d;
     }
-}
-
-// One block of points (bx) against one range of directions (by).  With
-// best_out the packed (d2, index) minimum is merged atomically across ranges;
-// without it the block covers every direction and writes idx/dist directly.
-template <int M>
-__device__ __forceinline__ void assoc_scan_block(int bx, int by, const float* __restrict__ x, int x_stride,
-                                                 const float* __restrict__ scale,
-                                                 const float* __restrict__ refs, int H, int n, int split_len,
-                                                 float delta, unsigned long long* __restrict__ best_out,
-                                                 int* __restrict__ idx_out, float* __restrict__ dist_out)
-{
-    constexpr int TL = DirTile<M>::kLen;
-    __shared__ __align__(16) float s_dir[TL * ((M <= 4) ? 4 : M)];
-    const int i = bx * kAssocThreads + threadIdx.x;
-    const int j_begin = by * split_len;
-    const int j_end = min(H, j_begin + split_len);
-    if (bx * kAssocThreads >= n || j_begin >= j_end) return;
-    const bool valid = i < n;
-    float xr[M];
-    float xx = 0.0f;
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-        float v = valid ? x[(size_t)m * x_stride + i] : 0.0f;
-        if (scale) v = v * scale[m];
-        xr[m] = v;
-        xx = fmaf(v, v, xx);
+    cluster.sync();  // CTA 0 holds every CTA's maximum
+    if (c == 0 && threadIdx.x == 0) {
+        for (int r = 0; r < kDeltaCtas; ++r) d = fmax(d, s_max[r]);
+        out[0] = __double2float_ru(fmin(d, 1e30));
     }
-    const float margin = assoc_margin(M, xx, delta);
-    // coarse pre-pass over a strided subset to start with a tight threshold
-    float maxd = -INFINITY;
-    for (int j = j_begin; j < j_end; j += 61) {
-        float dot = 0.0f;
-#pragma unroll
-        for (int m = 0; m < M; ++m) dot = fmaf(xr[m], __ldg(refs + (size_t)m * H + j), dot);
-        maxd = fmaxf(maxd, dot * dot);
-    }
-    float thr = maxd - margin;
-    if (!(thr == thr)) thr = -INFINITY;
-    float best = INFINITY;
-    int bj = -1;
-    for (int t0 = j_begin; t0 < j_end; t0 += TL) {
-        const int cnt = min(TL, j_end - t0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < cnt; t += kAssocThreads) {
-            if (M <= 4) {
-                float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
-                d.x = refs[t0 + t];
-                if (M > 1) d.y = refs[(size_t)H + t0 + t];
-                if (M > 2) d.z = refs[(size_t)2 * H + t0 + t];
-                if (M > 3) d.w = refs[(size_t)3 * H + t0 + t];
-                reinterpret_cast<float4*>(s_dir)[t] = d;
-            } else {
-#pragma unroll
-                for (int m = 0; m < M; ++m) s_dir[(size_t)m * TL + t] = refs[(size_t)m * H + t0 + t];
-            }
-        }
-        __syncthreads();
-        if (!valid) continue;
-#pragma unroll 4
-        for (int t = 0; t < cnt; ++t) {
-            float r[M];
-            if (M <= 4) {
-                const float4 d = reinterpret_cast<const float4*>(s_dir)[t];
-                r[0] = d.x;
-                if (M > 1) r[1 % M] = d.y;
-                if (M > 2) r[2 % M] = d.z;
-                if (M > 3) r[3 % M] = d.w;
-            } else {
-#pragma unroll
-                for (int m = 0; m < M; ++m) r[m] = s_dir[(size_t)m * TL + t];
-            }
-            float dot = 0.0f;
-#pragma unroll
-            for (int m = 0; m < M; ++m) dot = fmaf(xr[m], r[m], dot);
-            const float dd = dot * dot;
-            if (dd >= thr) {
-                float d2 = 0.0f;
-#pragma unroll
-                for (int m = 0; m < M; ++m) {
-                    const float res = fmaf(-dot, r[m], xr[m]);
-                    d2 = fmaf(res, res, d2);
-                }
-                if (d2 < best) { best = d2; bj = t0 + t; }
-                if (dd > maxd) {
-                    maxd = dd;
-                    const float nt = maxd - margin;
-                    thr = (nt == nt) ? nt : -INFINITY;
-                }
-            }
-        }
-    }
-    if (best_out) {
-        if (valid && best < INFINITY) {
-            const unsigned long long packed =
-                ((unsigned long long)__float_as_uint(best) << 32) | (unsigned)bj;
-            atomicMin(best_out + i, packed);
-        }
-    } else if (valid) {
-        const bool found = best < INFINITY;
-        idx_out[i] = found ? bj : -1;
-        dist_out[i] = found ? sqrtf(best) : INFINITY;
-    }
-}
-
-template <int M>
-__global__ void __launch_bounds__(kAssocThreads)
-assoc_plain(const float* __restrict__ x, int x_stride, const float* __restrict__ scale,
-            const float* __restrict__ refs, int H, const int* __restrict__ d_n, int split_len,
-            const float* __restrict__ d_delta, unsigned long long* __restrict__ best_out)
-{
-    assoc_scan_block<M>(blockIdx.x, blockIdx.y, x, x_stride, scale, refs, H, *d_n, split_len, *d_delta, best_out,
-                        nullptr, nullptr);
 }
 
 __global__ void assoc_reset(unsigned long long* best, int n_cap)
@@ -970,31 +855,16 @@ __global__ void assoc_finish(const unsigned long long* __restrict__ best, const 
     }
 }
 
-template <int M>
-void launch_assoc(const float* x, int x_stride, const float* scale, const float* refs, int H,
-                  const int* d_n, int n_cap, const float* d_delta, unsigned long long* best, int sms,
-                  cudaStream_t stream)
-{
-    const int pb = ceil_div(n_cap, kAssocThreads);
-    int splits = ceil_div(8LL * sms, pb);
-    const int max_splits = ceil_div(H, kAssocTile);
-    if (splits > max_splits) splits = max_splits;
-    if (splits < 1) splits = 1;
-    const int split_len = ceil_div(H, splits);
-    assoc_plain<M><<<dim3(pb, splits), kAssocThreads, 0, stream>>>(x, x_stride, scale, refs, H, d_n,
-                                                                   split_len, d_delta, best);
-}
-
 // ---- cone-tree search ------------------------------------------------------
 //
 // One warp per point.  The directions sit in the leaves of a 32-ary cone tree
 // (at most 32 per leaf, children of a node contiguous).  The warp keeps the
-// same running state as the scan kernel -- the largest dot^2 seen (maxd), the
-// threshold thr = maxd - margin, and the best packed (d2 bits, index) -- and
+// running state of a scan -- the largest dot^2 seen (maxd), the threshold
+// thr = maxd - margin, and the best packed (d2 bits, index) -- and
 // visits children best first (largest projection on the cone axis).  A
 // subtree is skipped when a bound on the FP32 dot^2 of every member lies
-// below thr: such members are never candidates in the scan kernel either,
-// and skipping them cannot change maxd.  Ties are resolved by the packed
+// below thr: such members are never candidates of a scan either, and skipping
+// them cannot change maxd.  Ties are resolved by the packed
 // minimum on the original index, so the result equals the reference argmin.
 //
 // Bound for a cone with axis c and half angle rho: the angle between x and a
@@ -1008,9 +878,24 @@ void launch_assoc(const float* x, int x_stride, const float* scale, const float*
 constexpr int kTreeWarps = 8;
 constexpr int kTreeMaxDepth = kDirTreeMaxDepth;
 // Above this many objectives the cones prune little: the tensor-core search
-// (large problems) or one thread per point over all directions is cheaper
-// than one warp per point over the tree.
+// (large problems) or the dense one is cheaper than a warp per point over the
+// tree.
 constexpr int kTreeMaxObjectives = 5;
+// Whether the dense search is the faster one at or below that many objectives.
+// The tree takes 2-3 ns per point whatever the directions when points fill the
+// device and a few microseconds when they do not; the dense search H (M + 1)
+// instructions per point.  Up to three objectives the tree prunes well, so the
+// dense search wins with many points and few directions only (N=32768: 1,891
+// directions 78 -> 33 us, 4,005 78 -> 53, 8,128 even; N=4096, 4,005 directions
+// 20 -> 23 us).  At four and five it wins up to about 8,192 directions (M=5:
+// N=3002, 2,380 directions 49 -> 20 us; N=8192, 5,985 directions 100 -> 49).
+inline bool dense_preferred(int M, int n_cap, int H)
+{
+    return M <= 3 ? 16ll * H <= n_cap : H <= 8192;
+}
+// In a batch the instances fill the device together (85 instances a launch:
+// M=3 295 -> 150 us, M=5 783 -> 216 us).
+inline bool dense_preferred_batch(int max_h) { return max_h <= 8192; }
 
 struct TreeArgs {
     const float* dirs;    // (M, H) in tree order
@@ -1265,16 +1150,6 @@ __global__ void gather_fronts(const int* __restrict__ surv, int N, const int* __
     if (i < N) out[i] = fronts[surv[i]];
 }
 
-int sm_count(int device)
-{
-    static int cached[64] = {0};
-    if (device >= 0 && device < 64 && cached[device]) return cached[device];
-    int s = 148;
-    cudaDeviceGetAttribute(&s, cudaDevAttrMultiProcessorCount, device);
-    if (device >= 0 && device < 64) cached[device] = s;
-    return s;
-}
-
 // ---------------------------------------------------------------------------
 // fused batch: selection stages of every instance, one launch per stage
 // ---------------------------------------------------------------------------
@@ -1416,53 +1291,6 @@ fused_prep(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
     }
     __syncthreads();
     norm_solve<M>(I.nds_objs, I.n_max, s_ext, s_max, I.rcp_b, I.extreme, nullptr);
-}
-
-template <int M>
-__global__ void __launch_bounds__(kAssocThreads)
-fused_scan(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
-{
-    const BatchInst& I = insts[ids[blockIdx.y]];
-    assoc_scan_block<M>(blockIdx.x, 0, I.nds_objs, I.n_max, I.rcp_b, I.t_dirs_orig, I.H, I.sizes[3], I.H,
-                        I.t_delta, nullptr, I.assoc_idx, I.assoc_dist);
-}
-
-// The same scan with the directions split into `splits` ranges (blockIdx.z),
-// merged through the packed (d2 bits, index) minimum as in the staged path;
-// fused_scan_reset before it, fused_scan_finish after.  An instance's scan
-// then runs on `splits` times the CTAs: within one fused generation the
-// instances of a group run side by side and each stage lasts as long as its
-// slowest instance, so the long scans of the many-direction instances are
-// split rather than run by one thread per point over every direction.
-template <int M>
-__global__ void __launch_bounds__(kAssocThreads)
-fused_scan_split(const BatchInst* __restrict__ insts, const int* __restrict__ ids, int splits)
-{
-    const BatchInst& I = insts[ids[blockIdx.y]];
-    assoc_scan_block<M>(blockIdx.x, blockIdx.z, I.nds_objs, I.n_max, I.rcp_b, I.t_dirs_orig, I.H, I.sizes[3],
-                        (I.H + splits - 1) / splits, I.t_delta, I.assoc_best, nullptr, nullptr);
-}
-
-__global__ void fused_scan_reset(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
-{
-    const BatchInst& I = insts[ids[blockIdx.y]];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < I.sizes[3]) I.assoc_best[i] = ~0ull;
-}
-
-__global__ void fused_scan_finish(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
-{
-    const BatchInst& I = insts[ids[blockIdx.y]];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= I.sizes[3]) return;
-    const unsigned long long b = I.assoc_best[i];
-    if (b == ~0ull) {
-        I.assoc_idx[i] = -1;
-        I.assoc_dist[i] = INFINITY;
-    } else {
-        I.assoc_idx[i] = (int)(unsigned)(b & 0xFFFFFFFFull);
-        I.assoc_dist[i] = sqrtf(__uint_as_float((unsigned)(b >> 32)));
-    }
 }
 
 template <int M>
@@ -1812,7 +1640,7 @@ bool tensor_preferred(int M, int n_cap, int H)
 
 int run_dir_delta(const float* refs, int M, int H, float* out, cudaStream_t stream)
 {
-    dir_delta_kernel<<<1, 1024, 0, stream>>>(refs, M, H, out);
+    dir_delta_kernel<<<kDeltaCtas, kDeltaThreads, 0, stream>>>(refs, M, H, out);
     MOEA_CUDA_TRY(cudaGetLastError());
     return MOEA_OK;
 }
@@ -1848,16 +1676,14 @@ int run_associate(Workspace& ws, const float* x, int x_stride, const float* scal
     if (mode == MOEA_ASSOC_TREE) {
         if (!direction_tree_ready(ws, refs, M, H))
             return set_error(MOEA_ERR_STATE, "associate: no cone tree prepared for these directions");
-        if (ws.tree_depth <= kTreeMaxDepth && M <= kTreeMaxObjectives) {
+        if (ws.tree_depth <= kTreeMaxDepth && M <= kTreeMaxObjectives && !dense_preferred(M, n_cap, H)) {
             const TreeArgs t{ws.tree_dirs, ws.tree_order, ws.tree_center, ws.tree_cos, ws.tree_sin,
                              ws.tree_link, H, ws.tree_nodes, ws.tree_delta};
             const int blocks = ceil_div(n_cap, kTreeWarps);
             switch (M) {
 #define MOEA_TREE_CASE(K) case K: assoc_tree<K><<<blocks, kTreeWarps * 32, 0, stream>>>(x, x_stride, scale, t, d_n, idx, dist); break;
             MOEA_TREE_CASE(1) MOEA_TREE_CASE(2) MOEA_TREE_CASE(3) MOEA_TREE_CASE(4)
-            MOEA_TREE_CASE(5) MOEA_TREE_CASE(6) MOEA_TREE_CASE(7) MOEA_TREE_CASE(8)
-            MOEA_TREE_CASE(9) MOEA_TREE_CASE(10) MOEA_TREE_CASE(11) MOEA_TREE_CASE(12)
-            MOEA_TREE_CASE(13) MOEA_TREE_CASE(14) MOEA_TREE_CASE(15) MOEA_TREE_CASE(16)
+            MOEA_TREE_CASE(5)
 #undef MOEA_TREE_CASE
             default: return set_error(MOEA_ERR_UNSUPPORTED, "associate: M=%d", M);
             }
@@ -1865,52 +1691,24 @@ int run_associate(Workspace& ws, const float* x, int x_stride, const float* scal
             return MOEA_OK;
         }
         // many objectives: the tensor-core search where it was prepared (the
-        // cones prune little), else -- and for a tree deeper than the
-        // kernel's stack -- the scan
+        // cones prune little), else -- and for few directions and a tree deeper
+        // than the kernel's stack -- the dense search
         if (tensor_preferred(M, n_cap, H) && tensor_directions_ready(ws, refs, M, H))
             return run_associate_tensor(ws, x, x_stride, scale, refs, M, d_n, n_cap, H, idx, dist, stream);
+        return run_assoc_dense(x, x_stride, scale, refs, M, d_n, n_cap, H, ws.tree_delta, nullptr, idx, dist, stream);
     }
-    dir_delta_kernel<<<1, 1024, 0, stream>>>(refs, M, H, ws.dir_delta);
-    assoc_reset<<<ceil_div(n_cap, 256), 256, 0, stream>>>(ws.assoc_best, n_cap);
-    const int sms = sm_count(ws.device);
-    switch (M) {
-#define MOEA_ASSOC_CASE(K) case K: launch_assoc<K>(x, x_stride, scale, refs, H, d_n, n_cap, ws.dir_delta, ws.assoc_best, sms, stream); break;
-    MOEA_ASSOC_CASE(1) MOEA_ASSOC_CASE(2) MOEA_ASSOC_CASE(3) MOEA_ASSOC_CASE(4)
-    MOEA_ASSOC_CASE(5) MOEA_ASSOC_CASE(6) MOEA_ASSOC_CASE(7) MOEA_ASSOC_CASE(8)
-    MOEA_ASSOC_CASE(9) MOEA_ASSOC_CASE(10) MOEA_ASSOC_CASE(11) MOEA_ASSOC_CASE(12)
-    MOEA_ASSOC_CASE(13) MOEA_ASSOC_CASE(14) MOEA_ASSOC_CASE(15) MOEA_ASSOC_CASE(16)
-#undef MOEA_ASSOC_CASE
-    default: return set_error(MOEA_ERR_UNSUPPORTED, "associate: M=%d", M);
-    }
-    MOEA_CUDA_TRY(cudaGetLastError());
-    assoc_finish<<<ceil_div(n_cap, 256), 256, 0, stream>>>(ws.assoc_best, d_n, idx, dist);
-    MOEA_CUDA_TRY(cudaGetLastError());
-    return MOEA_OK;
+    MOEA_TRY(run_dir_delta(refs, M, H, ws.dir_delta, stream));
+    return run_assoc_dense(x, x_stride, scale, refs, M, d_n, n_cap, H, 0.0f, ws.dir_delta, idx, dist, stream);
 }
 
 // The full-scan association with caller-provided scratch instead of a
-// workspace: best (n_cap packed minima), delta (1 float), d_n (device count).
-// Used by the allocation-free entry point (noalloc.cu).
-int run_associate_scan_scratch(const float* x, const float* refs, int M, const int* d_n, int n_cap,
-                               int H, int* idx, float* dist, unsigned long long* best, float* delta,
-                               int device, cudaStream_t stream)
+// workspace: delta (1 float), d_n (device count).  Used by the allocation-free
+// entry point (noalloc.cu).
+int run_associate_scan_scratch(const float* x, const float* refs, int M, const int* d_n, int n_cap, int H, int* idx,
+                               float* dist, float* delta, cudaStream_t stream)
 {
-    dir_delta_kernel<<<1, 1024, 0, stream>>>(refs, M, H, delta);
-    assoc_reset<<<ceil_div(n_cap, 256), 256, 0, stream>>>(best, n_cap);
-    const int sms = sm_count(device);
-    switch (M) {
-#define MOEA_SCRATCH_CASE(K) case K: launch_assoc<K>(x, n_cap, nullptr, refs, H, d_n, n_cap, delta, best, sms, stream); break;
-    MOEA_SCRATCH_CASE(1) MOEA_SCRATCH_CASE(2) MOEA_SCRATCH_CASE(3) MOEA_SCRATCH_CASE(4)
-    MOEA_SCRATCH_CASE(5) MOEA_SCRATCH_CASE(6) MOEA_SCRATCH_CASE(7) MOEA_SCRATCH_CASE(8)
-    MOEA_SCRATCH_CASE(9) MOEA_SCRATCH_CASE(10) MOEA_SCRATCH_CASE(11) MOEA_SCRATCH_CASE(12)
-    MOEA_SCRATCH_CASE(13) MOEA_SCRATCH_CASE(14) MOEA_SCRATCH_CASE(15) MOEA_SCRATCH_CASE(16)
-#undef MOEA_SCRATCH_CASE
-    default: return set_error(MOEA_ERR_UNSUPPORTED, "associate: M=%d", M);
-    }
-    MOEA_CUDA_TRY(cudaGetLastError());
-    assoc_finish<<<ceil_div(n_cap, 256), 256, 0, stream>>>(best, d_n, idx, dist);
-    MOEA_CUDA_TRY(cudaGetLastError());
-    return MOEA_OK;
+    MOEA_TRY(run_dir_delta(refs, M, H, delta, stream));
+    return run_assoc_dense(x, n_cap, nullptr, refs, M, d_n, n_cap, H, 0.0f, delta, idx, dist, stream);
 }
 
 int run_niching(Workspace& ws, uint64_t seed, const int* nds_gidx, const float* dist,
@@ -2049,26 +1847,6 @@ int fused_select_configure()
     return MOEA_OK;
 }
 
-// Association of a bucket of M > kTreeMaxObjectives instances: one thread
-// per point over every direction, or, above kFusedScanSplitLen directions,
-// the direction-split scan (at most kFusedScanMaxSplits ranges).
-constexpr int kFusedScanSplitLen = 1024;
-constexpr int kFusedScanMaxSplits = 8;
-
-template <int M>
-void fused_scan_launch(const BatchInst* d_inst, const FusedBucket& b, cudaStream_t s)
-{
-    const int splits = std::min(kFusedScanMaxSplits, std::max(1, ceil_div(b.max_H, kFusedScanSplitLen)));
-    const dim3 grid(ceil_div(b.max_n, kAssocThreads), b.count);
-    if (splits == 1) {
-        fused_scan<M><<<grid, kAssocThreads, 0, s>>>(d_inst, b.d_ids);
-        return;
-    }
-    fused_scan_reset<<<grid, kAssocThreads, 0, s>>>(d_inst, b.d_ids);
-    fused_scan_split<M><<<dim3(grid.x, grid.y, splits), kAssocThreads, 0, s>>>(d_inst, b.d_ids, splits);
-    fused_scan_finish<<<grid, kAssocThreads, 0, s>>>(d_inst, b.d_ids);
-}
-
 int fused_select(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s)
 {
     const int sort_smem = (int)sizeof(FusedSelStorage);
@@ -2077,11 +1855,11 @@ int fused_select(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s)
 #define MOEA_FP_CASE(K)                                                                              \
         case K:                                                                                      \
             fused_prep<K><<<b.count, kFusedThreads, 0, s>>>(d_inst, b.d_ids);                        \
-            if (K <= kTreeMaxObjectives)                                                             \
+            if (K <= kTreeMaxObjectives && !dense_preferred_batch(b.max_H))                          \
                 fused_assoc<K><<<dim3(ceil_div(b.max_n, kTreeWarps), b.count), kTreeWarps * 32, 0,    \
                                  s>>>(d_inst, b.d_ids);                                              \
             else                                                                                     \
-                fused_scan_launch<K>(d_inst, b, s);                                                  \
+                MOEA_TRY(fused_associate_dense(d_inst, b, s));                                                \
             break;
         MOEA_FP_CASE(1) MOEA_FP_CASE(2) MOEA_FP_CASE(3) MOEA_FP_CASE(4)
         MOEA_FP_CASE(5) MOEA_FP_CASE(6) MOEA_FP_CASE(7) MOEA_FP_CASE(8)
