@@ -1157,10 +1157,12 @@ BatchInst fused_describe(moea_algorithm* a, int P, int X)
     b.varsO = a->vars[1]; b.objsO = a->objs[1]; b.cvO = a->cv[1];
     b.varsX = a->vars[X]; b.objsX = a->objs[X]; b.cvX = a->cv[X]; b.rankX = a->rank[X];
     b.bounds = a->bounds; b.pidx = a->parent_idx; b.d_gen = a->d_gen; b.ideal = a->ideal_last;
-    b.key0 = w.key0; b.key64 = w.key64[0]; b.perm = w.perm[0]; b.vals = w.sel_vals[0];
+    b.key0 = w.key0; b.key64 = w.key64[0]; b.key64b = w.key64[1]; b.vals = w.sel_vals[0];
+    b.perm_a = w.perm[0]; b.perm_b = w.perm[1]; b.perm = b.n > kFusedSortTile ? w.perm[0] : w.perm[1];
+    b.long_runs = w.run_start; b.block_tables = w.block_tables;
     b.sorted_f = w.sorted_f; b.qinfo = w.qinfo; b.blocker = w.blocker; b.front_sorted = w.front_sorted;
-    b.front_list = w.front_list; b.counters = w.counters; b.rows = w.rows; b.chunk_keys = w.chunk_keys;
-    b.chunk_bits = w.chunk_bits; b.fronts = w.fronts; b.nds_gidx = w.nds_gidx; b.sizes = w.sizes;
+    b.front_list = w.front_list; b.counters = w.counters; b.rows = w.rows;
+    b.fronts = w.fronts; b.nds_gidx = w.nds_gidx; b.sizes = w.sizes;
     b.nds_objs = w.nds_objs; b.rcp_b = w.rcp_b; b.extreme = w.extreme; b.assoc_idx = w.assoc_idx;
     b.assoc_dist = w.assoc_dist; b.rho = w.rho; b.selected = w.selected; b.flags = w.flags;
     b.survivors = a->survivors; b.offset = w.offset_dev;

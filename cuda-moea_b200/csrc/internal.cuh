@@ -267,6 +267,7 @@ constexpr int kFusedMaxPoints = 8192;
 constexpr int kDirTreeMaxDepth = 8;   // stack depth of the tree association kernels
 constexpr int kFusedThreads = 1024;
 constexpr int kFusedItems = kFusedMaxPoints / kFusedThreads;
+constexpr int kFusedSortTile = 1024;  // points per sorted tile; more are merged once
 
 struct BatchInst {
     int N, D, M, H, n, n_max, W, kind, tournament, mutate, T;
@@ -277,9 +278,14 @@ struct BatchInst {
     float* varsO; float* objsO; float* cvO;
     float* varsX; float* objsX; float* cvX; int* rankX;
     const float* bounds; int* pidx; int* d_gen; float* ideal;
-    uint64_t* key0; uint64_t* key64; int* perm; int* vals; float* sorted_f; int* qinfo;
+    uint64_t* key0; uint64_t* key64; uint64_t* key64b; float* sorted_f; int* qinfo;
+    int* perm_a; int* perm_b;   // sort tiles' and merge's permutations
+    int* perm;                  // the final one: the buffer that the last of them leaves free
+    int* long_runs;             // runs of equal keys longer than a thread ranks
+    int* vals;
+    uint32_t* block_tables;
     int* blocker; int* front_sorted; int* front_list; int* counters;
-    uint32_t* rows; uint32_t* chunk_keys; uint32_t* chunk_bits;
+    uint32_t* rows;
     int* fronts; int* nds_gidx; int* sizes; float* nds_objs; float* rcp_b; int* extreme;
     int* assoc_idx; float* assoc_dist; int* rho; int* selected; int* flags; int* survivors;
     unsigned long long* offset;
@@ -291,7 +297,7 @@ struct BatchInst {
 // Launch plan of one M value: instance ids and the prefix of their tile blocks.
 struct FusedBucket {
     int M = 0, count = 0, max_n = 0, tile_blocks = 0;
-    int shape = 0;                 // dominance tile shape (fused_tile_blocks)
+    int shape = 0;                 // dominator positions per row CTA (fused_tile_blocks)
     int max_H = 0;                 // most directions of an instance
     int* d_ids = nullptr;          // (count) instance indices
     int* d_tile_prefix = nullptr;  // (count + 1) first tile block of each instance

@@ -119,15 +119,15 @@ constexpr int kSortWays = 8;   // runs merged per pass
 
 // key0[i] = class << 32 | order key of f0 (class 0) or cv (class 2); sorted
 // tiles of (sort_key, index) into skey and perm.  Clears the sort's counters.
-__global__ void __launch_bounds__(kSortTile)
-nds_sort_tiles(SplitPop pop, int M, uint64_t* __restrict__ key0, uint64_t* __restrict__ skey, int* __restrict__ perm,
-               int* __restrict__ counters)
+__device__ __forceinline__ void sort_tile(int tile, const SplitPop& pop, int M, uint64_t* __restrict__ key0,
+                                          uint64_t* __restrict__ skey, int* __restrict__ perm,
+                                          int* __restrict__ counters)
 {
     __shared__ uint64_t s_a[kSortTile], s_b[kSortTile];
     __shared__ unsigned short s_i[kSortTile];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int base = blockIdx.x * kSortTile, i = base + t;
-    if (blockIdx.x == 0 && t < 20 && (t < 5 || (t >= 10 && t <= 13) || t >= 16)) counters[t] = 0;
+    const int base = tile * kSortTile, i = base + t;
+    if (tile == 0 && t < 20 && (t < 5 || (t >= 10 && t <= 13) || t >= 16)) counters[t] = 0;
     uint64_t key = (1ull << kSortKeyBits) - 1ull;  // padding: above every real key
     if (i < pop.n) {
         uint32_t val;
@@ -187,13 +187,19 @@ nds_sort_tiles(SplitPop pop, int M, uint64_t* __restrict__ key0, uint64_t* __res
     }
 }
 
-// Sorted runs of L keys (L a power of two) merged in groups of kSortWays.
-__global__ void __launch_bounds__(256)
-nds_sort_merge(const uint64_t* __restrict__ key_in, const int* __restrict__ perm_in, uint64_t* __restrict__ key_out,
-               int* __restrict__ perm_out, int n, int L)
+__global__ void __launch_bounds__(kSortTile)
+nds_sort_tiles(SplitPop pop, int M, uint64_t* __restrict__ key0, uint64_t* __restrict__ skey, int* __restrict__ perm,
+               int* __restrict__ counters)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    sort_tile(blockIdx.x, pop, M, key0, skey, perm, counters);
+}
+
+// Key i of sorted runs of L keys (L a power of two) to its place among the
+// kSortWays runs of its group.
+__device__ __forceinline__ void sort_merge_key(int i, const uint64_t* __restrict__ key_in,
+                                               const int* __restrict__ perm_in, uint64_t* __restrict__ key_out,
+                                               int* __restrict__ perm_out, int n, int L)
+{
     const uint64_t key = key_in[i];
     const int run = i / L, r0 = run & ~(kSortWays - 1);
     const long long first = (long long)r0 * L;
@@ -216,6 +222,14 @@ nds_sort_merge(const uint64_t* __restrict__ key_in, const int* __restrict__ perm
     perm_out[at] = perm_in[i];
 }
 
+__global__ void __launch_bounds__(256)
+nds_sort_merge(const uint64_t* __restrict__ key_in, const int* __restrict__ perm_in, uint64_t* __restrict__ key_out,
+               int* __restrict__ perm_out, int n, int L)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) sort_merge_key(i, key_in, perm_in, key_out, perm_out, n, L);
+}
+
 // Total order inside a run of equal sort keys of class 0: lexicographic on
 // the order keys of f1 .. f_{M-1}, then the point index.
 __device__ __forceinline__ bool tie_less(const SplitPop& pop, int M, int a, int b)
@@ -235,12 +249,11 @@ constexpr int kTieSmemSort = 4096;    // longer runs: bitonic in shared memory u
 // Runs of equal keys in class 0 into lexicographic order: every member of a run
 // of at most kTieShort counts the members before it; longer runs are copied
 // and listed for nds_tie_fix_long.
-__global__ void nds_tie_rank(SplitPop pop, int M, const uint64_t* __restrict__ skey, const int* __restrict__ perm_in,
-                             int* __restrict__ perm_out, int* __restrict__ long_runs, int* __restrict__ n_long)
+__device__ __forceinline__ void tie_rank(int pos, const SplitPop& pop, int M, const uint64_t* __restrict__ skey,
+                                         const int* __restrict__ perm_in, int* __restrict__ perm_out,
+                                         int* __restrict__ long_runs, int* __restrict__ n_long)
 {
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = pop.n;
-    if (pos >= n) return;
     const uint64_t k = skey[pos];
     const int pt = perm_in[pos];
     int to = pos;
@@ -257,6 +270,13 @@ __global__ void nds_tie_rank(SplitPop pop, int M, const uint64_t* __restrict__ s
         }
     }
     perm_out[to] = pt;
+}
+
+__global__ void nds_tie_rank(SplitPop pop, int M, const uint64_t* __restrict__ skey, const int* __restrict__ perm_in,
+                             int* __restrict__ perm_out, int* __restrict__ long_runs, int* __restrict__ n_long)
+{
+    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
+    if (pos < pop.n) tie_rank(pos, pop, M, skey, perm_in, perm_out, long_runs, n_long);
 }
 
 // Ascending bitonic network over a[0, L) with virtual +inf padding to the
@@ -292,17 +312,18 @@ __device__ void tie_bitonic(const SplitPop& pop, int M, int* a, int L)
     }
 }
 
-// One CTA per listed run longer than kTieShort: its length, then a bitonic
-// sort unless the run is already in order (runs of identical vectors are).
-__global__ void __launch_bounds__(kTieLongThreads)
-nds_tie_fix_long(SplitPop pop, int M, const uint64_t* __restrict__ skey, int* __restrict__ perm,
-                 const int* __restrict__ long_runs, const int* __restrict__ n_long)
+// One CTA per listed run longer than kTieShort (first, first + step, ... of the
+// list): its length, then a bitonic sort unless the run is already in order
+// (runs of identical vectors are).
+__device__ __forceinline__ void tie_fix_long(int first, int step, const SplitPop& pop, int M,
+                                             const uint64_t* __restrict__ skey, int* __restrict__ perm,
+                                             const int* __restrict__ long_runs, const int* __restrict__ n_long)
 {
     __shared__ int s_arr[kTieSmemSort];
     __shared__ int s_len, s_unsorted;
     const int n = pop.n;
     const int count = *n_long;
-    for (int r = blockIdx.x; r < count; r += gridDim.x) {
+    for (int r = first; r < count; r += step) {
         const int start = long_runs[r];
         const uint64_t k = skey[start];
         if (threadIdx.x == 0) {
@@ -337,21 +358,25 @@ nds_tie_fix_long(SplitPop pop, int M, const uint64_t* __restrict__ skey, int* __
     }
 }
 
+__global__ void __launch_bounds__(kTieLongThreads)
+nds_tie_fix_long(SplitPop pop, int M, const uint64_t* __restrict__ skey, int* __restrict__ perm,
+                 const int* __restrict__ long_runs, const int* __restrict__ n_long)
+{
+    tie_fix_long(blockIdx.x, gridDim.x, pop, M, skey, perm, long_runs, n_long);
+}
+
 // Sorted copy of objectives 1..M-1, the dup positions, the peel's initial state
 // and the class counts.  The start of a run of identical vectors (class 0) or
 // violations (class 2) is found by doubling steps back and a binary search:
 // positions between two identical ones are identical, and nearly every run has
 // one member, so no scan over the positions is needed.
-__global__ void nds_finalize_rows(SplitPop pop, int M, const uint64_t* __restrict__ key0,
-                                  const uint64_t* __restrict__ skey, const int* __restrict__ perm,
-                                  float* __restrict__ sf, int sf_stride, int* __restrict__ counters,
-                                  int* __restrict__ qinfo, int* __restrict__ blocker, int* __restrict__ front_sorted,
-                                  uint32_t* __restrict__ fmask, int fmask_words)
+__device__ __forceinline__ void finalize_row(int pos, const SplitPop& pop, int M, const uint64_t* __restrict__ key0,
+                                             const uint64_t* __restrict__ skey, const int* __restrict__ perm,
+                                             float* __restrict__ sf, int sf_stride, int* __restrict__ counters,
+                                             int* __restrict__ qinfo, int* __restrict__ blocker,
+                                             int* __restrict__ front_sorted)
 {
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = pop.n;
-    for (int w = pos; w < fmask_words; w += gridDim.x * blockDim.x) fmask[w] = 0u;
-    if (pos >= n) return;
     const int pt = perm[pos];
     const uint64_t k0 = key0[pt];
     const uint32_t cls = (uint32_t)(k0 >> 32);
@@ -408,6 +433,19 @@ __global__ void nds_finalize_rows(SplitPop pop, int M, const uint64_t* __restric
         if (cls < 2u) counters[0] = n;
         if (cls == 2u) atomicAdd(counters + 10, n);
     }
+}
+
+// Also empties the peel's front masks.
+__global__ void nds_finalize_rows(SplitPop pop, int M, const uint64_t* __restrict__ key0,
+                                  const uint64_t* __restrict__ skey, const int* __restrict__ perm,
+                                  float* __restrict__ sf, int sf_stride, int* __restrict__ counters,
+                                  int* __restrict__ qinfo, int* __restrict__ blocker, int* __restrict__ front_sorted,
+                                  uint32_t* __restrict__ fmask, int fmask_words)
+{
+    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int w = pos; w < fmask_words; w += gridDim.x * blockDim.x) fmask[w] = 0u;
+    if (pos < pop.n)
+        finalize_row(pos, pop, M, key0, skey, perm, sf, sf_stride, counters, qinfo, blocker, front_sorted);
 }
 
 // ---------------------------------------------------------------------------
@@ -472,14 +510,6 @@ template <int M>
 struct TileCfg {
     static constexpr int kPW = (M <= 4) ? 32 : ((M <= 8) ? 16 : 8);
     static constexpr int kMF = (M > 1) ? M - 1 : 1;   // objectives 1..M-1
-};
-
-// Words per tile CTA of a tile shape: shape 0 is TileCfg's, shape 1 half of
-// it (twice the CTAs, each with half the staged word tables).  The batch's
-// autotuner picks the shape per objective count by measured time.
-template <int M, int S>
-struct TileShape {
-    static constexpr int kPW = S == 0 ? TileCfg<M>::kPW : TileCfg<M>::kPW / 2;
 };
 
 // Count of the 32 ascending keys at shared address a that are <= v, as the
@@ -1431,14 +1461,14 @@ __device__ __forceinline__ int count_le32(const uint32_t* a, uint32_t x)
 // by position.  Then the tree placement of the sorted keys, and warp w builds
 // word w of every prefix set with one ballot per set.
 template <int B>
-__global__ void __launch_bounds__(B)
-nds_block_tables(const float* __restrict__ sf, int sf_stride, int n, int MF, uint32_t* __restrict__ tables)
+__device__ __forceinline__ void block_table(int cta, const float* __restrict__ sf, int sf_stride, int n, int MF,
+                                            uint32_t* __restrict__ tables)
 {
     using T = BlockTable<B>;
     constexpr int NW = B / 32;
     __shared__ uint32_t s_sorted[NW][32];
     __shared__ int s_rank[B];
-    const int blk = blockIdx.x / MF, m = blockIdx.x - blk * MF;
+    const int blk = cta / MF, m = cta - blk * MF;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int p = blk * B + threadIdx.x;
     const uint32_t key = p < n ? dom_key(sf[(size_t)m * sf_stride + p]) : 0xFFFFFFFFu;
@@ -1488,6 +1518,13 @@ nds_block_tables(const float* __restrict__ sf, int sf_stride, int n, int MF, uin
     }
 }
 
+template <int B>
+__global__ void __launch_bounds__(B)
+nds_block_tables(const float* __restrict__ sf, int sf_stride, int n, int MF, uint32_t* __restrict__ tables)
+{
+    block_table<B>(blockIdx.x, sf, sf_stride, n, MF, tables);
+}
+
 __device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 constexpr int kRowSegWords = 16;   // row words per lane collected before the stores
@@ -1512,10 +1549,9 @@ constexpr bool collect_rows() { return B == 256; }
 // the highest dominator seen and raises blocker[q] to it once.  Infeasible q
 // are skipped: the peel never reaches them, so their rows are never read.
 template <int M, int B>
-__global__ void __launch_bounds__(kBlkThreads)
-nds_block_rows(const float* __restrict__ sf, int sf_stride, const int* __restrict__ qinfo,
-               const uint32_t* __restrict__ tables, int n, int W, int bpc, uint32_t* __restrict__ rows,
-               int* __restrict__ blocker)
+__device__ __forceinline__ void block_rows(int bx, int by, const float* __restrict__ sf, int sf_stride,
+                                           const int* __restrict__ qinfo, const uint32_t* __restrict__ tables, int n,
+                                           int W, int bpc, uint32_t* __restrict__ rows, int* __restrict__ blocker)
 {
     using T = BlockTable<B>;
     constexpr int MF = M - 1;
@@ -1526,11 +1562,11 @@ nds_block_rows(const float* __restrict__ sf, int sf_stride, const int* __restric
     extern __shared__ uint4 s_tab[];  // [2][CH] tables, then (collect_rows) [kBlkThreads][kOutStride] row words
     __shared__ unsigned char s_live[kBlkThreads];
     uint32_t* s_out = reinterpret_cast<uint32_t*>(s_tab + 2 * CH);
-    const int q0 = blockIdx.y * kBlkThreads;
+    const int q0 = by * kBlkThreads;
     if (q0 >= n) return;
     const int qend = min(q0 + kBlkThreads, n);
     const int nb = (qend - 1 + B - 1) / B;  // blocks holding the dominators (positions < qend - 1)
-    const int b_lo = blockIdx.x * bpc;
+    const int b_lo = bx * bpc;
     if (b_lo >= nb) return;
     const int b_hi = min(nb, b_lo + bpc);
     const int q = q0 + threadIdx.x;
@@ -1643,6 +1679,15 @@ nds_block_rows(const float* __restrict__ sf, int sf_stride, const int* __restric
     if (best >= 0) atomicMax(blocker + q, best);
 }
 
+template <int M, int B>
+__global__ void __launch_bounds__(kBlkThreads)
+nds_block_rows(const float* __restrict__ sf, int sf_stride, const int* __restrict__ qinfo,
+               const uint32_t* __restrict__ tables, int n, int W, int bpc, uint32_t* __restrict__ rows,
+               int* __restrict__ blocker)
+{
+    block_rows<M, B>(blockIdx.x, blockIdx.y, sf, sf_stride, qinfo, tables, n, W, bpc, rows, blocker);
+}
+
 template <int M>
 constexpr int block_rows_smem()
 {
@@ -1699,314 +1744,98 @@ void launch_tiles(const Workspace& ws, int n, cudaStream_t stream)
 // fused batch: one launch per stage for every instance (n = 2N <= 8192)
 // ---------------------------------------------------------------------------
 
-// Block sorts with 2, 4 or 8 items per thread: the smallest that holds the
-// instance (the sort's work grows with the items).
-template <int ITEMS>
-using FusedSort64 = cub::BlockRadixSort<uint64_t, kFusedThreads, ITEMS, int>;
-using FusedScan = cub::BlockScan<int, kFusedThreads>;
-union FusedSortStorage {
-    typename FusedSort64<kFusedItems>::TempStorage s64;
-    typename FusedSort64<4>::TempStorage s64_4;
-    typename FusedSort64<2>::TempStorage s64_2;
-    typename FusedScan::TempStorage scan;
-    int list[kFusedThreads + 4];  // long runs of fused_lex_onekey
-};
-
-// The order of fused_lexsort for n > kFusedThreads, as the staged path
-// builds it: one block radix sort of the sort keys (sort_key) with ITEMS keys
-// per thread, then each run of equal keys in class 0 put in lexicographic
-// order (f1 .. f_{M-1}, index) -- runs of up to kTieShort points by one
-// thread each (insertion sort), longer ones (when not already in order) by the
-// whole CTA, each member counting the members that precede it.  One sort of
-// kSortKeyBits bits replaces M-1 stable passes of 32 bits and one of 34.  The
-// permutation goes to I.perm[0 .. n); I.key64 holds the sorted keys and
-// I.vals serves the long runs as scratch.
-template <int ITEMS>
-__device__ __forceinline__ void fused_lex_onekey(const BatchInst& I, const SplitPop& pop, int n, int M,
-                                                 FusedSortStorage& tmp)
+// The sort and the dominance rows of every instance (blockIdx.y) by the CTAs
+// and threads of the staged path: tiles, one rank merge above kSortTile points,
+// runs of equal keys, sorted objectives and dup positions.  The passes of one
+// CTA per instance that these replace (a block radix sort, and the rows from
+// per-word tables) took 269 + 71 + 913 us over 256 instances.
+static_assert(kFusedSortTile == kSortTile && kFusedMaxPoints == kSortTile * kSortWays, "one merge pass");
+__device__ __forceinline__ SplitPop batch_pop(const BatchInst& I)
 {
-    const int t = threadIdx.x;
-    uint64_t keys[ITEMS];
-    int vals[ITEMS];
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const int pt = t * ITEMS + j;
-        vals[j] = pt;
-        if (pt < n) {
-            const uint64_t k0 = I.key0[pt];
-            keys[j] = sort_key(pop, M, pt, (uint32_t)(k0 >> 32), (uint32_t)k0);
-        } else {
-            keys[j] = (1ull << kSortKeyBits) - 1ull;  // above every real key
-        }
-    }
-    FusedSort64<ITEMS>(*reinterpret_cast<typename FusedSort64<ITEMS>::TempStorage*>(&tmp))
-        .Sort(keys, vals, 0, kSortKeyBits);
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const int pos = t * ITEMS + j;
-        if (pos < n) {
-            I.key64[pos] = keys[j];
-            I.perm[pos] = vals[j];
-        }
-    }
-    __syncthreads();
-    const uint64_t* K = I.key64;
-    int* P = I.perm;
-    // short runs, one thread per run head
-    for (int pos = t; pos < n; pos += kFusedThreads) {
-        const uint64_t k = K[pos];
-        if ((k >> kSortClassShift) != 0u || (pos > 0 && K[pos - 1] == k)) continue;
-        int L = 1;
-        while (L <= kTieShort && pos + L < n && K[pos + L] == k) ++L;
-        if (L == 1 || L > kTieShort) continue;
-        for (int a = pos + 1; a < pos + L; ++a) {
-            const int v = P[a];
-            int b = a - 1;
-            while (b >= pos && tie_less(pop, M, v, P[b])) {
-                P[b + 1] = P[b];
-                --b;
-            }
-            P[b + 1] = v;
-        }
-    }
-    __syncthreads();
-    // long runs, one after another by the whole CTA (the sort storage is free)
-    int* s_heads = reinterpret_cast<int*>(&tmp);
-    int* s_misc = s_heads + kFusedThreads;  // [0] heads, [1] run end, [2] out of order
-    for (int base = 0; base < n; base += kFusedThreads) {
-        if (t == 0) s_misc[0] = 0;
-        __syncthreads();
-        const int pos = base + t;
-        if (pos < n) {
-            const uint64_t k = K[pos];
-            if ((k >> kSortClassShift) == 0u && (pos == 0 || K[pos - 1] != k) && pos + kTieShort < n &&
-                K[pos + kTieShort] == k)
-                s_heads[atomicAdd(s_misc, 1)] = pos;
-        }
-        __syncthreads();
-        const int nh = s_misc[0];
-        for (int h = 0; h < nh; ++h) {
-            const int head = s_heads[h];
-            const uint64_t k = K[head];
-            if (t == 0) {
-                s_misc[1] = n;
-                s_misc[2] = 0;
-            }
-            __syncthreads();
-            for (int a = head + 1 + t; a < n; a += kFusedThreads)
-                if (K[a] != k) {
-                    atomicMin(s_misc + 1, a);
-                    break;
-                }
-            __syncthreads();
-            const int end = s_misc[1];
-            for (int a = head + 1 + t; a < end; a += kFusedThreads)
-                if (tie_less(pop, M, P[a], P[a - 1])) s_misc[2] = 1;
-            __syncthreads();
-            if (s_misc[2]) {
-                for (int a = head + t; a < end; a += kFusedThreads) {
-                    const int v = P[a];
-                    int r = 0;
-                    for (int b = head; b < end; ++b) r += tie_less(pop, M, P[b], v) ? 1 : 0;
-                    I.vals[head + r] = v;
-                }
-                __syncthreads();
-                for (int a = head + t; a < end; a += kFusedThreads) P[a] = I.vals[a];
-            }
-            __syncthreads();
-        }
-    }
+    return SplitPop{I.objsP, I.objsO, I.cvP, I.cvO, I.N, I.N, I.N, I.n};
 }
 
-// Classification, sorted order, sorted objectives, dup positions and peel
-// state of one instance per CTA: the stages of run_ndsort up to the
-// dominance rows.  Instances of more than kFusedThreads points take the
-// staged path's order (fused_lex_onekey); smaller ones count ranks under the
-// lexicographic order (class and f0, f1 .. f_{M-1}, index).  Either order
-// has what the rows and the peel need (dominators first, identical vectors
-// adjacent, f0 non-decreasing in class 0), and the fronts depend on the
-// relation only.
-template <bool kLarge>
-__device__ __forceinline__ void fused_lexsort_body(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
-{
-    extern __shared__ __align__(16) unsigned char fused_smem[];
-    FusedSortStorage& tmp = *reinterpret_cast<FusedSortStorage*>(fused_smem);
-    __shared__ int s_feas;
-    const BatchInst& I = insts[ids[blockIdx.x]];
-    const SplitPop pop{I.objsP, I.objsO, I.cvP, I.cvO, I.N, I.N, I.N, I.n};
-    const int n = I.n, M = I.M, t = threadIdx.x;
-    if (t == 0) s_feas = 0;
-    __syncthreads();
-    int feas = 0;
-    for (int i = t; i < n; i += kFusedThreads) {
-        const float cv = pop.cvv(i);
-        uint32_t cls, val = 0;
-        if (cv == 0.0f) {
-            bool nan = false;
-            for (int m = 0; m < M; ++m) nan |= isnan(pop.obj(m, i));
-            cls = nan ? 1u : 0u;
-            if (!nan) val = float_order_key(pop.obj(0, i));
-        } else {
-            cls = isnan(cv) ? 3u : 2u;
-            if (cls == 2u) val = float_order_key(cv);
-        }
-        I.key0[i] = ((uint64_t)cls << 32) | val;
-        feas += cls <= 1u;
-    }
-    atomicAdd(&s_feas, feas);
-    __syncthreads();
-    int vals[kFusedItems];
-#pragma unroll
-    for (int j = 0; j < kFusedItems; ++j) vals[j] = t * kFusedItems + j;
-    if (n <= kFusedThreads) {
-        // Small instances: the stable passes below order by (class and f0,
-        // then f1 .. f_{M-1} for class 0, then the index); here each point
-        // counts the points before it under that order directly, instead of
-        // block sorts sized for kFusedMaxPoints.  Same permutation.
-        uint64_t* s_k0 = reinterpret_cast<uint64_t*>(fused_smem);
-        int* s_perm = reinterpret_cast<int*>(s_k0 + kFusedThreads);
-        if (t < n) s_k0[t] = I.key0[t];
-        __syncthreads();
-        if (t < n) {
-            const uint64_t ki = s_k0[t];
-            const bool cls0 = (ki >> 32) == 0;
-            int r = 0;
-            for (int u = 0; u < n; ++u) {
-                const uint64_t ku = s_k0[u];
-                bool less = ku < ki;
-                if (ku == ki) {
-                    less = u < t;
-                    if (cls0) {
-                        for (int m = 1; m < M; ++m) {
-                            const uint32_t a = float_order_key(pop.obj(m, u));
-                            const uint32_t b = float_order_key(pop.obj(m, t));
-                            if (a != b) {
-                                less = a < b;
-                                break;
-                            }
-                        }
-                    }
-                }
-                r += less ? 1 : 0;
-            }
-            s_perm[r] = t;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < kFusedItems; ++j) {
-            const int pos = t * kFusedItems + j;
-            vals[j] = (pos < n) ? s_perm[pos] : pos;
-        }
-        __syncthreads();  // the shared storage is reused below
-    } else {
-        if constexpr (kLarge) {
-            if (n <= 2 * kFusedThreads) fused_lex_onekey<2>(I, pop, n, M, tmp);
-            else if (n <= 4 * kFusedThreads) fused_lex_onekey<4>(I, pop, n, M, tmp);
-            else fused_lex_onekey<kFusedItems>(I, pop, n, M, tmp);
-            __syncthreads();  // the permutation in I.perm, written by every thread
-#pragma unroll
-            for (int j = 0; j < kFusedItems; ++j) {
-                const int pos = t * kFusedItems + j;
-                vals[j] = (pos < n) ? I.perm[pos] : pos;
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < kFusedItems; ++j) {
-        const int pos = t * kFusedItems + j;
-        if (pos < n) I.perm[pos] = vals[j];
-    }
-    __syncthreads();
-    int heads[kFusedItems];
-#pragma unroll
-    for (int j = 0; j < kFusedItems; ++j) {
-        const int pos = t * kFusedItems + j;
-        heads[j] = 0;
-        if (pos >= n) continue;
-        const int pt = vals[j];
-        const uint64_t k0 = I.key0[pt];
-        const uint32_t cls = (uint32_t)(k0 >> 32);
-        for (int m = 1; m < M; ++m) I.sorted_f[(size_t)(m - 1) * I.n_max + pos] = pop.obj(m, pt);
-        bool is_head = true;
-        if (pos > 0) {
-            const int pp = I.perm[pos - 1];
-            if (I.key0[pp] == k0) {
-                if (cls == 0u) {
-                    bool same = true;
-                    for (int m = 1; m < M; ++m)
-                        same &= float_order_key(pop.obj(m, pt)) == float_order_key(pop.obj(m, pp));
-                    is_head = !same;
-                } else {
-                    is_head = false;
-                }
-            }
-        }
-        heads[j] = is_head ? pos : 0;
-    }
-    FusedScan(tmp.scan).InclusiveScan(heads, heads, cub::Max());
-    __syncthreads();
-    const int feasible = s_feas;
-#pragma unroll
-    for (int j = 0; j < kFusedItems; ++j) {
-        const int pos = t * kFusedItems + j;
-        if (pos >= n) continue;
-        const uint32_t cls = (uint32_t)(I.key0[vals[j]] >> 32);
-        uint32_t d;
-        switch (cls) {
-        case 0u: d = (uint32_t)heads[j]; break;
-        case 1u: d = 0u; break;
-        case 2u: d = (uint32_t)heads[j] | kInfeasibleBit; break;
-        default: d = (uint32_t)feasible | kInfeasibleBit; break;
-        }
-        I.qinfo[pos] = (int)d;
-        I.blocker[pos] = -1;
-        I.front_sorted[pos] = -1;
-    }
-    if (t == 0) {
-        I.counters[0] = feasible;
-        for (int c = 1; c <= 4; ++c) I.counters[c] = 0;
-    }
-}
-
-__global__ void __launch_bounds__(kFusedThreads)
-fused_lexsort(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
-{
-    fused_lexsort_body<true>(insts, ids);
-}
-
-// Groups whose instances all have at most kFusedThreads points: the same
-// body without the block sorts, a much smaller kernel (its instances are
-// launch- and latency-bound, and the sort code around the counting path
-// slowed them by 9%).
-__global__ void __launch_bounds__(kFusedThreads)
-fused_lexsort_small(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
-{
-    fused_lexsort_body<false>(insts, ids);
-}
-
-// Shared memory of fused_lexsort_small: the counting path's keys and
-// permutation, or the block scan's storage.
-constexpr int kFusedLexSmallSmem =
-    (int)(kFusedThreads * (sizeof(uint64_t) + sizeof(int)) > sizeof(FusedScan::TempStorage)
-              ? kFusedThreads * (sizeof(uint64_t) + sizeof(int))
-              : sizeof(FusedScan::TempStorage));
-
-__global__ void fused_chunks(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
+__global__ void __launch_bounds__(kSortTile)
+fused_sort_tiles(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
 {
     const BatchInst& I = insts[ids[blockIdx.y]];
-    const int W = (I.n + 31) >> 5;
-    const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (gw >= W * (I.M - 1)) return;
-    chunk_warp(gw, threadIdx.x & 31, I.sorted_f, I.n_max, I.n, W, I.chunk_keys, I.chunk_bits);
+    if ((int)blockIdx.x * kSortTile < I.n) sort_tile(blockIdx.x, batch_pop(I), I.M, I.key0, I.key64, I.perm_a, I.counters);
 }
 
-// Tile CTAs of all instances with M objectives, flattened: CTA b belongs to
-// the instance whose range [prefix[k], prefix[k+1]) contains b.
-template <int M, int S>
-__global__ void __launch_bounds__(kTileThreads)
-fused_tiles(const BatchInst* __restrict__ insts, const int* __restrict__ ids,
-            const int* __restrict__ prefix, int count)
+__global__ void __launch_bounds__(256)
+fused_sort_merge(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
 {
+    const BatchInst& I = insts[ids[blockIdx.y]];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (I.n > kSortTile && i < I.n) sort_merge_key(i, I.key64, I.perm_a, I.key64b, I.perm_b, I.n, kSortTile);
+}
+
+__global__ void __launch_bounds__(256)
+fused_tie_rank(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
+{
+    const BatchInst& I = insts[ids[blockIdx.y]];
+    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
+    if (pos < I.n)
+        tie_rank(pos, batch_pop(I), I.M, I.n > kSortTile ? I.key64b : I.key64, I.n > kSortTile ? I.perm_b : I.perm_a,
+                 I.perm, I.long_runs, I.counters + 13);
+}
+
+__global__ void __launch_bounds__(kTieLongThreads)
+fused_tie_long(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
+{
+    const BatchInst& I = insts[ids[blockIdx.x]];
+    tie_fix_long(0, 1, batch_pop(I), I.M, I.n > kSortTile ? I.key64b : I.key64, I.perm, I.long_runs, I.counters + 13);
+}
+
+__global__ void __launch_bounds__(256)
+fused_finalize_rows(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
+{
+    const BatchInst& I = insts[ids[blockIdx.y]];
+    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
+    if (pos < I.n)
+        finalize_row(pos, batch_pop(I), I.M, I.key0, I.n > kSortTile ? I.key64b : I.key64, I.perm, I.sorted_f, I.n_max,
+                     I.counters, I.qinfo, I.blocker, I.front_sorted);
+}
+
+template <int M>
+__global__ void __launch_bounds__(BlockCfg<M>::kB)
+fused_block_tables(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
+{
+    const BatchInst& I = insts[ids[blockIdx.y]];
+    if ((int)(blockIdx.x / (M - 1)) * BlockCfg<M>::kB < I.n)
+        block_table<BlockCfg<M>::kB>(blockIdx.x, I.sorted_f, I.n_max, I.n, M - 1, I.block_tables);
+}
+
+// Row CTAs of one instance of n points with bpc blocks each; the CTA `cta`
+// of them as (block range, tile).
+template <int B>
+__host__ __device__ inline int row_ctas(int n, int bpc, int cta, int* bx, int* by)
+{
+    int first = 0;
+    for (int t = 0; t * kBlkThreads < n; ++t) {
+        const int end = (t + 1) * kBlkThreads < n ? (t + 1) * kBlkThreads : n;
+        const int nb = (end - 1 + B - 1) / B, here = (nb + bpc - 1) / bpc;
+        if (cta >= first && cta < first + here) {
+            *bx = cta - first;
+            *by = t;
+        }
+        first += here;
+    }
+    return first;
+}
+
+// Dominator positions per row CTA of a batch (tile shapes 0 and 1): batches
+// fill the device, so a CTA keeps many blocks and stages them in turn.
+constexpr int kBatchRowPositions[kTileShapes] = {1024, 512};
+
+// Row CTAs of all instances with M objectives, flattened: CTA b belongs to
+// the instance whose range [prefix[k], prefix[k+1]) contains b.
+template <int M>
+__global__ void __launch_bounds__(kBlkThreads)
+fused_block_rows(const BatchInst* __restrict__ insts, const int* __restrict__ ids, const int* __restrict__ prefix,
+                 int count, int bpc)
+{
+    constexpr int B = BlockCfg<M>::kB;
     const int b = blockIdx.x;
     int lo = 0, hi = count;  // largest k with prefix[k] <= b
     while (hi - lo > 1) {
@@ -2014,12 +1843,29 @@ fused_tiles(const BatchInst* __restrict__ insts, const int* __restrict__ ids,
         if (__ldg(prefix + mid) <= b) lo = mid; else hi = mid;
     }
     const BatchInst& I = insts[__ldg(ids + lo)];
+    int bx = 0, by = 0;
+    row_ctas<B>(I.n, bpc, b - __ldg(prefix + lo), &bx, &by);
+    block_rows<M, B>(bx, by, I.sorted_f, I.n_max, I.qinfo, I.block_tables, I.n, I.W, bpc, I.rows, I.blocker);
+}
+
+// One objective: rows from the dup positions alone.
+__global__ void __launch_bounds__(kTileThreads)
+fused_tiles_one(const BatchInst* __restrict__ insts, const int* __restrict__ ids, const int* __restrict__ prefix,
+                int count)
+{
+    const int b = blockIdx.x;
+    int lo = 0, hi = count;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(prefix + mid) <= b) lo = mid; else hi = mid;
+    }
+    const BatchInst& I = insts[__ldg(ids + lo)];
     const int maxw = (I.n + 31) >> 5;
-    constexpr int PW = TileShape<M, S>::kPW;
+    constexpr int PW = TileCfg<1>::kPW;
     const int gx = (maxw + PW - 1) / PW;
     const int lb = b - __ldg(prefix + lo);
-    tile_block<M, PW>(lb % gx, lb / gx, I.sorted_f, I.n_max, I.qinfo, I.chunk_keys, I.chunk_bits, I.n, I.W, maxw,
-                      I.rows, I.blocker);
+    tile_block<1, PW>(lb % gx, lb / gx, I.sorted_f, I.n_max, I.qinfo, nullptr, nullptr, I.n, I.W, maxw, I.rows,
+                      I.blocker);
 }
 
 constexpr int kFusedPeelThreads = 1024;
@@ -2179,18 +2025,24 @@ __global__ void fused_scatter(const BatchInst* __restrict__ insts, const int* __
 template <int M>
 int tile_blocks_of(int n, int shape)
 {
-    const int maxw = ceil_div(n, 32);
-    const int pw = shape == 0 ? TileShape<M, 0>::kPW : TileShape<M, 1>::kPW;
-    return ceil_div(maxw, pw) * ceil_div(n, kQB);
+    if constexpr (M == 1) return ceil_div(ceil_div(n, 32), TileCfg<1>::kPW) * ceil_div(n, kQB);
+    int bx, by;
+    return row_ctas<BlockCfg<M>::kB>(n, kBatchRowPositions[shape] / BlockCfg<M>::kB, -1, &bx, &by);
 }
 
 template <int M>
-void launch_fused_tiles(const BatchInst* d_inst, const FusedBucket& b, cudaStream_t s)
+int launch_fused_rows(const BatchInst* d_inst, const FusedBucket& b, cudaStream_t s)
 {
-    if (b.shape == 0)
-        fused_tiles<M, 0><<<b.tile_blocks, kTileThreads, 0, s>>>(d_inst, b.d_ids, b.d_tile_prefix, b.count);
-    else
-        fused_tiles<M, 1><<<b.tile_blocks, kTileThreads, 0, s>>>(d_inst, b.d_ids, b.d_tile_prefix, b.count);
+    if constexpr (M == 1) {
+        fused_tiles_one<<<b.tile_blocks, kTileThreads, 0, s>>>(d_inst, b.d_ids, b.d_tile_prefix, b.count);
+    } else {
+        constexpr int B = BlockCfg<M>::kB;
+        fused_block_tables<M><<<dim3(ceil_div(b.max_n, B) * (M - 1), b.count), B, 0, s>>>(d_inst, b.d_ids);
+        fused_block_rows<M><<<b.tile_blocks, kBlkThreads, block_rows_smem<M>(), s>>>(
+            d_inst, b.d_ids, b.d_tile_prefix, b.count, kBatchRowPositions[b.shape] / B);
+    }
+    MOEA_CUDA_TRY(cudaGetLastError());
+    return MOEA_OK;
 }
 
 // Self-test of the peel's two barrier waits with a short limit: every CTA
@@ -2426,8 +2278,13 @@ size_t fused_peel_smem(int W, int n) { return (size_t)W * sizeof(uint32_t) + 3 *
 
 int fused_ndsort_configure()
 {
-    MOEA_CUDA_TRY(cudaFuncSetAttribute(fused_lexsort, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sizeof(FusedSortStorage)));
+#define MOEA_BR_CASE(K) \
+    if (block_rows_smem<K>() > 48 * 1024) \
+        MOEA_TRY(raise_dynamic_smem((const void*)fused_block_rows<K>, block_rows_smem<K>()));
+    MOEA_BR_CASE(2) MOEA_BR_CASE(3) MOEA_BR_CASE(4) MOEA_BR_CASE(5) MOEA_BR_CASE(6) MOEA_BR_CASE(7)
+    MOEA_BR_CASE(8) MOEA_BR_CASE(9) MOEA_BR_CASE(10) MOEA_BR_CASE(11) MOEA_BR_CASE(12) MOEA_BR_CASE(13)
+    MOEA_BR_CASE(14) MOEA_BR_CASE(15) MOEA_BR_CASE(16)
+#undef MOEA_BR_CASE
     MOEA_CUDA_TRY(cudaFuncSetAttribute(fused_peel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)fused_peel_smem(4 * ceil_div(kFusedMaxPoints, 128), kFusedMaxPoints)));
     return MOEA_OK;
@@ -2435,19 +2292,16 @@ int fused_ndsort_configure()
 
 int fused_ndsort(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s)
 {
-    const int sort_smem = (int)sizeof(FusedSortStorage);
-    if (g.max_n <= kFusedThreads)
-        fused_lexsort_small<<<g.count, kFusedThreads, kFusedLexSmallSmem, s>>>(d_inst, g.d_ids);
-    else
-        fused_lexsort<<<g.count, kFusedThreads, sort_smem, s>>>(d_inst, g.d_ids);
+    const dim3 points(ceil_div(g.max_n, 256), g.count);
+    fused_sort_tiles<<<dim3(ceil_div(g.max_n, kSortTile), g.count), kSortTile, 0, s>>>(d_inst, g.d_ids);
+    if (g.max_n > kSortTile) fused_sort_merge<<<points, 256, 0, s>>>(d_inst, g.d_ids);
+    fused_tie_rank<<<points, 256, 0, s>>>(d_inst, g.d_ids);
+    fused_tie_long<<<g.count, kTieLongThreads, 0, s>>>(d_inst, g.d_ids);
+    fused_finalize_rows<<<points, 256, 0, s>>>(d_inst, g.d_ids);
     MOEA_CUDA_TRY(cudaGetLastError());
-    if (g.max_M > 1) {
-        const int warps = ceil_div(g.max_n, 32) * (g.max_M - 1);
-        fused_chunks<<<dim3(ceil_div(warps, 8), g.count), 256, 0, s>>>(d_inst, g.d_ids);
-    }
     for (const FusedBucket& b : g.buckets) {
         switch (b.M) {
-#define MOEA_FT_CASE(K) case K: launch_fused_tiles<K>(d_inst, b, s); break;
+#define MOEA_FT_CASE(K) case K: MOEA_TRY(launch_fused_rows<K>(d_inst, b, s)); break;
         MOEA_FT_CASE(1) MOEA_FT_CASE(2) MOEA_FT_CASE(3) MOEA_FT_CASE(4)
         MOEA_FT_CASE(5) MOEA_FT_CASE(6) MOEA_FT_CASE(7) MOEA_FT_CASE(8)
         MOEA_FT_CASE(9) MOEA_FT_CASE(10) MOEA_FT_CASE(11) MOEA_FT_CASE(12)
@@ -2456,7 +2310,6 @@ int fused_ndsort(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s)
         default: return set_error(MOEA_ERR_UNSUPPORTED, "fused ndsort: M=%d", b.M);
         }
     }
-    MOEA_CUDA_TRY(cudaGetLastError());
     fused_peel<<<g.count, kFusedPeelThreads, fused_peel_smem(g.max_W, g.max_n), s>>>(d_inst, g.d_ids);
     fused_scatter<<<dim3(ceil_div(g.max_n, 256), g.count), 256, 0, s>>>(d_inst, g.d_ids);
     MOEA_CUDA_TRY(cudaGetLastError());
