@@ -123,6 +123,73 @@ __device__ float row_objective(int m, float total_sum, const float* x, int D, in
     }
 }
 
+// The two factors of position variable q that row_objective evaluates (with its
+// multiply-adds spelled out): cosine
+// and sine of its angle, or the factors of its term in DTLZ7's h.
+template <int B>
+__device__ __forceinline__ void row_factors(int q, float total_sum, const float* x, int D, int M, float* a, float* b)
+{
+    const int k = D - (M - 1);
+    if (B == kDTLZ2 || B == kDTLZ3 || B == kConvexDTLZ2) {
+        *a = safe_cos_hp(x[q]);
+        *b = sinf(x[q] * M_PI / 2.0f);
+    } else if (B == kDTLZ4) {
+        const float p = powf(x[q], 100.0f);
+        *a = fmaxf(0.0f, cosf(p * M_PI / 2.0f));
+        *b = sinf(p * M_PI / 2.0f);
+    } else if (B == kDTLZ5 || B == kDTLZ6) {
+        const float g = total_sum;
+        float t = x[0];
+        if (q > 0) {
+            t = fmaf(2.0f * g, x[q], 1.0f) / (2.0f * (1.0f + g));
+            if (B == kDTLZ5) t = fmaxf(0.0f, fminf(1.0f, t));
+        }
+        *a = (B == kDTLZ5) ? fmaxf(0.0f, __cosf(t * M_PI * 0.5f)) : fmaxf(0.0f, cosf(t * M_PI * 0.5f));
+        *b = (B == kDTLZ5) ? __sinf(t * M_PI * 0.5f) : sinf(t * M_PI * 0.5f);
+    } else {  // kDTLZ7
+        const float g = fmaf(9.0f / static_cast<float>(k), total_sum, 1.0f);
+        const float fi = x[q];
+        *a = fi / (1.0f + g);
+        *b = 1.0f + sinf(3.0f * M_PI * fi);
+    }
+}
+
+// row_objective from the factors (called by every lane of the group; m >= M and
+// rows that are not valid give no result).
+template <int B, class FA, class FB>
+__device__ __forceinline__ float combine_factors(int m, float total_sum, const float* x, int D, int M, bool valid,
+                                                 FA fa, FB fb)
+{
+    const int k = D - (M - 1);
+    if (B == kDTLZ7) {
+        const float g = fmaf(9.0f / static_cast<float>(k), total_sum, 1.0f);
+        float h_sum = 0.0f;
+        for (int i = 0; i < M - 1; ++i) {
+            const float a = fa(i), b = fb(i);
+            h_sum = fmaf(a, b, h_sum);
+        }
+        const float h = static_cast<float>(M) - h_sum;
+        return m < M - 1 ? (valid ? x[m] : 0.0f) : (1.0f + g) * h;
+    }
+    const float g = (B == kDTLZ3) ? 100.0f * (static_cast<float>(k) + total_sum) : total_sum;
+    float f = 1.0f + g;
+    for (int j = 0; j < M - 1; ++j) {
+        const float c = fa(j);
+        if (j < M - 1 - m) f *= c;
+    }
+    const float s = fb(m > 0 && m < M ? M - 1 - m : 0);
+    if (m > 0) f *= s;
+    if (B == kConvexDTLZ2) {
+        if (m < M - 1) {
+            f = f * f;
+            f = f * f;
+        } else {
+            f = f * f;
+        }
+    }
+    return f;
+}
+
 // A group of G lanes (8 or 32) per row; valid when the row has at most 256
 // g-terms.  Every lane of the warp calls; rows that are not `valid` write
 // nothing.  The partials are those of a shuffle-down tree over 32 lanes: with
@@ -156,8 +223,39 @@ __device__ __forceinline__ void dtlz_group_row(int row, bool valid, int gl, cons
     }
     float total = (gl == 0) ? fold_partials<B>(ws) : 0.0f;
     total = __shfl_sync(0xFFFFFFFFu, total, 0, G);
-    if (valid)
-        for (int m = gl; m < M; m += G) objs[(size_t)m * N + row] = row_objective<B>(m, total, x, D, M);
+    if constexpr (B == kDTLZ1) {
+        if (valid)
+            for (int m = gl; m < M; m += G) objs[(size_t)m * N + row] = row_objective<B>(m, total, x, D, M);
+    } else {
+        // The factors of position variable j (cosine and sine, or the two
+        // factors of a DTLZ7 term) belong to every objective: lane j mod G
+        // evaluates them once and the products pick them up with shuffles, in
+        // row_objective's order (M - 1 evaluations per lane without: eight
+        // objectives of DTLZ4 took 14 powf per child and lane).
+        constexpr int kSlots = kMaxObjectives / G > 0 ? kMaxObjectives / G : 1;
+        float fa[kSlots], fb[kSlots];
+#pragma unroll
+        for (int v = 0; v < kSlots; ++v) {
+            const int q = gl + G * v;
+            fa[v] = fb[v] = 0.0f;
+            if (valid && q < M - 1) row_factors<B>(q, total, x, D, M, &fa[v], &fb[v]);
+        }
+        auto pick = [&](const float (&f)[kSlots], int q) {  // factor q of the row, by every lane
+            float r = 0.0f;
+#pragma unroll
+            for (int v = 0; v < kSlots; ++v) {
+                const float y = __shfl_sync(0xFFFFFFFFu, f[v], q & (G - 1), G);
+                if (q / G == v) r = y;
+            }
+            return r;
+        };
+        for (int m0 = 0; m0 < M; m0 += G) {
+            const int m = m0 + gl;
+            const float f = combine_factors<B>(m, total, x, D, M, valid, [&](int q) { return pick(fa, q); },
+                                               [&](int q) { return pick(fb, q); });
+            if (valid && m < M) objs[(size_t)m * N + row] = f;
+        }
+    }
 }
 
 // Constraint violation of one row from its objectives f[m * N]
