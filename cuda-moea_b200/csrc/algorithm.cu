@@ -84,8 +84,9 @@ namespace {
 __global__ void gather_next(const float* __restrict__ vars_a, const float* __restrict__ vars_b,
                             SplitPop pop, const int* __restrict__ surv, const int* __restrict__ fronts,
                             int N, int D, int M, float* __restrict__ vars, float* __restrict__ objs,
-                            float* __restrict__ cv, int* __restrict__ rank)
+                            float* __restrict__ cv, int* __restrict__ rank, int* gen)
 {
+    if (gen && blockIdx.x == 0 && threadIdx.x == 0) *gen += 1;  // the generation's last launch
     const int vec = (D & 3) == 0 ? 4 : 1;
     const int units = D / vec;                                    // per row
     const int lanes = units >= (int)blockDim.x ? (int)blockDim.x : (units < 1 ? 1 : units);
@@ -158,7 +159,7 @@ int run_gather_next(const float* vars_a, const float* vars_b, const SplitPop& po
                     cudaStream_t stream)
 {
     gather_next<<<gather_blocks(N, D), 256, 0, stream>>>(vars_a, vars_b, pop, survivors, fronts, N, D, M, vars,
-                                                          objs, cv, rank);
+                                                          objs, cv, rank, nullptr);
     MOEA_CUDA_TRY(cudaGetLastError());
     return MOEA_OK;
 }
@@ -723,7 +724,7 @@ struct moea_algorithm {
             MOEA_TRY(run_nsga3_select(ws, pop, M, N, refs, H, seed, ideal_last, survivors, nullptr,
                                       assoc_mode(), stream, &sort_pop));
             gather_next<<<gather_blocks(N, D), 256, 0, stream>>>(
-                vars[P], vars[O], pop, survivors, ws.fronts, N, D, M, vars[X], objs[X], cv[X], rank[X]);
+                vars[P], vars[O], pop, survivors, ws.fronts, N, D, M, vars[X], objs[X], cv[X], rank[X], d_gen);
             MOEA_CUDA_TRY(cudaGetLastError());
         } else {
             if (rvea_block_eligible(2 * N, M, H)) {
@@ -741,7 +742,7 @@ struct moea_algorithm {
             MOEA_TRY(run_rvea_update(pop, vars[P], vars[O], survivors, d_active, N, D, M, vars[X], objs[X],
                                      cv[X], stream, nan_rows + X));
         }
-        bump_generation<<<1, 1, 0, stream>>>(d_gen);
+        if (!nsga3()) bump_generation<<<1, 1, 0, stream>>>(d_gen);
         MOEA_CUDA_TRY(cudaGetLastError());
         stage_mark("survivors", stream);
         return MOEA_OK;
@@ -1164,7 +1165,8 @@ BatchInst fused_describe(moea_algorithm* a, int P, int X)
     b.front_list = w.front_list; b.counters = w.counters; b.rows = w.rows;
     b.fronts = w.fronts; b.nds_gidx = w.nds_gidx; b.sizes = w.sizes;
     b.nds_objs = w.nds_objs; b.rcp_b = w.rcp_b; b.extreme = w.extreme; b.assoc_idx = w.assoc_idx;
-    b.assoc_dist = w.assoc_dist; b.rho = w.rho; b.selected = w.selected; b.flags = w.flags;
+    b.assoc_dist = w.assoc_dist; b.rho = w.rho; b.niche_last = w.niche_last; b.niche_start = w.niche_start;
+    b.niche_hist = w.niche_hist; b.selected = w.selected; b.flags = w.flags;
     b.survivors = a->survivors; b.offset = w.offset_dev;
     b.t_dirs_orig = a->refs;
     b.t_dirs = w.tree_dirs; b.t_order = w.tree_order; b.t_center = w.tree_center; b.t_cos = w.tree_cos;

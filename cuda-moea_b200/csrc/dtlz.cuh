@@ -5,6 +5,7 @@
 #include <math_constants.h>
 
 #include "internal.cuh"
+#include "variation.cuh"
 
 namespace moea {
 namespace {
@@ -24,15 +25,32 @@ __host__ __device__ inline int base_kind(int kind)
     }
 }
 
+// The math functions as calls for the kernels that hold many of them (see
+// powf_call).
+__device__ __noinline__ float cosf_call(float a) { return cosf(a); }
+__device__ __noinline__ float sinf_call(float a) { return sinf(a); }
+template <bool kCall>
+__device__ __forceinline__ float cosine(float a)
+{
+    if constexpr (kCall) return cosf_call(a);
+    else return cosf(a);
+}
+template <bool kCall>
+__device__ __forceinline__ float sine(float a)
+{
+    if constexpr (kCall) return sinf_call(a);
+    else return sinf(a);
+}
+
 // One g-term added to a running partial.
-template <int B>
+template <int B, bool kCall = false>
 __device__ __forceinline__ float g_accumulate(float thread_sum, float xv)
 {
     if (B == kDTLZ1 || B == kDTLZ3) {
         const float val = xv - 0.5f;
-        thread_sum += val * val - cosf(20.0f * M_PI * val);
+        thread_sum += val * val - cosf(20.0f * M_PI * val);  // contracted with the cosine's last product: inline
     } else if (B == kDTLZ6) {
-        thread_sum += powf(xv, 0.1f);
+        thread_sum += power<kCall>(xv, 0.1f);
     } else if (B == kDTLZ7) {
         thread_sum += xv;
     } else {
@@ -126,17 +144,17 @@ __device__ float row_objective(int m, float total_sum, const float* x, int D, in
 // The two factors of position variable q that row_objective evaluates (with its
 // multiply-adds spelled out): cosine
 // and sine of its angle, or the factors of its term in DTLZ7's h.
-template <int B>
+template <int B, bool kCall>
 __device__ __forceinline__ void row_factors(int q, float total_sum, const float* x, int D, int M, float* a, float* b)
 {
     const int k = D - (M - 1);
     if (B == kDTLZ2 || B == kDTLZ3 || B == kConvexDTLZ2) {
-        *a = safe_cos_hp(x[q]);
-        *b = sinf(x[q] * M_PI / 2.0f);
+        *a = fmaxf(0.0f, cosine<kCall>(x[q] * M_PI / 2.0f));
+        *b = sine<kCall>(x[q] * M_PI / 2.0f);
     } else if (B == kDTLZ4) {
-        const float p = powf(x[q], 100.0f);
-        *a = fmaxf(0.0f, cosf(p * M_PI / 2.0f));
-        *b = sinf(p * M_PI / 2.0f);
+        const float p = power<kCall>(x[q], 100.0f);
+        *a = fmaxf(0.0f, cosine<kCall>(p * M_PI / 2.0f));
+        *b = sine<kCall>(p * M_PI / 2.0f);
     } else if (B == kDTLZ5 || B == kDTLZ6) {
         const float g = total_sum;
         float t = x[0];
@@ -144,13 +162,13 @@ __device__ __forceinline__ void row_factors(int q, float total_sum, const float*
             t = fmaf(2.0f * g, x[q], 1.0f) / (2.0f * (1.0f + g));
             if (B == kDTLZ5) t = fmaxf(0.0f, fminf(1.0f, t));
         }
-        *a = (B == kDTLZ5) ? fmaxf(0.0f, __cosf(t * M_PI * 0.5f)) : fmaxf(0.0f, cosf(t * M_PI * 0.5f));
-        *b = (B == kDTLZ5) ? __sinf(t * M_PI * 0.5f) : sinf(t * M_PI * 0.5f);
+        *a = (B == kDTLZ5) ? fmaxf(0.0f, __cosf(t * M_PI * 0.5f)) : fmaxf(0.0f, cosine<kCall>(t * M_PI * 0.5f));
+        *b = (B == kDTLZ5) ? __sinf(t * M_PI * 0.5f) : sine<kCall>(t * M_PI * 0.5f);
     } else {  // kDTLZ7
         const float g = fmaf(9.0f / static_cast<float>(k), total_sum, 1.0f);
         const float fi = x[q];
         *a = fi / (1.0f + g);
-        *b = 1.0f + sinf(3.0f * M_PI * fi);
+        *b = 1.0f + sine<kCall>(3.0f * M_PI * fi);
     }
 }
 
@@ -194,24 +212,21 @@ __device__ __forceinline__ float combine_factors(int m, float total_sum, const f
 // g-terms.  Every lane of the warp calls; rows that are not `valid` write
 // nothing.  The partials are those of a shuffle-down tree over 32 lanes: with
 // G = 8 a lane holds four of its leaves and folds the first two levels itself.
-template <int B, int G>
+template <int B, int G, bool kCall = false>
 __device__ __forceinline__ void dtlz_group_row(int row, bool valid, int gl, const float* x, int N, int D, int M,
                                                float* objs)
 {
     constexpr int kLeaves = 32 / G;
     const int start = (B == kDTLZ7) ? D - (D - M + 1) : M - 1;
     const int k = D - start;
-    float ws[8];
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-        ws[w] = 0.0f;  // no term: the tree of zeros
-        if (32 * w >= k) continue;
+    // partial w: the tree over the terms 32 w .. 32 w + 31 (zero without terms)
+    auto partial = [&](int w) {
         float v[kLeaves];
 #pragma unroll
         for (int i = 0; i < kLeaves; ++i) {
             const int t = gl + G * i + 32 * w;
             v[i] = 0.0f;
-            if (valid && t < k) v[i] = g_accumulate<B>(v[i], x[start + t]);
+            if (valid && t < k) v[i] = g_accumulate<B, kCall>(v[i], x[start + t]);
         }
 #pragma unroll
         for (int o = kLeaves / 2; o > 0; o >>= 1)
@@ -219,9 +234,19 @@ __device__ __forceinline__ void dtlz_group_row(int row, bool valid, int gl, cons
             for (int i = 0; i < o; ++i) v[i] += v[i + o];
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) v[0] += __shfl_down_sync(0xFFFFFFFFu, v[0], o, G);
-        ws[w] = v[0];
+        return v[0];
+    };
+    float total = 0.0f;
+    if constexpr (B == kDTLZ5) {
+        float ws[8];
+#pragma unroll
+        for (int w = 0; w < 8; ++w) ws[w] = 32 * w < k ? partial(w) : 0.0f;
+        total = fold_partials<B>(ws);
+    } else {
+        // in order, as fold_partials adds them
+#pragma unroll 1
+        for (int w = 0; 32 * w < k; ++w) total += partial(w);
     }
-    float total = (gl == 0) ? fold_partials<B>(ws) : 0.0f;
     total = __shfl_sync(0xFFFFFFFFu, total, 0, G);
     if constexpr (B == kDTLZ1) {
         if (valid)
@@ -238,7 +263,7 @@ __device__ __forceinline__ void dtlz_group_row(int row, bool valid, int gl, cons
         for (int v = 0; v < kSlots; ++v) {
             const int q = gl + G * v;
             fa[v] = fb[v] = 0.0f;
-            if (valid && q < M - 1) row_factors<B>(q, total, x, D, M, &fa[v], &fb[v]);
+            if (valid && q < M - 1) row_factors<B, kCall>(q, total, x, D, M, &fa[v], &fb[v]);
         }
         auto pick = [&](const float (&f)[kSlots], int q) {  // factor q of the row, by every lane
             float r = 0.0f;

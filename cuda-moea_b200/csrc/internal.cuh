@@ -287,7 +287,8 @@ struct BatchInst {
     int* blocker; int* front_sorted; int* front_list; int* counters;
     uint32_t* rows;
     int* fronts; int* nds_gidx; int* sizes; float* nds_objs; float* rcp_b; int* extreme;
-    int* assoc_idx; float* assoc_dist; int* rho; int* selected; int* flags; int* survivors;
+    int* assoc_idx; float* assoc_dist; int* selected; int* flags; int* survivors;
+    int* rho; int* niche_last; int* niche_start; int* niche_hist;
     unsigned long long* offset;
     const float* t_dirs_orig;  // (M, H) directions in their own order
     const float* t_dirs; const int* t_order; const float* t_center; const float* t_cos;

@@ -1920,6 +1920,7 @@ fused_peel(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
                 if (ck == 0 && total < target) atomicExch(I.counters + 6, kDevPeelInconsistent);
             }
             for (int i = t; i < len; i += blockDim.x) I.front_list[i] = list[i];
+            for (int q = t; q < n; q += blockDim.x) I.fronts[I.perm[q]] = I.front_sorted[q];
             return;
         }
         if (t == 0) s_qn = 0;
@@ -2013,13 +2014,6 @@ fused_peel(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
         len = s_cnt;
         ++k;
     }
-}
-
-__global__ void fused_scatter(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
-{
-    const BatchInst& I = insts[ids[blockIdx.y]];
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos < I.n) I.fronts[I.perm[pos]] = I.front_sorted[pos];
 }
 
 template <int M>
@@ -2311,7 +2305,6 @@ int fused_ndsort(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s)
         }
     }
     fused_peel<<<g.count, kFusedPeelThreads, fused_peel_smem(g.max_W, g.max_n), s>>>(d_inst, g.d_ids);
-    fused_scatter<<<dim3(ceil_div(g.max_n, 256), g.count), 256, 0, s>>>(d_inst, g.d_ids);
     MOEA_CUDA_TRY(cudaGetLastError());
     return MOEA_OK;
 }

@@ -1381,28 +1381,17 @@ __device__ __forceinline__ void fused_niching_sorted(const BatchInst& I, FusedSe
     }
 }
 
-// Niche selection of one instance per CTA: run_niching with block sorts.
-__global__ void __launch_bounds__(kFusedThreads)
-fused_niching(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
+// The niche selection of one instance by one CTA with sorts, for a last front
+// that a few directions hold (niche_buckets declined; I.rho is complete): up to
+// kFusedThreads members each stage counts, for every member, the members before
+// it, above it is a stable block sort.  Leaves the selection in I.selected.
+__device__ void fused_niching_sorts(const BatchInst& I, unsigned char* smem, int np, int nl, int nrem, int H,
+                                    unsigned long long off)
 {
-    extern __shared__ __align__(16) unsigned char fused_smem[];
-    FusedSelStorage& tmp = *reinterpret_cast<FusedSelStorage*>(fused_smem);
-    const BatchInst& I = insts[ids[blockIdx.x]];
+    FusedSelStorage& tmp = *reinterpret_cast<FusedSelStorage*>(smem);
     const int t = threadIdx.x;
-    const int np = I.sizes[0], nl = I.sizes[1], nrem = I.sizes[2], H = I.H;
-    const unsigned long long off = *I.offset;
-    for (int r = t; r < H; r += kFusedThreads) I.rho[r] = 0;
-    __syncthreads();
-    for (int i = t; i < np; i += kFusedThreads) {
-        I.selected[i] = I.nds_gidx[i];
-        const int r = I.assoc_idx[i];
-        if (r >= 0 && r < H) atomicAdd(I.rho + r, 1);
-    }
     if (nl <= kFusedThreads) {
-        // Small fronts: each stage is a stable sort by (key, position), done by
-        // counting for every member the members before it, instead of block
-        // sorts sized for kFusedMaxPoints.  Same orders, same random words.
-        uint64_t* s_key = reinterpret_cast<uint64_t*>(fused_smem);   // [2][kFusedThreads]
+        uint64_t* s_key = reinterpret_cast<uint64_t*>(smem);   // [2][kFusedThreads]
         int* s_val = reinterpret_cast<int*>(s_key + 2 * kFusedThreads);  // [2][kFusedThreads]
         int* s_wmax = s_val + 2 * kFusedThreads;                        // [kFusedThreads / 32]
         int cur = 0;
@@ -1467,45 +1456,52 @@ fused_niching(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
     } else {
         fused_niching_sorted<kFusedItems>(I, tmp, np, nl, nrem, H, off);
     }
-    if (t == 0) *I.offset = off + 2ull * (unsigned long long)nl;
 }
 
-// Survivors in ascending mixed index (run_order_selection) of one instance per CTA.
-__global__ void __launch_bounds__(kFusedThreads)
-fused_order(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
+// Niche selection and ascending survivors of every instance, two CTAs each
+// (niche_select.cuh): the sorts of one CTA per instance took 220 us over 256
+// instances and the survivor order 10.
+constexpr int kFusedNicheCtas = 2;
+constexpr int kFusedNicheItems = kFusedMaxPoints / (kFusedThreads * kFusedNicheCtas);
+union FusedNicheShared {
+    NicheShared<kFusedThreads, kFusedNicheItems> buckets;
+    FusedSelStorage sorts;
+};
+
+__global__ void __cluster_dims__(kFusedNicheCtas, 1, 1) __launch_bounds__(kFusedThreads)
+fused_niche_select(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
 {
-    __shared__ typename FusedScanInt::TempStorage scan_tmp;
-    __shared__ unsigned char s_flag[kFusedMaxPoints];
-    const BatchInst& I = insts[ids[blockIdx.x]];
-    const int t = threadIdx.x, n = I.n, N = I.N;
-    for (int i = t; i < kFusedMaxPoints; i += kFusedThreads) s_flag[i] = 0;
-    __syncthreads();
-    for (int i = t; i < N; i += kFusedThreads) s_flag[I.selected[i]] = 1;
-    __syncthreads();
-    int c = 0;
-#pragma unroll
-    for (int j = 0; j < kFusedItems; ++j) {
-        const int i = t * kFusedItems + j;
-        c += (i < n && s_flag[i]) ? 1 : 0;
+    extern __shared__ __align__(16) unsigned char fused_smem[];
+    FusedNicheShared& sm = *reinterpret_cast<FusedNicheShared*>(fused_smem);
+    NicheCluster grp;
+    const BatchInst& I = insts[ids[blockIdx.x / kFusedNicheCtas]];
+    const int c = grp.rank();
+    const int np = I.sizes[0], nl = I.sizes[1], nrem = I.sizes[2];
+    const unsigned long long off = *I.offset;
+    const NicheScratch S{I.rho, I.niche_last, I.niche_start, I.key64, I.key64b, I.vals,
+                         reinterpret_cast<uint32_t*>(I.flags), I.niche_hist};
+    if (!niche_buckets<kFusedThreads, kFusedNicheItems>(grp, sm.buckets, S, I.assoc_idx, I.assoc_dist, I.nds_gidx, np, nl,
+                                                        nrem, I.H, I.nich_seed, off, I.n)) {
+        if (c == 0) {
+            fused_niching_sorts(I, fused_smem, np, nl, nrem, I.H, off);
+            __syncthreads();
+            for (int i = threadIdx.x; i < min(nrem, nl); i += kFusedThreads) niche_mark(S.mask, I.selected[np + i]);
+        }
+        grp.sync();
     }
-    FusedScanInt(scan_tmp).ExclusiveSum(c, c);
-#pragma unroll
-    for (int j = 0; j < kFusedItems; ++j) {
-        const int i = t * kFusedItems + j;
-        if (i < n && s_flag[i]) I.survivors[c++] = i;
-    }
+    if (c == 0 && threadIdx.x == 0) *I.offset = off + 2ull * (unsigned long long)nl;
+    niche_survivors<kFusedThreads, kFusedNicheItems>(grp, sm.buckets, S.mask, I.n, I.survivors, I.N);
 }
 
-// Next parents from the survivors (gather_next), then the generation counter.
+// Next parents from the survivors (gather_next), and the generation counter.
 __global__ void fused_gather(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
 {
     const BatchInst& I = insts[ids[blockIdx.y]];
     const int N = I.N, D = I.D, M = I.M;
     const SplitPop pop{I.objsP, I.objsO, I.cvP, I.cvO, N, N, N, I.n};
-    const long long total = (long long)N * D;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(e / D), d = (int)(e % D);
+    const unsigned total = (unsigned)N * (unsigned)D;  // at most 4096 x 271
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
+        const unsigned r = e / (unsigned)D, d = e - r * (unsigned)D;
         const int s = I.survivors[r];
         I.varsX[e] = (s < N) ? I.varsP[(size_t)s * D + d] : I.varsO[(size_t)(s - N) * D + d];
     }
@@ -1515,12 +1511,7 @@ __global__ void fused_gather(const BatchInst* __restrict__ insts, const int* __r
         I.cvX[r] = pop.cvv(s);
         I.rankX[r] = I.fronts[s];
     }
-}
-
-__global__ void fused_bump(const BatchInst* __restrict__ insts, const int* __restrict__ ids, int count)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < count) *insts[ids[k]].d_gen += 1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *I.d_gen += 1;  // the generation's last launch
 }
 
 }  // namespace
@@ -1842,14 +1833,13 @@ int run_quantize_cv(const float* cv, float* out, int n, float eps, float clip, f
 
 int fused_select_configure()
 {
-    MOEA_CUDA_TRY(cudaFuncSetAttribute(fused_niching, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sizeof(FusedSelStorage)));
+    MOEA_CUDA_TRY(cudaFuncSetAttribute(fused_niche_select, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(FusedNicheShared)));
     return MOEA_OK;
 }
 
 int fused_select(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s)
 {
-    const int sort_smem = (int)sizeof(FusedSelStorage);
     for (const FusedBucket& b : g.buckets) {
         switch (b.M) {
 #define MOEA_FP_CASE(K)                                                                              \
@@ -1870,12 +1860,10 @@ int fused_select(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s)
         }
     }
     MOEA_CUDA_TRY(cudaGetLastError());
-    fused_niching<<<g.count, kFusedThreads, sort_smem, s>>>(d_inst, g.d_ids);
-    fused_order<<<g.count, kFusedThreads, 0, s>>>(d_inst, g.d_ids);
+    fused_niche_select<<<g.count * kFusedNicheCtas, kFusedThreads, sizeof(FusedNicheShared), s>>>(d_inst, g.d_ids);
     const long long per = (long long)g.max_N * g.max_D;
     const unsigned gx = (unsigned)std::min<long long>(64, (per + 255) / 256);
     fused_gather<<<dim3(gx, g.count), 256, 0, s>>>(d_inst, g.d_ids);
-    fused_bump<<<ceil_div(g.count, 256), 256, 0, s>>>(d_inst, g.d_ids, g.count);
     MOEA_CUDA_TRY(cudaGetLastError());
     return MOEA_OK;
 }

@@ -39,21 +39,21 @@ __device__ __forceinline__ void offspring_pair(int p, float* rows, const Offspri
     const float eta_c = annealed_eta(A.sbx_eta0, A.sbx_eta1, (int)gen, A.total);
     if (children)
         for (int j = gl; j < D4; j += G)
-            crossover_group(p * D4 + j, p, j, A.parents, A.pidx, A.bounds, base, pairs, D, A.vec != 0, eta_c, A.sbx_prob,
+            crossover_group<true>(p * D4 + j, p, j, A.parents, A.pidx, A.bounds, base, pairs, D, A.vec != 0, eta_c, A.sbx_prob,
                             A.copy_prob, A.seed, gen);
     __syncwarp();
     if (A.mutate) {
         const bool mine = (gl >> 2) < children;  // four lanes per child
-        mutate_child4(mine ? ca + (gl >> 2) : ca, mine, gl & 3, base, A.bounds, A.n_off, D,
+        mutate_child4<true>(mine ? ca + (gl >> 2) : ca, mine, gl & 3, base, A.bounds, A.n_off, D,
                       annealed_eta(A.pm_eta0, A.pm_eta1, (int)gen, A.total), A.pm_prob, A.seed, gen);
         __syncwarp();
     }
     for (int i = gl; i < children * D; i += G) A.off[(size_t)ca * D + i] = rows[i];
     if constexpr (B != 0) {
-#pragma unroll
+#pragma unroll 1
         for (int h = 0; h < 2; ++h) {
             const int r = ca + h;
-            dtlz_group_row<B, G>(r, h < children, gl, rows + (size_t)h * D, A.n_off, D, A.M, A.objs);
+            dtlz_group_row<B, G, true>(r, h < children, gl, rows + (size_t)h * D, A.n_off, D, A.M, A.objs);
             if (A.kind >= 9) __syncwarp();  // the row's objectives, written by the group's other lanes
             if (gl == 0 && h < children)
                 A.cv_out[r] = A.kind >= 9 && (!A.cv_table || A.cv_table[gen])
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kOffThreads) offspring_kernel(OffspringArgs A)
 // Every instance of a batch (blockIdx.y): problem kinds 1..8, whose violation
 // is zero.  Batches fill the device, so a pair takes eight lanes.
 constexpr int kFusedGroup = 8;
-__global__ void __launch_bounds__(kOffThreads)
+__global__ void __launch_bounds__(kOffThreads, 3)
 fused_offspring(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
 {
     extern __shared__ __align__(16) float off_rows[];

@@ -31,8 +31,21 @@ __device__ __forceinline__ float annealed_eta(float begin, float end, int gen, i
     return __fadd_rn(begin, __fmul_rn(__fsub_rn(end, begin), p));
 }
 
+// powf as a call (the same function, one copy of its code in a kernel).  The
+// kernels that do everything for a pair of children hold up to a dozen powf,
+// sinf and cosf; inlined, their code outgrew the instruction cache (a batch of
+// mixed problems: 4.8 of 11 stall cycles per instruction were fetches).
+__device__ __noinline__ float powf_call(float a, float b) { return powf(a, b); }
+template <bool kCall>
+__device__ __forceinline__ float power(float a, float b)
+{
+    if constexpr (kCall) return powf_call(a, b);
+    else return powf(a, b);
+}
+
 // SBX on one variable pair (sbx_crossover.cu:44-70).  Returns false when the
 // pair is copied unchanged.
+template <bool kCall = false>
 __device__ __forceinline__ void sbx_pair(float x1, float x2, float u1, float u2, int sign,
                                          float copy, float eta, float prob, float copy_prob,
                                          float lo, float hi, float& c1, float& c2)
@@ -42,11 +55,11 @@ __device__ __forceinline__ void sbx_pair(float x1, float x2, float u1, float u2,
         c2 = x2;
         return;
     }
-    const float power = 1.0f / (1.0f + eta);
+    const float exponent = 1.0f / (1.0f + eta);
     // one powf on the selected base (the same value as calling it in either
     // branch, without a warp running both when its lanes disagree)
     const float base = u1 < 0.5f ? 2.0f * u1 : 1.0f / (2.0f - 2.0f * u1);
-    float beta = powf(base, power);
+    float beta = power<kCall>(base, exponent);
     beta *= 2 * sign - 1;
     const float midpoint = 0.5f * (x1 + x2);
     const float delta = 0.5f * beta * (x1 - x2);
@@ -55,6 +68,9 @@ __device__ __forceinline__ void sbx_pair(float x1, float x2, float u1, float u2,
 }
 
 // Deb's bounded polynomial mutation of one value (polynomial_mutation.cu:30-59).
+// The outer powf stay inline: their last product is contracted with the
+// subtraction, so as a call they would round differently.
+template <bool kCall = false>
 __device__ __forceinline__ float pm_value(float value, float u1, float u2, float eta, float prob,
                                           int D, float lo, float hi)
 {
@@ -65,11 +81,11 @@ __device__ __forceinline__ float pm_value(float value, float u1, float u2, float
     float delta;
     if (u2 <= 0.5f) {
         const float xy = 1.0f - normalized;
-        const float value_mut = 2.0f * u2 + (1.0f - 2.0f * u2) * powf(xy, exponent);
+        const float value_mut = 2.0f * u2 + (1.0f - 2.0f * u2) * power<kCall>(xy, exponent);
         delta = powf(value_mut, 1.0f / exponent) - 1.0f;
     } else {
         const float xy = normalized;
-        const float value_mut = 2.0f * (1.0f - u2) + 2.0f * (u2 - 0.5f) * powf(xy, exponent);
+        const float value_mut = 2.0f * (1.0f - u2) + 2.0f * (u2 - 0.5f) * power<kCall>(xy, exponent);
         delta = 1.0f - powf(value_mut, 1.0f / exponent);
     }
     return fminf(fmaxf(value + delta * range, lo), hi);
@@ -115,6 +131,7 @@ __device__ __forceinline__ void mating_child(int i, const float* __restrict__ cv
 // variable mutation test: at large D the variation is then bound by its
 // powf and its HBM stream, not by Philox rounds.
 
+template <bool kCall = false>
 __device__ __forceinline__ void crossover_group(int t, int p, int j, const float* __restrict__ parents,
                                                 const int* __restrict__ pidx, const float* __restrict__ bounds,
                                                 float* __restrict__ off, int pairs, int D, bool vec, float eta_c,
@@ -156,7 +173,7 @@ __device__ __forceinline__ void crossover_group(int t, int p, int j, const float
     float c1[4], c2[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-        sbx_pair(a[i], bv[i], u32_to_unit(r[i]), u32_to_unit(rt[i]), (int)(r[i] & 1u), u32_to_unit(rc[i]), eta_c,
+        sbx_pair<kCall>(a[i], bv[i], u32_to_unit(r[i]), u32_to_unit(rt[i]), (int)(r[i] & 1u), u32_to_unit(rc[i]), eta_c,
                  sbx_prob, copy_prob, lo[i], hi[i], c1[i], c2[i]);
     float* oa = off + (size_t)ca * D + d0;
     float* ob = off + (size_t)cb * D + d0;
@@ -177,6 +194,7 @@ __device__ __forceinline__ void crossover_group(int t, int p, int j, const float
 // mutates its own site (sites are distinct).  Each draw moves the site by at
 // least one, so a child takes at most D/4 + 1 rounds.  All four lanes of the
 // group call this together (c and `active` uniform within the group).
+template <bool kCall = false>
 __device__ __forceinline__ void mutate_child4(int c, bool active, int sub, float* __restrict__ off,
                                               const float* __restrict__ bounds, int n_off, int D, float eta_m,
                                               float pm_prob, uint64_t seed, uint32_t gen)
@@ -209,7 +227,7 @@ __device__ __forceinline__ void mutate_child4(int c, bool active, int sub, float
         if (live && my_site < D) {
             const int d = (int)my_site;
             // test draw 0 < limit: the site mutates (pm_value's own test passes)
-            row[d] = pm_value(row[d], 0.0f, u32_to_unit(w[1]), eta_m, pm_prob, D, bounds[2 * d], bounds[2 * d + 1]);
+            row[d] = pm_value<kCall>(row[d], 0.0f, u32_to_unit(w[1]), eta_m, pm_prob, D, bounds[2 * d], bounds[2 * d + 1]);
         }
         site = __shfl_sync(group, my_site, 3, 4);
         live = live && site < D;
