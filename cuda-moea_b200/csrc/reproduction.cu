@@ -11,6 +11,8 @@
 // every GPU, and the streams can be regenerated on the host for checking.  The
 // `*_explicit` kernels take the draws as arrays instead, which is how the
 // stage parity tests feed identical numbers to the oracle.
+#include <algorithm>
+
 #include "internal.cuh"
 #include "variation.cuh"
 
@@ -94,6 +96,52 @@ __global__ void crossover_philox(const float* __restrict__ parents, const int* _
     }
 }
 
+// Crossover of long rows (D a multiple of 4, 16-byte aligned): blockIdx.y walks
+// the pairs and blockIdx.x the groups of four variables, so a thread divides
+// nothing and its block reads the parent indices once; kPlain: every variable
+// is crossed (no test or copy draw can change it).  Bound by instruction issue
+// (the powf): at D = 131072, 512 pairs, the flat kernel above spent a fifth of
+// its instructions on the 64-bit division of its group index and the tests
+// (378 -> 317 us a launch).
+template <bool kPlain>
+__global__ void __launch_bounds__(256)
+crossover_rows(const float* __restrict__ parents, const int* __restrict__ pidx, const float* __restrict__ bounds,
+               float* __restrict__ off, int pairs, int D, float sbx_eta0, float sbx_eta1, float sbx_prob,
+               float copy_prob, int total, uint64_t seed, const int* __restrict__ d_gen, uint32_t gen_host)
+{
+    const int D4 = D >> 2;
+    const uint32_t gen = d_gen ? (uint32_t)*d_gen : gen_host;
+    const float eta = annealed_eta(sbx_eta0, sbx_eta1, (int)gen, total);
+    for (int p = blockIdx.y; p < pairs; p += gridDim.y) {
+        const float4* xa = reinterpret_cast<const float4*>(parents + (size_t)pidx[2 * p] * D);
+        const float4* xb = reinterpret_cast<const float4*>(parents + (size_t)pidx[2 * p + 1] * D);
+        float4* oa = reinterpret_cast<float4*>(off + (size_t)(2 * p) * D);
+        float4* ob = oa + D4;
+        for (int j = blockIdx.x * 256 + threadIdx.x; j < D4; j += gridDim.x * 256) {
+            const float4 a4 = __ldg(xa + j), b4 = __ldg(xb + j);
+            const float4 l01 = __ldg(reinterpret_cast<const float4*>(bounds) + 2 * j);
+            const float4 l23 = __ldg(reinterpret_cast<const float4*>(bounds) + 2 * j + 1);
+            const uint64_t block = (uint64_t)((uint32_t)p * (uint32_t)D4 + (uint32_t)j);
+            uint32_t r[4], rt[4] = {0u, 0u, 0u, 0u}, rc[4] = {0u, 0u, 0u, 0u};
+            rng_block(seed, block, gen, kTagCrossover, r);
+            if (!kPlain) {
+                if (sbx_prob < 1.0f) rng_block(seed, block, gen, kTagCrossTest, rt);
+                if (copy_prob > 0.0f) rng_block(seed, block, gen, kTagCopy, rc);
+            }
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+            const float lo[4] = {l01.x, l01.z, l23.x, l23.z}, hi[4] = {l01.y, l01.w, l23.y, l23.w};
+            float c1[4], c2[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                sbx_pair(a[i], b[i], u32_to_unit(r[i]), kPlain ? 0.0f : u32_to_unit(rt[i]), (int)(r[i] & 1u),
+                         kPlain ? 0.0f : u32_to_unit(rc[i]), eta, kPlain ? 1.0f : sbx_prob, kPlain ? 0.0f : copy_prob,
+                         lo[i], hi[i], c1[i], c2[i]);
+            oa[j] = make_float4(c1[0], c1[1], c1[2], c1[3]);
+            ob[j] = make_float4(c2[0], c2[1], c2[2], c2[3]);
+        }
+    }
+}
+
 __global__ void mutation_philox(float* __restrict__ off, const float* __restrict__ bounds, int n_off, int D,
                                 float pm_eta0, float pm_eta1, float pm_prob, int total, uint64_t seed,
                                 const int* __restrict__ d_gen, uint32_t gen_host)
@@ -115,19 +163,47 @@ __global__ void rng_blocks_kernel(uint64_t seed, uint32_t gen, uint32_t tag, lon
     out[e] = make_uint4(r[0], r[1], r[2], r[3]);
 }
 
-// x = lb + u (ub - lb) (population.cu:12-24, 97-115) with Philox draws.
-__global__ void init_uniform(float* __restrict__ vars, const float* __restrict__ bounds,
-                             long long count, int D, uint64_t seed)
+// x = lb + u (ub - lb) (population.cu:12-24, 97-115) with Philox draws: a
+// thread takes the four elements of one block of draws (one element per thread,
+// each with the whole block and a 64-bit remainder, took 773 us for 134 M
+// elements; 164 us now).
+__global__ void init_uniform(float* __restrict__ vars, const float* __restrict__ bounds, long long count, int D,
+                             uint64_t seed)
 {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= count) return;
-    uint32_t r[4];
-    rng_block(seed, (uint64_t)(e >> 2), 0u, kTagInit, r);
-    const float u = u32_to_unit(r[e & 3]);
-    const int d = (int)(e % D);
-    const float lower = bounds[2 * d], upper = bounds[2 * d + 1];
-    vars[e] = lower + u * (upper - lower);
+    const long long blocks = (count + 3) >> 2;
+    const long long step = (long long)gridDim.x * blockDim.x;
+    long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    int d = (int)((4 * e) % D);
+    const int advance = (int)((4 * step) % D);
+    const bool vec = (D & 3) == 0 && ((uintptr_t)vars & 15) == 0 && ((uintptr_t)bounds & 15) == 0;
+    for (; e < blocks; e += step) {
+        uint32_t r[4];
+        rng_block(seed, (uint64_t)e, 0u, kTagInit, r);
+        if (vec) {  // D a multiple of 4: the four elements are one aligned group of a row
+            const float4 l01 = __ldg(reinterpret_cast<const float4*>(bounds + 2 * d));
+            const float4 l23 = __ldg(reinterpret_cast<const float4*>(bounds + 2 * d) + 1);
+            reinterpret_cast<float4*>(vars)[e] =
+                make_float4(l01.x + u32_to_unit(r[0]) * (l01.y - l01.x), l01.z + u32_to_unit(r[1]) * (l01.w - l01.z),
+                            l23.x + u32_to_unit(r[2]) * (l23.y - l23.x), l23.z + u32_to_unit(r[3]) * (l23.w - l23.z));
+            d += advance;
+            if (d >= D) d -= D;
+            continue;
+        }
+        int dk = d;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (4 * e + k < count) {
+                const float lower = bounds[2 * dk], upper = bounds[2 * dk + 1];
+                vars[4 * e + k] = lower + u32_to_unit(r[k]) * (upper - lower);
+            }
+            dk = dk + 1 < D ? dk + 1 : 0;
+        }
+        d += advance;
+        if (d >= D) d -= D;
+    }
 }
+
+constexpr int kRowCrossoverD = 1024;  // rows from which a block of 256 groups is one row's
 
 inline int grid_for(long long count, int threads, int cap = 148 * 32)
 {
@@ -157,9 +233,21 @@ int run_variation_pass(int passes, const float* parents, const int* pidx, const 
         // 16-byte loads and stores when every row and the bounds are aligned
         const bool vec = (D & 3) == 0 && ((uintptr_t)parents & 15) == 0 && ((uintptr_t)off & 15) == 0 &&
                          ((uintptr_t)bounds & 15) == 0;
-        crossover_philox<<<grid_for(count, 256), 256, 0, stream>>>(parents, pidx, bounds, off, n_off, D, vec,
-                                                                   sbx_eta0, sbx_eta1, sbx_prob, copy_prob, total,
-                                                                   seed, d_gen, gen);
+        if (vec && D >= kRowCrossoverD && (n_off & 1) == 0 && count < (1ll << 31)) {
+            // 32 blocks per SM in flight, rows split into blocks of 256 groups
+            const int gx = std::min(ceil_div(D / 4, 256), 64);
+            const dim3 grid(gx, std::max(1, std::min(n_off / 2, 148 * 32 / gx)));
+            if (sbx_prob >= 1.0f && copy_prob <= 0.0f)
+                crossover_rows<true><<<grid, 256, 0, stream>>>(parents, pidx, bounds, off, n_off / 2, D, sbx_eta0, sbx_eta1,
+                                                               sbx_prob, copy_prob, total, seed, d_gen, gen);
+            else
+                crossover_rows<false><<<grid, 256, 0, stream>>>(parents, pidx, bounds, off, n_off / 2, D, sbx_eta0,
+                                                                sbx_eta1, sbx_prob, copy_prob, total, seed, d_gen, gen);
+        } else {
+            crossover_philox<<<grid_for(count, 256), 256, 0, stream>>>(parents, pidx, bounds, off, n_off, D, vec,
+                                                                       sbx_eta0, sbx_eta1, sbx_prob, copy_prob, total,
+                                                                       seed, d_gen, gen);
+        }
         MOEA_CUDA_TRY(cudaGetLastError());
     }
     if ((passes & kPassMutation) && mutate && n_off > 0) {
@@ -183,7 +271,7 @@ int run_init_uniform(float* vars, const float* bounds, int N, int D, uint64_t se
                      cudaStream_t stream)
 {
     const long long count = (long long)N * D;
-    init_uniform<<<(int)((count + 255) / 256), 256, 0, stream>>>(vars, bounds, count, D, seed);
+    init_uniform<<<grid_for((count + 3) / 4, 256), 256, 0, stream>>>(vars, bounds, count, D, seed);
     MOEA_CUDA_TRY(cudaGetLastError());
     return MOEA_OK;
 }
