@@ -65,11 +65,12 @@ int run_rvea_elitism(Workspace& ws, const int* idx, const SplitPop& pop, const f
                      int K, int* survivors, int* d_active, cudaStream_t s);
 bool rvea_block_eligible(int n, int M, int K);
 int run_rvea_select_block(const SplitPop& pop, const float* refs, int M, int K, const float* gamma, int* d_active,
-                          int N, const float* ps_table, const int* d_gen, float ps_host, float* t, int t_stride,
-                          float* zmin, float* theta, int* idx, float* apd, int* survivors, cudaStream_t s);
+                          int N, const float* ps_table, int* d_gen, float ps_host, float* t, int t_stride,
+                          float* zmin, float* theta, int* idx, float* apd, int* survivors, int* nan_slot, int* nan_fill,
+                          cudaStream_t s);
 int run_rvea_update(const SplitPop& pop, const float* vars_a, const float* vars_b,
                     const int* survivors, const int* d_active, int N, int D, int M, float* vars,
-                    float* objs, float* cv, cudaStream_t s, int* nan_rows = nullptr);
+                    float* objs, float* cv, cudaStream_t s, int* nan_rows = nullptr, bool mark = true);
 int run_fill_int(int* p, int count, int value, cudaStream_t s);
 int run_rvea_adapt(const float* v0, const float* objs, int stride, const int* d_active,
                    int n_active, int M, int K, float* range_tmp, float* v, cudaStream_t s);
@@ -242,7 +243,7 @@ struct moea_algorithm {
     // fills only the dead rows below it.  Reset whenever the rows may have
     // been written outside the update (start, snapshot load, a population
     // view handed out).
-    int* nan_rows = nullptr;
+    int* nan_rows = nullptr;  // (3), then the count for the update of the generation in flight
     uint64_t seed = 0;
     uint32_t epoch = 0;
     int generation = 0;
@@ -471,7 +472,7 @@ struct moea_algorithm {
         MOEA_TRY(dmalloc(&zmin, (size_t)M));
         MOEA_TRY(dmalloc(&survivors, (size_t)2 * N));
         MOEA_TRY(dmalloc(&frontzero, (size_t)N));
-        MOEA_TRY(dmalloc(&nan_rows, 3));
+        MOEA_TRY(dmalloc(&nan_rows, 4));
         std::vector<float> hb(2 * (size_t)D);
         for (int d = 0; d < D; ++d) {
             hb[2 * d] = lower.empty() ? 0.0f : lower[d];
@@ -727,10 +728,12 @@ struct moea_algorithm {
                 vars[P], vars[O], pop, survivors, ws.fronts, N, D, M, vars[X], objs[X], cv[X], rank[X], d_gen);
             MOEA_CUDA_TRY(cudaGetLastError());
         } else {
-            if (rvea_block_eligible(2 * N, M, H)) {
-                // small merged populations: the whole selection in one CTA
+            const bool block = rvea_block_eligible(2 * N, M, H);
+            if (block) {
+                // small merged populations: the elitism in one CTA
                 MOEA_TRY(run_rvea_select_block(pop, refs, M, H, gamma, d_active, N, ps_table, d_gen, 0.0f, t_buf,
-                                               2 * N, zmin, theta, part_idx, apd, survivors, stream));
+                                               2 * N, zmin, theta, part_idx, apd, survivors, nan_rows + X, nan_rows + 3,
+                                               stream));
             } else {
                 MOEA_TRY(run_rvea_translate(pop, M, t_buf, 2 * N, zmin, stream));
                 MOEA_TRY(run_rvea_partition(t_buf, 2 * N, 2 * N, refs, M, H, d_active, N, N, theta, part_idx,
@@ -740,9 +743,9 @@ struct moea_algorithm {
                 MOEA_TRY(run_rvea_elitism(ws, part_idx, pop, apd, N, H, survivors, d_active, stream));
             }
             MOEA_TRY(run_rvea_update(pop, vars[P], vars[O], survivors, d_active, N, D, M, vars[X], objs[X],
-                                     cv[X], stream, nan_rows + X));
+                                     cv[X], stream, nan_rows + (block ? 3 : X), !block));
+            if (!block) bump_generation<<<1, 1, 0, stream>>>(d_gen);
         }
-        if (!nsga3()) bump_generation<<<1, 1, 0, stream>>>(d_gen);
         MOEA_CUDA_TRY(cudaGetLastError());
         stage_mark("survivors", stream);
         return MOEA_OK;

@@ -409,12 +409,14 @@ __global__ void adapt_kernel(const float* __restrict__ v0, const float* __restri
 //
 // For 2N <= kRveaBlockPoints merged points and K <= kRveaBlockDirs directions
 // the staged translate (two launches), partition, APD and elitism (about ten
-// launches with two library sorts and a scan) become three launches:
-//   rvea_translate_block  one CTA: zmin and the translated objectives;
+// launches with two library sorts and a scan) become two or three launches:
+//   rvea_translate_block  one CTA: zmin and the translated objectives (only
+//                         above kRveaTranslateMax values);
 //   partition_apd_kernel  a warp per point: the partition of partition_kernel
 //                         and, on lane 0, the APD of apd_kernel;
 //   rvea_elite_block      one CTA: each direction's winner, the survivors in
-//                         ascending order and the active count.
+//                         ascending order, the active count, the bookkeeping
+//                         of the dead rows and the generation.
 // Every value comes from the same expressions in the same order as the staged
 // kernels, and the elitism keeps the same survivors:
 //   - the winner of direction j is the point with the smallest
@@ -465,24 +467,54 @@ rvea_translate_block(SplitPop pop, float* __restrict__ t, int t_stride, float* _
         for (int m = 0; m < M; ++m) t[(size_t)m * t_stride + i] = fmaxf(pop.obj(m, i) - s_z[m], 1e-32f);
 }
 
-// partition_kernel with apd_kernel on the warp's lane 0.
-template <int M>
+// partition_kernel with apd_kernel on the warp's lane 0.  kTranslate: the
+// objective minima and the translation too, the minima by every block for
+// itself (a launch of one CTA less; for n M <= kRveaTranslateMax).
+constexpr int kRveaTranslateMax = 16384;
+template <int M, bool kTranslate>
 __global__ void __launch_bounds__(256)
-partition_apd_kernel(const float* __restrict__ t, int t_stride, int n, const float* __restrict__ refs, int K,
+partition_apd_kernel(SplitPop pop, const float* __restrict__ t, int t_stride, int n, const float* __restrict__ refs, int K,
                      const int* __restrict__ d_active, int n_parent, const float* __restrict__ gamma,
                      const float* __restrict__ ps_table, const int* __restrict__ d_gen, float ps_host,
-                     float* __restrict__ theta, int* __restrict__ idx, float* __restrict__ apd)
+                     float* __restrict__ zmin, float* __restrict__ theta, int* __restrict__ idx,
+                     float* __restrict__ apd)
 {
     const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ float s_dir[M][kDirStage];
     float x[M];
     float sqr = 0.f;
+    if constexpr (kTranslate) {
+        __shared__ float s_z[8][M];
+        float z[M];
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-        const float v = i < n ? t[(size_t)m * t_stride + i] : 0.f;
-        x[m] = v;
-        sqr = fmaf(v, v, sqr);
+        for (int m = 0; m < M; ++m) z[m] = CUDART_INF_F;
+#pragma unroll 2
+        for (int k = threadIdx.x; k < n; k += 256)
+#pragma unroll
+            for (int m = 0; m < M; ++m) z[m] = fminf(z[m], pop.obj(m, k));
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) z[m] = fminf(z[m], __shfl_xor_sync(0xFFFFFFFFu, z[m], o));
+            if (lane == 0) s_z[warp][m] = z[m];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            float r = s_z[0][m];
+            for (int w = 1; w < 8; ++w) r = fminf(r, s_z[w][m]);
+            if (blockIdx.x == 0 && threadIdx.x == 0) zmin[m] = r;
+            x[m] = i < n ? fmaxf(pop.obj(m, i) - r, 1e-32f) : 0.f;
+            sqr = fmaf(x[m], x[m], sqr);
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const float v = i < n ? t[(size_t)m * t_stride + i] : 0.f;
+            x[m] = v;
+            sqr = fmaf(v, v, sqr);
+        }
     }
     const float inv_norm = rsqrtf(sqr + 1e-12f);
     float best;
@@ -514,7 +546,7 @@ partition_apd_kernel(const float* __restrict__ t, int t_stride, int n, const flo
 
 __global__ void __launch_bounds__(kRveaBlockThreads, 1)
 rvea_elite_block(SplitPop pop, const int* __restrict__ idx, const float* __restrict__ apd, int K, int N,
-                 int* __restrict__ d_active, int* __restrict__ survivors)
+                 int* __restrict__ d_active, int* __restrict__ survivors, int* nan_slot, int* nan_fill, int* gen)
 {
     extern __shared__ unsigned long long s_key[];  // max(K, n): winners, then the W = 0 keys
     __shared__ unsigned char s_flag[kRveaBlockPoints];
@@ -606,7 +638,16 @@ rvea_elite_block(SplitPop pop, const int* __restrict__ idx, const float* __restr
     int pos = incl - c + (warp > 0 ? s_red[warp - 1] : 0);
     for (int i = b0; i < b1; ++i)
         if (s_flag[i]) survivors[pos++] = i;
-    if (tid == 0) *d_active = active;
+    if (tid == 0) {
+        *d_active = active;
+        // the update that follows fills the dead rows below *nan_fill, after
+        // which every row from the active count on holds the sentinels
+        if (nan_slot) {
+            *nan_fill = *nan_slot;
+            *nan_slot = active;
+        }
+        if (gen) *gen += 1;  // read by the partition, not after it
+    }
 }
 
 #define MOEA_DISPATCH_M(M, CALL)                                                      \
@@ -668,24 +709,36 @@ int run_rvea_apd(const float* t, int t_stride, int n, const float* theta, const 
     return MOEA_OK;
 }
 
-// Whether the three-launch selection applies, and its launches.  Writes the
-// same t / zmin / theta / idx / apd values, survivors and active count as the
-// staged translate, partition, APD and elitism.
+// Whether the short selection applies, and its two or three launches.  Computes
+// the same theta / idx / apd values, survivors and active count as the staged
+// translate, partition, APD and elitism.  nan_slot (may be null): the first row
+// of the next slot from which every row holds the sentinels, moved to *nan_fill
+// for run_rvea_update and replaced by the active count; gen (may be null): the
+// generation, incremented.
 bool rvea_block_eligible(int n, int M, int K)
 {
     return n >= 1 && n <= kRveaBlockPoints && K >= 1 && K <= kRveaBlockDirs && M >= 1 && M <= 16;
 }
 
 int run_rvea_select_block(const SplitPop& pop, const float* refs, int M, int K, const float* gamma, int* d_active,
-                          int N, const float* ps_table, const int* d_gen, float ps_host, float* t, int t_stride,
-                          float* zmin, float* theta, int* idx, float* apd, int* survivors, cudaStream_t s)
+                          int N, const float* ps_table, int* d_gen, float ps_host, float* t, int t_stride,
+                          float* zmin, float* theta, int* idx, float* apd, int* survivors, int* nan_slot, int* nan_fill,
+                          cudaStream_t s)
 {
     const int n = pop.n;
-    MOEA_DISPATCH_M(M, (rvea_translate_block<MM><<<1, kRveaBlockThreads, 0, s>>>(pop, t, t_stride, zmin)));
-    MOEA_DISPATCH_M(M, (partition_apd_kernel<MM><<<ceil_div(n, 8), 256, 0, s>>>(
-                           t, t_stride, n, refs, K, d_active, N, gamma, ps_table, d_gen, ps_host, theta, idx, apd)));
+    if (n * M <= kRveaTranslateMax) {
+        MOEA_DISPATCH_M(M, (partition_apd_kernel<MM, true><<<ceil_div(n, 8), 256, 0, s>>>(
+                               pop, t, t_stride, n, refs, K, d_active, N, gamma, ps_table, d_gen, ps_host, zmin, theta, idx,
+                               apd)));
+    } else {
+        MOEA_DISPATCH_M(M, (rvea_translate_block<MM><<<1, kRveaBlockThreads, 0, s>>>(pop, t, t_stride, zmin)));
+        MOEA_DISPATCH_M(M, (partition_apd_kernel<MM, false><<<ceil_div(n, 8), 256, 0, s>>>(
+                               pop, t, t_stride, n, refs, K, d_active, N, gamma, ps_table, d_gen, ps_host, zmin, theta, idx,
+                               apd)));
+    }
     const size_t smem = sizeof(unsigned long long) * (size_t)(K > n ? K : n);
-    rvea_elite_block<<<1, kRveaBlockThreads, smem, s>>>(pop, idx, apd, K, N, d_active, survivors);
+    rvea_elite_block<<<1, kRveaBlockThreads, smem, s>>>(pop, idx, apd, K, N, d_active, survivors, nan_slot, nan_fill,
+                                                        d_gen);
     MOEA_CUDA_TRY(cudaGetLastError());
     return MOEA_OK;
 }
@@ -727,12 +780,12 @@ int run_rvea_elitism(Workspace& ws, const int* idx, const SplitPop& pop, const f
 
 int run_rvea_update(const SplitPop& pop, const float* vars_a, const float* vars_b,
                     const int* survivors, const int* d_active, int N, int D, int M, float* vars,
-                    float* objs, float* cv, cudaStream_t s, int* nan_rows)
+                    float* objs, float* cv, cudaStream_t s, int* nan_rows, bool mark)
 {
     const long long items = (long long)N * ((D + kUpdateChunk - 1) / kUpdateChunk);
     const int blocks = (int)std::max(1ll, std::min(items, (long long)148 * 16));
     rvea_update<<<blocks, 256, 0, s>>>(pop, vars_a, vars_b, survivors, d_active, nan_rows, N, D, M, vars, objs, cv);
-    if (nan_rows) rvea_mark_nan_rows<<<1, 1, 0, s>>>(nan_rows, d_active);
+    if (nan_rows && mark) rvea_mark_nan_rows<<<1, 1, 0, s>>>(nan_rows, d_active);
     MOEA_CUDA_TRY(cudaGetLastError());
     return MOEA_OK;
 }
