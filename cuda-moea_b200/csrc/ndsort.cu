@@ -2039,6 +2039,134 @@ int launch_fused_rows(const BatchInst* d_inst, const FusedBucket& b, cudaStream_
     return MOEA_OK;
 }
 
+// ---------------------------------------------------------------------------
+// small populations: the whole sort in one CTA
+// ---------------------------------------------------------------------------
+//
+// Up to kSmallPoints points nothing has to be ordered: a thread per point tests
+// every other point against its own and keeps its dominators as bits in
+// registers, and a front costs one look at the unassigned words in shared
+// memory and two barriers.  Infeasible points take part in the same relation
+// (every feasible point, and those of smaller violation, dominate one).  The
+// eight launches of the general sort are bound by their latency at this size
+// (n = 184, M = 3: 39 us and the gaps between them, against 8: 72 -> 51 us a
+// generation).  The pair tests grow with n^2 (M + 1): at 2^20 of them (512 points
+// of three objectives, 341 of eight) the general sort draws level.
+constexpr int kSmallPoints = 512;
+constexpr long long kSmallWork = 1ll << 20;
+constexpr int kSmallWords = kSmallPoints / 32;
+
+template <int M>
+__global__ void __launch_bounds__(kSmallPoints)
+nds_small(SplitPop pop, int target, int* __restrict__ fronts, int* __restrict__ counters)
+{
+    constexpr int kM4 = (M + 3) & ~3;
+    __shared__ __align__(16) float s_f[kSmallPoints][kM4];
+    __shared__ float s_cv[kSmallPoints];
+    __shared__ unsigned s_feas[kSmallWords], s_inf[kSmallWords];  // class 0; class 2
+    __shared__ unsigned s_any[kSmallWords];                       // class 0 or 1
+    __shared__ unsigned s_u[kSmallWords];                         // unassigned
+    __shared__ int s_cnt[2];
+    const int n = pop.n, q = threadIdx.x, lane = q & 31, warp = q >> 5;
+    const int words = (n + 31) >> 5;
+    float f[kM4];
+#pragma unroll
+    for (int m = 0; m < kM4; ++m) f[m] = 0.0f;
+    float cv = 0.0f;
+    int cls = 4;
+    if (q < n) {
+        cv = pop.cvv(q);
+        bool nan = false;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            f[m] = pop.obj(m, q);
+            nan |= isnan(f[m]);
+        }
+        cls = cv == 0.0f ? (nan ? 1 : 0) : (isnan(cv) ? 3 : 2);
+    }
+#pragma unroll
+    for (int m = 0; m < kM4; ++m) s_f[q][m] = f[m];
+    s_cv[q] = cv;
+    const unsigned c0 = __ballot_sync(0xFFFFFFFFu, cls == 0), c2 = __ballot_sync(0xFFFFFFFFu, cls == 2);
+    const unsigned c01 = __ballot_sync(0xFFFFFFFFu, cls <= 1), all = __ballot_sync(0xFFFFFFFFu, cls <= 3);
+    if (lane == 0) {
+        s_feas[warp] = c0;
+        s_inf[warp] = c2;
+        s_any[warp] = c01;
+        s_u[warp] = all;
+    }
+    if (q < 2) s_cnt[q] = 0;
+    __syncthreads();
+    // dominators of q among the words of points
+    uint32_t row[kSmallWords];
+#pragma unroll
+    for (int w = 0; w < kSmallWords; ++w) {
+        row[w] = 0u;
+        if (w >= words) continue;
+        uint32_t bits = 0u;
+        if (cls == 0) {
+#pragma unroll 4
+            for (int k = 0; k < 32; ++k) {
+                bool le = true, lt = false;
+#pragma unroll
+                for (int v = 0; v < kM4; v += 4) {
+                    const float4 g = *reinterpret_cast<const float4*>(&s_f[32 * w + k][v]);
+                    const float p[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+                    for (int m = v; m < v + 4 && m < M; ++m) {
+                        le &= p[m - v] <= f[m];
+                        lt |= p[m - v] < f[m];
+                    }
+                }
+                bits |= (le && lt ? 1u : 0u) << k;
+            }
+            bits &= s_feas[w];
+        } else if (cls == 2) {
+            for (int k = 0; k < 32; ++k) bits |= (s_cv[32 * w + k] < cv ? 1u : 0u) << k;
+            bits = (bits & s_inf[w]) | s_any[w];
+        } else if (cls == 3) {
+            bits = s_any[w];
+        }
+        row[w] = bits;
+    }
+    int mine = -1, total = 0, k = 0;
+    bool alive = q < n;
+    for (;; ++k) {
+        uint32_t left = 0u;
+#pragma unroll
+        for (int w = 0; w < kSmallWords; ++w)
+            if (w < words) left |= row[w] & s_u[w];
+        const bool is_free = alive && left == 0u;
+        const unsigned fm = __ballot_sync(0xFFFFFFFFu, is_free);
+        if (lane == 0 && fm) atomicAdd(&s_cnt[k & 1], __popc(fm));
+        if (is_free) {
+            mine = k;
+            alive = false;
+        }
+        __syncthreads();  // everyone has read U; the front's size is complete
+        const int ck = s_cnt[k & 1];
+        if (lane == 0) s_u[warp] &= ~fm;
+        total += ck;
+        if (total >= target || ck == 0) {
+            if (q == 0) {
+                counters[2] = k;
+                counters[3] = total;
+                if (ck == 0 && total < target) atomicExch(counters + 6, kDevPeelInconsistent);
+            }
+            break;
+        }
+        if (q == 0) s_cnt[(k + 1) & 1] = 0;
+        __syncthreads();  // U without front k; the next counter is clear
+    }
+    if (q < n) fronts[q] = mine;
+}
+
+template <int M>
+void launch_small(const SplitPop& pop, int target, int* fronts, int* counters, cudaStream_t stream)
+{
+    nds_small<M><<<1, ((pop.n + 31) >> 5) * 32, 0, stream>>>(pop, target, fronts, counters);
+}
+
 // Self-test of the peel's two barrier waits with a short limit: every CTA
 // arrives, but the barrier asks for one arrival more than the grid has, so
 // the wait runs out and records kDevBarrierTimeout.  which 0: the counted
@@ -2089,6 +2217,20 @@ int run_ndsort(Workspace& ws, const SplitPop& pop, int M, int target, int* out_f
     int* fronts = out_fronts ? out_fronts : ws.fronts;
     const int T = 256, G = ceil_div(n, T);
 
+    if (n <= kSmallPoints && (long long)n * n * (M + 1) <= kSmallWork && !ws.peel_general && !ws.word_tiles) {
+        switch (M) {
+#define MOEA_SM_CASE(K) case K: launch_small<K>(pop, target, fronts, ws.counters, stream); break;
+        MOEA_SM_CASE(1) MOEA_SM_CASE(2) MOEA_SM_CASE(3) MOEA_SM_CASE(4)
+        MOEA_SM_CASE(5) MOEA_SM_CASE(6) MOEA_SM_CASE(7) MOEA_SM_CASE(8)
+        MOEA_SM_CASE(9) MOEA_SM_CASE(10) MOEA_SM_CASE(11) MOEA_SM_CASE(12)
+        MOEA_SM_CASE(13) MOEA_SM_CASE(14) MOEA_SM_CASE(15) MOEA_SM_CASE(16)
+#undef MOEA_SM_CASE
+        default: return set_error(MOEA_ERR_UNSUPPORTED, "ndsort: M=%d", M);
+        }
+        MOEA_CUDA_TRY(cudaGetLastError());
+        stage_mark("ndsort.peel", stream);
+        return MOEA_OK;
+    }
     nds_sort_tiles<<<ceil_div(n, kSortTile), kSortTile, 0, stream>>>(pop, M, ws.key0, ws.key64[0], ws.perm[0],
                                                                      ws.counters);
     int cur = 0;
