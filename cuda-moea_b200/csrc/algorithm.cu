@@ -603,7 +603,7 @@ struct moea_algorithm {
         ideal_ready = L.ideal_ready != 0;
         frontzero_count = 0;
         MOEA_TRY(forget_nan_rows());
-        drop_graphs();  // captured generations hold the seed of their epoch
+        if (graphable()) drop_graphs();  // captured generations hold the seed of their epoch
         return MOEA_OK;
     }
 
@@ -711,6 +711,12 @@ struct moea_algorithm {
     int generation_body()
     {
         MOEA_TRY(reproduce_evaluate());
+        return select_body();
+    }
+
+    // Environmental selection into the next slot.
+    int select_body()
+    {
         SplitPop pop{objs[P], objs[O], cv[P], cv[O], N, N, N, 2 * N};
         if (nsga3()) {
             SplitPop sort_pop = pop;
@@ -751,10 +757,10 @@ struct moea_algorithm {
         return MOEA_OK;
     }
 
-    bool graphable() const
-    {
-        return cfg.use_graphs && cfg.problem_kind != 0 && cfg.mating != MOEA_MATING_CALLBACK;
-    }
+    // A generation without callbacks is replayed whole; with a callback
+    // problem or mating (which runs on the host) its selection is, about fifteen
+    // launches that would otherwise be issued one by one between the callbacks.
+    bool graphable() const { return cfg.problem_kind != 0 && cfg.mating != MOEA_MATING_CALLBACK; }
 
     // Work before a generation's body: the constraint activation switch
     // refreshes parent violations and re-sorts them (problem_evaluator
@@ -801,12 +807,14 @@ struct moea_algorithm {
         MOEA_CUDA_TRY(cudaSetDevice(cfg.device));
         MOEA_TRY(pre_step());
         bool done = false;
-        if (graphable() && !graph_failed) {
+        const bool whole = graphable();
+        if (!whole) MOEA_TRY(reproduce_evaluate());
+        if (cfg.use_graphs && !graph_failed) {
             const int parity = (P == 0) ? 0 : 1;
             if (!graph[parity]) {
                 cudaGraph_t g = nullptr;
                 MOEA_CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-                const int st = generation_body();
+                const int st = whole ? generation_body() : select_body();
                 cudaError_t ce = cudaStreamEndCapture(stream, &g);
                 if (st == MOEA_OK && ce == cudaSuccess) {
                     size_t count = 0;
@@ -835,7 +843,7 @@ struct moea_algorithm {
                 done = true;
             }
         }
-        if (!done) MOEA_TRY(generation_body());
+        if (!done) MOEA_TRY(whole ? generation_body() : select_body());
         MOEA_TRY(post_step());
         return snapshot_now();
     }
@@ -873,7 +881,7 @@ struct moea_algorithm {
     {
         if (!initialized) return MOEA_OK;
         MOEA_CUDA_TRY(cudaStreamSynchronize(stream));
-        drop_graphs();  // the draws of the new epoch use a different seed
+        if (graphable()) drop_graphs();  // they hold the seed of the epoch's draws; the selection alone has none
         ++epoch;
         if (H > 0) {
             MOEA_CUDA_TRY(cudaMemcpyAsync(refs, refs0, sizeof(float) * (size_t)M * H, cudaMemcpyDeviceToDevice,
@@ -1028,8 +1036,8 @@ moea_status moea_algorithm_view(moea_algorithm* a, moea_population_view* v)
     v->finished = a->initialized && a->generation >= a->T;
     v->device = a->cfg.device;
     v->total_ms = a->total_ms;
-    v->kernels_per_generation = a->graph_kernels;
-    v->graph_active = (a->graph[0] || a->graph[1]) ? 1 : 0;
+    v->kernels_per_generation = a->graphable() ? a->graph_kernels : 0;
+    v->graph_active = a->graphable() && (a->graph[0] || a->graph[1]) ? 1 : 0;
     v->last_max_front = -1;
     if (!a->initialized) return MOEA_OK;
     // the caller may write the rows it is given
