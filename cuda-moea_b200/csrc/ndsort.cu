@@ -1869,33 +1869,88 @@ fused_tiles_one(const BatchInst* __restrict__ insts, const int* __restrict__ ids
 }
 
 constexpr int kFusedPeelThreads = 1024;
+constexpr int kWalkHops = 64;  // waiting points followed from one member before the pass over all points
 
-// Peel of one instance per CTA with the blockers, the front list and a queue
-// of woken points in shared memory.  Once front k is known and removed from
-// the unassigned set U, one parallel pass over the blockers queues the
-// points whose blocker was in front k; each queued point (one lane each)
-// probes its row from the former blocker's word downwards (bits above it stay
-// free of unassigned dominators) and either records the next unassigned
-// dominator found as its blocker or, having none, joins front k + 1.  A front
-// costs three block barriers and one or two memory latencies.  Shared memory:
-// U (W words), blocker, list and queue (n ints each).
+// Highest unassigned dominator of a row in its words 0 .. sw (-1: none), found
+// by G lanes of a warp (l their rank, the same result in each): 256 words a
+// step, in chunks of four from the top, those without unassigned points not
+// read at all.  Every lane of the warp calls it, a group without a row with
+// sw = -1.
+template <int G>
+__device__ __forceinline__ int scan_row_group(const uint32_t* __restrict__ row, const uint32_t* U, int sw, int l)
+{
+    constexpr int kLoads = 64 / G;  // 16-byte chunks a lane has in flight
+    const uint4* row4 = reinterpret_cast<const uint4*>(row);
+    const uint4* U4 = reinterpret_cast<const uint4*>(U);
+    int found = -1;
+    int top = sw >= 0 ? sw >> 2 : -1;  // highest chunk not yet read
+    while (__any_sync(0xFFFFFFFFu, top >= 0)) {
+        uint4 v[kLoads];
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) {
+            const int c = top - l - G * i;
+            v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (c < 0) continue;
+            uint4 u = U4[c];
+            if (4 * c + 3 > sw) {  // words above the start are probed, or not of this row
+                u.w = 0u;
+                if (4 * c + 2 > sw) u.z = 0u;
+                if (4 * c + 1 > sw) u.y = 0u;
+            }
+            if (u.x | u.y | u.z | u.w) {
+                const uint4 r = __ldg(row4 + c);
+                v[i] = make_uint4(r.x & u.x, r.y & u.y, r.z & u.z, r.w & u.w);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) {
+            if (found >= 0 || !(v[i].x | v[i].y | v[i].z | v[i].w)) continue;
+            const int w = v[i].w ? 3 : v[i].z ? 2 : v[i].y ? 1 : 0;
+            const uint32_t bb = v[i].w ? v[i].w : v[i].z ? v[i].z : v[i].y ? v[i].y : v[i].x;
+            found = (4 * (top - l - G * i) + w) * 32 + (31 - __clz(bb));
+        }
+#pragma unroll
+        for (int o = G / 2; o; o >>= 1) found = max(found, __shfl_xor_sync(0xFFFFFFFFu, found, o));
+        top = found >= 0 ? -1 : top - 64;
+    }
+    return found;
+}
+
+// Peel of one instance per CTA in shared memory.  Every unassigned point waits
+// for one unassigned dominator, its blocker, and the points that wait for the
+// same one form a list (head, next).  A member of front k leaves the
+// unassigned set U and queues its list; each queued point is searched from the
+// former blocker's word downwards (bits above it stay free of unassigned
+// dominators) and either waits for the next unassigned dominator found or,
+// having none, joins front k + 1.  Thin fronts bound the peel (DTLZ4, M=3: 460
+// fronts of ten points), each a chain of two block barriers, the lists and one
+// row read: 1.33 ms with a pass over all blockers per front, a probe of two
+// words and then a scan by a warp, 1.08 ms now.  Shared memory: U (W words), blocker, head,
+// next, list and queue (n ints each).
 __global__ void __launch_bounds__(kFusedPeelThreads, 1)
 fused_peel(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
 {
     extern __shared__ __align__(16) uint32_t fp_smem[];
-    __shared__ int s_cnt, s_qn;
+    __shared__ int s_cnt, s_qn[2], s_long[2];
     const BatchInst& I = insts[ids[blockIdx.x]];
     const int n = I.n, W = I.W, target = I.N;
     uint32_t* U = fp_smem;
     int* blk = reinterpret_cast<int*>(fp_smem + W);
     int* list = blk + n;
     int* queue = list + n;
+    int* head = queue + n;
+    int* next = head + n;
     const uint32_t* rows = I.rows;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
 
     for (int w = t; w < W; w += blockDim.x) {
         const int lo = w * 32;
         U[w] = (lo + 32 <= n) ? 0xFFFFFFFFu : (lo >= n ? 0u : ((1u << (n - lo)) - 1u));
+    }
+    for (int q = t; q < n; q += blockDim.x) head[q] = -1;
+    if (t < 2) {
+        s_qn[t] = 0;
+        s_long[t] = 0;
     }
     if (t == 0) s_cnt = 0;
     __syncthreads();
@@ -1905,6 +1960,8 @@ fused_peel(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
         if (b < 0) {
             list[atomicAdd(&s_cnt, 1)] = q;
             I.front_sorted[q] = 0;
+        } else {
+            next[q] = atomicExch(head + b, q);
         }
     }
     __syncthreads();
@@ -1923,28 +1980,62 @@ fused_peel(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
             for (int q = t; q < n; q += blockDim.x) I.fronts[I.perm[q]] = I.front_sorted[q];
             return;
         }
-        if (t == 0) s_qn = 0;
+        const int par = k & 1;
         for (int i = t; i < ck; i += blockDim.x) {
             const int p = list[len_prev + i];
             atomicAnd(U + (p >> 5), ~(1u << (p & 31)));
+            int hops = 0;
+            for (int q = head[p]; q >= 0; q = next[q]) {
+                if (++hops > kWalkHops) {
+                    s_long[par] = 1;
+                    break;
+                }
+                queue[atomicAdd(&s_qn[par], 1)] = q;
+            }
         }
         __syncthreads();
-        // points still unassigned whose blocker has just been assigned
-        for (int q = t; q < n; q += blockDim.x) {
-            const int b = blk[q];
-            if (b >= 0 && ((U[q >> 5] >> (q & 31)) & 1u) && !((U[b >> 5] >> (b & 31)) & 1u))
-                queue[atomicAdd(&s_qn, 1)] = q;
+        if (s_long[par]) {
+            // a list longer than one thread should follow: a pass over all
+            // blockers instead (a member of a front has none)
+            __syncthreads();
+            if (t == 0) s_qn[par] = 0;
+            __syncthreads();
+            for (int q = t; q < n; q += blockDim.x) {
+                const int b = blk[q];
+                if (b >= 0 && !((U[b >> 5] >> (b & 31)) & 1u)) queue[atomicAdd(&s_qn[par], 1)] = q;
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        const int qn = s_qn;
-        // entries interleaved over the warps: a short queue uses every warp
+        const int qn = s_qn[par];
+        if (t == 0) {  // of the next front: last read before two barriers
+            s_qn[par ^ 1] = 0;
+            s_long[par ^ 1] = 0;
+        }
+        // Entries interleaved over the warps.  Up to one row per warp it is
+        // read by all lanes, up to four by eight lanes each; a longer queue
+        // probes two words per lane first, which resolves most rows.
+        const int width = qn <= nwarps ? 32 : qn <= 4 * nwarps ? 8 : 1;
+        const int sub = lane / width;
         for (int r = 0; r * 32 * nwarps < qn; ++r) {
-            const int e = warp + nwarps * (r * 32 + lane);
+            const int e = warp + nwarps * (width > 1 ? sub : r * 32 + lane);
             const bool act = e < qn;
             const int q = act ? queue[e] : 0;
             bool is_free = false, need = false;
             int start_w = -1;
-            if (act) {
+            if (width > 1) {
+                const int sw = act ? blk[q] >> 5 : -1;
+                const uint32_t* row = rows + (size_t)q * W;
+                const int found = width == 32 ? scan_row_group<32>(row, U, sw, lane)
+                                              : scan_row_group<8>(row, U, sw, lane & 7);
+                if (act && (lane & (width - 1)) == 0) {
+                    if (found >= 0) {
+                        blk[q] = found;
+                        next[q] = atomicExch(head + found, q);
+                    } else {
+                        is_free = true;
+                    }
+                }
+            } else if (act) {
                 const uint32_t* row = rows + (size_t)q * W;
                 int w = blk[q] >> 5;
                 const uint32_t hiw = __ldg(row + w);
@@ -1955,7 +2046,9 @@ fused_peel(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
                     bits = low & U[w];
                 }
                 if (bits) {
-                    blk[q] = w * 32 + (31 - __clz(bits));
+                    const int f = w * 32 + (31 - __clz(bits));
+                    blk[q] = f;
+                    next[q] = atomicExch(head + f, q);
                 } else if (w == 0) {
                     is_free = true;
                 } else {
@@ -1963,38 +2056,34 @@ fused_peel(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
                     start_w = w - 1;
                 }
             }
-            // rows not resolved by the probe: the whole warp scans each of
-            // them downwards over the words that still hold unassigned points
+            // rows not resolved by the probe: eight lanes scan each of them
+            // downwards over the words that still hold unassigned points,
+            // four rows of the warp side by side
+            const int grp = lane >> 3;
             unsigned needm = __ballot_sync(0xFFFFFFFFu, need);
             while (needm) {
-                const int L = __ffs(needm) - 1;
-                needm &= needm - 1;
-                const int qL = __shfl_sync(0xFFFFFFFFu, q, L);
-                const uint32_t* row = rows + (size_t)qL * W;
-                const int sw = __shfl_sync(0xFFFFFFFFu, start_w, L);
-                int found = -1;
-                for (int w0 = sw; w0 >= 0 && found < 0; w0 -= 256) {
-                    uint32_t acc[8];
+                unsigned m = needm;  // its sub-th set bit is this group's row
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int w = w0 - lane - 32 * i;
-                        const uint32_t u = (w >= 0) ? U[w] : 0u;
-                        acc[i] = u ? (__ldg(row + w) & u) : 0u;
-                    }
+                for (int j = 0; j < 3; ++j)
+                    if (j < grp) m &= m - 1;
+                const int L = m ? __ffs(m) - 1 : -1;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const unsigned nz = __ballot_sync(0xFFFFFFFFu, acc[i] != 0u);
-                        if (nz) {
-                            const int src = __ffs(nz) - 1;
-                            const uint32_t bb = __shfl_sync(0xFFFFFFFFu, acc[i], src);
-                            found = (w0 - src - 32 * i) * 32 + (31 - __clz(bb));
-                            break;
+                for (int j = 0; j < 4; ++j) needm &= needm - 1;
+                const int qL = __shfl_sync(0xFFFFFFFFu, q, max(L, 0));
+                const int sw = __shfl_sync(0xFFFFFFFFu, start_w, max(L, 0));
+                const int found = scan_row_group<8>(rows + (size_t)qL * W, U, L >= 0 ? sw : -1, lane & 7);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int Lj = __shfl_sync(0xFFFFFFFFu, L, 8 * j);
+                    const int fj = __shfl_sync(0xFFFFFFFFu, found, 8 * j);
+                    if (lane == Lj) {
+                        if (fj >= 0) {
+                            blk[q] = fj;
+                            next[q] = atomicExch(head + fj, q);
+                        } else {
+                            is_free = true;
                         }
                     }
-                }
-                if (lane == L) {
-                    if (found >= 0) blk[q] = found;
-                    else is_free = true;
                 }
             }
             const unsigned fm = __ballot_sync(0xFFFFFFFFu, is_free);
@@ -2409,8 +2498,9 @@ int fused_tile_blocks(int M, int n, int shape)
 }
 
 // U takes the workspace's row words W (4 * ceil(n / 128) for a workspace of n
-// merged points), then blockers, front list and queue of n entries each.
-size_t fused_peel_smem(int W, int n) { return (size_t)W * sizeof(uint32_t) + 3 * (size_t)n * sizeof(int); }
+// merged points), then blockers, front list, queue, heads and
+// links of n entries each.
+size_t fused_peel_smem(int W, int n) { return (size_t)W * sizeof(uint32_t) + 5 * (size_t)n * sizeof(int); }
 
 int fused_ndsort_configure()
 {

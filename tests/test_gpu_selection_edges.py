@@ -65,3 +65,23 @@ def test_rvea_generations_equal_the_stage_calls(oracle, N, M):
         cv = torch.full_like(cv, nan)
         x[:act], f[:, :act], cv[:act] = mx[s], mf[:, s], mcv[s]
         active = act
+
+
+@pytest.mark.parametrize("kind,M", [("DTLZ4", 3), ("DTLZ1", 2), ("DTLZ7", 8)])
+def test_batch_peel_of_thin_and_wide_fronts(kind, M):
+    """Hundreds of thin fronts (short queues, a warp or eight lanes per row)
+    and few wide ones (long queues, lists longer than one thread follows),
+    against the same instances alone."""
+    def make(N):
+        return cm.NSGA3(population_size=N, max_generations=6, problem=getattr(cm, kind)(M + 19, M), seed=N,
+                        print_progress=False)
+
+    sizes = [46, 92, 130, 510, 512, 514, 2050, 4096]
+    batch = cm.Batch([make(N) for N in sizes])
+    assert batch.fused
+    batch.run()
+    for i, N in enumerate(sizes):
+        want, got = make(N).run(), batch.result(i)
+        assert torch.equal(got.variables, want.variables)
+        assert torch.equal(got.objectives, want.objectives)
+        assert torch.equal(got.auxiliary_indices, want.auxiliary_indices)
