@@ -588,7 +588,7 @@ def measure_workload(name, steps, warmup, seed, torch, cm):
         bytes_ = 8.0 * w["N"] * D
         hbm, kind_ = _peaks()
         ms = total_ms / steps
-        out["roofline"] = {"kernel": "whole generation (crossover_philox, mutation_philox, dtlz_block_rows, "
+        out["roofline"] = {"kernel": "whole generation (crossover_rows, mutation_philox, dtlz_block_rows, "
                                      "RVEA selection, rvea_update)", "bound": "hbm",
                            "achieved": bytes_ / (ms / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
                            "frac": bytes_ / (ms / 1e3) / 1e9 / hbm, "peak_source": kind_,

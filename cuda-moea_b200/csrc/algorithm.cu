@@ -1173,7 +1173,7 @@ BatchInst fused_describe(moea_algorithm* a, int P, int X)
     b.perm_a = w.perm[0]; b.perm_b = w.perm[1]; b.perm = b.n > kFusedSortTile ? w.perm[0] : w.perm[1];
     b.long_runs = w.run_start; b.block_tables = w.block_tables;
     b.sorted_f = w.sorted_f; b.qinfo = w.qinfo; b.blocker = w.blocker; b.front_sorted = w.front_sorted;
-    b.front_list = w.front_list; b.counters = w.counters; b.rows = w.rows;
+    b.counters = w.counters; b.rows = w.rows;
     b.fronts = w.fronts; b.nds_gidx = w.nds_gidx; b.sizes = w.sizes;
     b.nds_objs = w.nds_objs; b.rcp_b = w.rcp_b; b.extreme = w.extreme; b.assoc_idx = w.assoc_idx;
     b.assoc_dist = w.assoc_dist; b.rho = w.rho; b.niche_last = w.niche_last; b.niche_start = w.niche_start;

@@ -71,9 +71,9 @@ int dalloc(Workspace& ws, T** p, size_t count)
 
 void free_all(Workspace& ws)
 {
-    void* ptrs[] = {ws.rows, ws.key32[0], ws.key32[1], ws.key64[0], ws.key64[1], ws.key0,
+    void* ptrs[] = {ws.rows, ws.key64[0], ws.key64[1], ws.key0,
                     ws.perm[0], ws.perm[1], ws.sorted_f, ws.qinfo, ws.head, ws.run_start,
-                    ws.blocker, ws.front_sorted, ws.front_list, ws.counters, ws.fronts,
+                    ws.blocker, ws.front_sorted, ws.counters, ws.fronts,
                     ws.nds_gidx, ws.sizes, ws.chunk_counts, ws.nds_objs, ws.norm_part,
                     ws.norm_part_idx, ws.rcp_b, ws.extreme, ws.ideal_tmp, ws.assoc_best,
                     ws.assoc_idx, ws.assoc_dist, ws.rho, ws.sel_vals[0], ws.sel_vals[1],
@@ -108,12 +108,11 @@ int workspace_init(Workspace& ws, int device, int n_max, int m_max, int h_max)
     int st = MOEA_OK;
 #define A(p, c) if (st == MOEA_OK) st = dalloc(ws, &(p), (c))
     A(ws.rows, n * (size_t)ws.words);
-    A(ws.key32[0], n); A(ws.key32[1], n);
     A(ws.key64[0], n); A(ws.key64[1], n); A(ws.key0, n);
     A(ws.perm[0], n); A(ws.perm[1], n);
     A(ws.sorted_f, n * (size_t)(m_max > 1 ? m_max - 1 : 1));
     A(ws.qinfo, n); A(ws.head, n); A(ws.run_start, n);
-    A(ws.blocker, n); A(ws.front_sorted, n); A(ws.front_list, n);
+    A(ws.blocker, n); A(ws.front_sorted, n);
     A(ws.chunk_keys, (size_t)(m_max > 1 ? m_max - 1 : 1) * ws.words * 32);
     A(ws.chunk_bits, (size_t)(m_max > 1 ? m_max - 1 : 1) * ws.words * 33);
     if (m_max > 1) A(ws.block_tables, block_table_words(n_max, m_max));

@@ -60,7 +60,6 @@ struct Workspace {
 
     // --- non-dominated sort ---
     uint32_t* rows = nullptr;       // [n_max][words] dominator bits per sorted point
-    uint32_t* key32[2] = {};        // LSD pass keys
     uint64_t* key64[2] = {};        // final pass keys / niching keys (ping-pong)
     uint64_t* key0 = nullptr;       // per point: class << 32 | order key of f0 or cv
     int* perm[2] = {};              // sorted position -> point index
@@ -74,7 +73,6 @@ struct Workspace {
                                        // tree of the keys and prefix sets (nds_block_rows)
     int* blocker = nullptr;         // per sorted position: last known unassigned dominator
     int* front_sorted = nullptr;    // per sorted position: front index or -1
-    int* front_list = nullptr;      // members of each peeled front, front by front
     int* counters = nullptr;        // [0] feasible count, [1] list length (batched peel),
                                     // [2] max_front, [3] assigned, [4] grid-barrier arrivals,
                                     // [6] device status, [10] class-2 count, [11] class-3 count,
@@ -261,8 +259,9 @@ size_t cub_temp_bytes_needed(int n_max);
 // One NSGA-III instance of a fused batch: sizes, parameters and every buffer a
 // generation touches, for one parity of the slot rotation (P parents, O
 // offspring, X next).  The fused generation runs each stage once for all
-// instances: one CTA per instance where the stage needs a block-wide sort,
-// scan or barrier (n = 2N <= kFusedMaxPoints), flattened work items elsewhere.
+// instances: one CTA or a small cluster per instance where the stage needs a
+// scan or a barrier over the instance (peel, extraction and intercepts, niche
+// buckets; n = 2N <= kFusedMaxPoints), flattened work items elsewhere.
 constexpr int kFusedMaxPoints = 8192;
 constexpr int kDirTreeMaxDepth = 8;   // stack depth of the tree association kernels
 constexpr int kFusedThreads = 1024;
@@ -284,7 +283,7 @@ struct BatchInst {
     int* long_runs;             // runs of equal keys longer than a thread ranks
     int* vals;
     uint32_t* block_tables;
-    int* blocker; int* front_sorted; int* front_list; int* counters;
+    int* blocker; int* front_sorted; int* counters;
     uint32_t* rows;
     int* fronts; int* nds_gidx; int* sizes; float* nds_objs; float* rcp_b; int* extreme;
     int* assoc_idx; float* assoc_dist; int* selected; int* flags; int* survivors;

@@ -6,7 +6,8 @@
 // front), different mechanism:
 //
 //  1. Sort of the points by (class, f0 | cv, S), a 56-bit key, in sorted tiles
-//     and rank merges (nds_sort_tiles, nds_sort_merge), S the top 22 bits of the order key of the FP32 sum f1 + ... + f_{M-1}.
+//     and rank merges (nds_sort_tiles, nds_sort_merge), S the top 22 bits of the
+//     order key of the FP32 sum f1 + ... + f_{M-1}.
 //     Class 0 = feasible, 1 = feasible with a NaN objective, 2 = infeasible,
 //     3 = infeasible with NaN violation.  FP32 addition rounds monotonically,
 //     so a feasible dominator p of q has f0(p) <= f0(q) and S(p) <= S(q); runs
@@ -23,12 +24,13 @@
 //       feasible q:    p dominates q  <=>  p < dup[q] and f_m(p) <= f_m(q), m >= 1
 //     which is the reference relation (non_dominated_sort.cu:190-239) with one
 //     integer and M-1 float comparisons per pair on the lower triangle only.
-//  3. For every word of 32 sorted positions and every objective m >= 1 the
-//     positions are sorted by f_m once, with the prefix sets of that order.
-//     A tile kernel then evaluates the test for one dominatee per lane: the
-//     dominators of a word with f_m(p) <= f_m(q) are one prefix set, found
-//     by a binary search, and the row word is the AND of those sets with the
-//     dup mask.  It stores for every q the bit row of its dominators.
+//  3. For every block of sorted positions (256 or 128; words of 32 in the
+//     alternative) and every objective m >= 1 the positions are sorted by f_m
+//     once, with the prefix sets of that order.  A row kernel then evaluates
+//     the test for one dominatee per lane: the dominators of a block with
+//     f_m(p) <= f_m(q) are one prefix set, found by a tree descent, and the
+//     row words are the AND of those sets with the dup mask.  It stores for
+//     every q the bit row of its dominators.
 //  4. One cooperative persistent kernel peels the fronts: q joins front k when
 //     no still-unassigned point is left in its row.  Each point remembers one
 //     unassigned dominator ("blocker"); while that blocker is unassigned the
@@ -36,6 +38,9 @@
 //     once over the whole sort.  Fronts are separated by a bounded grid barrier
 //     and the loop stops once `target` points are assigned, like the
 //     reference's front propagation loops (:792-843, :1070-1279).
+//
+// Populations whose pair tests one CTA does in a few microseconds skip the
+// order (nds_small): each thread keeps its point's dominators in registers.
 #include <algorithm>
 
 #include <cooperative_groups.h>
@@ -1976,7 +1981,6 @@ fused_peel(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
                 I.counters[3] = total;
                 if (ck == 0 && total < target) atomicExch(I.counters + 6, kDevPeelInconsistent);
             }
-            for (int i = t; i < len; i += blockDim.x) I.front_list[i] = list[i];
             for (int q = t; q < n; q += blockDim.x) I.fronts[I.perm[q]] = I.front_sorted[q];
             return;
         }

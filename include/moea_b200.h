@@ -585,8 +585,9 @@ typedef struct moea_batch moea_batch;
  * on the schedule or the tile shape. */
 #define MOEA_BATCH_AUTOTUNE 2
 /* Fused mode: half-width dominance tiles for every objective count (twice the
- * tile CTAs, each staging half the word tables).  Without it, and without
- * MOEA_BATCH_AUTOTUNE, every objective count uses the full-width tiles. */
+ * row CTAs, each covering up to 512 dominator positions instead of 1024).
+ * Without it, and without MOEA_BATCH_AUTOTUNE, every objective count uses the
+ * full-width tiles. */
 #define MOEA_BATCH_HALF_TILES 4
 #define MOEA_BATCH_GROUPS(g) (((g) & 0xFF) << 8)
 moea_status moea_batch_create(const moea_algorithm_config* cfgs, int count, void* stream, int flags,
