@@ -809,7 +809,15 @@ struct moea_algorithm {
         bool done = false;
         const bool whole = graphable();
         if (!whole) MOEA_TRY(reproduce_evaluate());
-        if (cfg.use_graphs && !graph_failed) {
+        bool replay = cfg.use_graphs && !graph_failed;
+        if (replay && !whole) {
+            // a caller that captures the step itself (its problem's kernels
+            // with the selection) gets the launches, as without graphs
+            cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+            MOEA_CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
+            replay = capturing == cudaStreamCaptureStatusNone;
+        }
+        if (replay) {
             const int parity = (P == 0) ? 0 : 1;
             if (!graph[parity]) {
                 cudaGraph_t g = nullptr;

@@ -85,3 +85,50 @@ def test_batch_peel_of_thin_and_wide_fronts(kind, M):
         assert torch.equal(got.variables, want.variables)
         assert torch.equal(got.objectives, want.objectives)
         assert torch.equal(got.auxiliary_indices, want.auxiliary_indices)
+
+
+class _Spheres(cm.PythonProblem):
+    def __init__(self):
+        super().__init__(6, 2)
+
+    def evaluate(self, x, context):
+        return torch.stack((x.square().sum(1), (x - 1).square().sum(1)), 1)
+
+
+def _callback_run(cls, graphs, seed=3):
+    with torch.cuda.stream(torch.cuda.Stream()):
+        algo = cls(population_size=64, max_generations=5, problem=_Spheres(), seed=seed, print_progress=False,
+                   use_graphs=graphs)
+        algo.initialize()
+    torch.cuda.synchronize()
+    return algo
+
+
+@pytest.mark.parametrize("cls", [cm.NSGA3, cm.RVEA])
+def test_callback_selection_graph_over_resets(cls):
+    """The selection's graphs outlive a reset after an odd number of
+    generations: every run equals the one of direct launches."""
+    a, b = _callback_run(cls, True), _callback_run(cls, False)
+    for _ in range(3):
+        x, y = a.run(), b.run()
+        assert torch.equal(x.variables.view(torch.int32), y.variables.view(torch.int32))
+        assert torch.equal(x.objectives.contiguous().view(torch.int32), y.objectives.contiguous().view(torch.int32))
+        a.reset()
+        b.reset()
+
+
+@pytest.mark.parametrize("cls", [cm.NSGA3, cm.RVEA])
+def test_callback_generations_inside_the_callers_capture(cls):
+    """A caller that captures the generations of a callback problem in a graph
+    of its own gets the same populations."""
+    a, b = _callback_run(cls, True), _callback_run(cls, True)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=a.stream):
+        a.step()
+        a.step()
+    graph.replay()
+    torch.cuda.synchronize()
+    for _ in range(2):
+        b.step()
+    x, y = a.result(), b.result()
+    assert torch.equal(x.variables.view(torch.int32), y.variables.view(torch.int32))
