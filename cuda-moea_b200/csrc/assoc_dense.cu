@@ -183,7 +183,7 @@ __device__ __forceinline__ void dense_block(DenseShared<M, PTS>& sm, int p0, con
                         const float res = fmaf(-dot, r[m], xq[m]);
                         d2 = fmaf(res, res, d2);
                     }
-                    if (d2 < best || (d2 == best && (unsigned)j < (unsigned)bj)) {
+                    if (d2 < best || (d2 == best && j < bj)) {  // an infinite distance is never taken
                         best = d2;
                         bj = j;
                     }

@@ -132,3 +132,19 @@ def test_callback_generations_inside_the_callers_capture(cls):
         b.step()
     x, y = a.result(), b.result()
     assert torch.equal(x.variables.view(torch.int32), y.variables.view(torch.int32))
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 10])
+@pytest.mark.parametrize("n", [2, 600, 9500])
+def test_dense_search_of_points_whose_distances_overflow(oracle, M, n):
+    """A point all of whose distances are infinite has no direction (-1)."""
+    rng = np.random.default_rng(n + M)
+    x = (rng.random((M, n)) * 3e38).astype(np.float32)
+    x[:, rng.random(n) < 0.2] = -0.0
+    d = rng.random((M, 37)) + 0.01
+    d = (d / np.linalg.norm(d, axis=0)).astype(np.float32)
+    want_i, want_d = oracle.associate(x, d)
+    got_i, got_d = st.associate(st.Workspace(n, M, 37), torch.from_numpy(x).cuda(), torch.from_numpy(d).cuda(),
+                                st.ASSOC_SCAN)
+    np.testing.assert_array_equal(got_i.cpu().numpy(), want_i)
+    np.testing.assert_array_equal(got_d.cpu().numpy(), want_d)
