@@ -806,7 +806,7 @@ dir_delta_kernel(const float* __restrict__ refs, int M, int H, float* __restrict
 {
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ double s_warp[kDeltaThreads / 32];
-    __shared__ double s_max[kDeltaCtas];
+    __shared__ double s_max;  // this CTA's maximum (read by CTA 0)
     const int c = (int)cluster.block_rank(), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double d = 0.0;
     for (int j = c * kDeltaThreads + threadIdx.x; j < H; j += kDeltaCtas * kDeltaThreads) {
@@ -825,13 +825,14 @@ dir_delta_kernel(const float* __restrict__ refs, int M, int H, float* __restrict
     if (warp == 0) {
         d = lane < kDeltaThreads / 32 ? s_warp[lane] : 0.0;
         for (int o = 16; o; o >>= 1) d = fmax(d, __shfl_xor_sync(0xffffffffu, d, o));
-        if (lane == 0) cluster.map_shared_rank(s_max, 0)[c] = d;
+        if (lane == 0) s_max = d;
     }
-    cluster.sync();  // CTA 0 holds every CTA's maximum
+    cluster.sync();  // every CTA has started and published its maximum
     if (c == 0 && threadIdx.x == 0) {
-        for (int r = 0; r < kDeltaCtas; ++r) d = fmax(d, s_max[r]);
+        for (int r = 1; r < kDeltaCtas; ++r) d = fmax(d, *cluster.map_shared_rank(&s_max, r));
         out[0] = __double2float_ru(fmin(d, 1e30));
     }
+    cluster.sync();  // CTA 0 has read every CTA's maximum
 }
 
 __global__ void assoc_reset(unsigned long long* best, int n_cap)
