@@ -253,35 +253,58 @@ constexpr int kTieSmemSort = 4096;    // longer runs: bitonic in shared memory u
 
 // Runs of equal keys in class 0 into lexicographic order: every member of a run
 // of at most kTieShort counts the members before it; longer runs are copied
-// and listed for nds_tie_fix_long.
-__device__ __forceinline__ void tie_rank(int pos, const SplitPop& pop, int M, const uint64_t* __restrict__ skey,
-                                         const int* __restrict__ perm_in, int* __restrict__ perm_out,
-                                         int* __restrict__ long_runs, int* __restrict__ n_long)
+// and listed for nds_tie_fix_long.  Every lane of the warp calls, with active
+// false past the last point.  The lanes of a run step through it together, and
+// no lane leaves a comparison early: lanes that each followed their own loops
+// ran one after another (5000 points of 243 vectors of five objectives: 258 us,
+// 20 now; points without ties 3-4 us either way).
+__device__ __forceinline__ void tie_rank(int pos, bool active, const SplitPop& pop, int M,
+                                         const uint64_t* __restrict__ skey, const int* __restrict__ perm_in,
+                                         int* __restrict__ perm_out, int* __restrict__ long_runs,
+                                         int* __restrict__ n_long)
 {
     const int n = pop.n;
-    const uint64_t k = skey[pos];
-    const int pt = perm_in[pos];
-    int to = pos;
-    if ((k >> kSortClassShift) == 0u) {
-        int a = pos, b = pos + 1;  // the run, as far as kTieShort reaches
-        while (a > 0 && pos - a <= kTieShort && skey[a - 1] == k) --a;
-        while (b < n && b - a <= kTieShort && skey[b] == k) ++b;
-        if (b - a > kTieShort) {
-            if (a == pos) long_runs[atomicAdd(n_long, 1)] = pos;
-        } else if (b - a > 1) {
-            to = a;
-            for (int x = a; x < b; ++x)
-                if (x != pos && tie_less(pop, M, perm_in[x], pt)) ++to;
-        }
+    const uint64_t k = active ? skey[pos] : 0ull;
+    const int pt = active ? perm_in[pos] : 0;
+    const bool ranked = active && (k >> kSortClassShift) == 0u;
+    int a = pos, b = pos + 1;  // the run, as far as kTieShort reaches
+    bool more = ranked;
+    while (__any_sync(0xFFFFFFFFu, more)) {
+        more = more && a > 0 && pos - a <= kTieShort && skey[a - 1] == k;
+        if (more) --a;
     }
-    perm_out[to] = pt;
+    more = ranked;
+    while (__any_sync(0xFFFFFFFFu, more)) {
+        more = more && b < n && b - a <= kTieShort && skey[b] == k;
+        if (more) ++b;
+    }
+    int to = pos, members = 0;
+    if (ranked && b - a > kTieShort) {
+        if (a == pos) long_runs[atomicAdd(n_long, 1)] = pos;
+    } else if (ranked && b - a > 1) {
+        to = a;
+        members = b - a;
+    }
+    const int steps = __reduce_max_sync(0xFFFFFFFFu, members);
+    for (int i = 0; i < steps; ++i) {
+        const int other = i < members ? perm_in[a + i] : pt;
+        bool less = false, equal = true;
+#pragma unroll 4
+        for (int m = 1; m < M; ++m) {
+            const uint32_t ka = float_order_key(pop.obj(m, other)), kb = float_order_key(pop.obj(m, pt));
+            less |= equal && ka < kb;
+            equal &= ka == kb;
+        }
+        to += (less || (equal && other < pt)) ? 1 : 0;
+    }
+    if (active) perm_out[to] = pt;
 }
 
 __global__ void nds_tie_rank(SplitPop pop, int M, const uint64_t* __restrict__ skey, const int* __restrict__ perm_in,
                              int* __restrict__ perm_out, int* __restrict__ long_runs, int* __restrict__ n_long)
 {
     const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos < pop.n) tie_rank(pos, pop, M, skey, perm_in, perm_out, long_runs, n_long);
+    tie_rank(pos, pos < pop.n, pop, M, skey, perm_in, perm_out, long_runs, n_long);
 }
 
 // Ascending bitonic network over a[0, L) with virtual +inf padding to the
@@ -1780,9 +1803,8 @@ fused_tie_rank(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
 {
     const BatchInst& I = insts[ids[blockIdx.y]];
     const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos < I.n)
-        tie_rank(pos, batch_pop(I), I.M, I.n > kSortTile ? I.key64b : I.key64, I.n > kSortTile ? I.perm_b : I.perm_a,
-                 I.perm, I.long_runs, I.counters + 13);
+    tie_rank(pos, pos < I.n, batch_pop(I), I.M, I.n > kSortTile ? I.key64b : I.key64,
+             I.n > kSortTile ? I.perm_b : I.perm_a, I.perm, I.long_runs, I.counters + 13);
 }
 
 __global__ void __launch_bounds__(kTieLongThreads)
