@@ -1212,11 +1212,13 @@ int fused_build_group(const std::vector<moea_algorithm*>& inst, const std::vecto
     for (int m = 1; m <= kMaxObjectives; ++m) {
         std::vector<int> bids, prefix{0};
         int mn = 0, mh = 0;
+        bool unit = true;
         const int shape = tile_shape ? tile_shape[m] : 0;
         for (int i : ids) {
             if (inst[i]->M != m) continue;
             bids.push_back(i);
             mh = std::max(mh, inst[i]->H);
+            unit &= inst[i]->ws.tree_delta <= kAssocMaxDelta;
             const int n = 2 * inst[i]->N;
             prefix.push_back(prefix.back() + fused_tile_blocks(m, n, shape));
             mn = std::max(mn, n);
@@ -1229,6 +1231,7 @@ int fused_build_group(const std::vector<moea_algorithm*>& inst, const std::vecto
         b.tile_blocks = prefix.back();
         b.shape = shape;
         b.max_H = mh;
+        b.unit = unit;
         MOEA_CUDA_TRY(cudaMalloc((void**)&b.d_ids, sizeof(int) * bids.size()));
         MOEA_CUDA_TRY(cudaMalloc((void**)&b.d_tile_prefix, sizeof(int) * prefix.size()));
         MOEA_CUDA_TRY(cudaMemcpy(b.d_ids, bids.data(), sizeof(int) * bids.size(), cudaMemcpyHostToDevice));

@@ -48,11 +48,110 @@ struct DenseShared {
     float margin[PTS], thr[PTS];
 };
 
+// dense_block for directions that are not of unit length (the margin is infinite
+// for every point): the pass over the tiles forms every distance itself, where
+// the re-score of all tiles would read the directions of each point again from
+// device memory.
 template <int M, int PTS>
+__device__ __noinline__ void dense_block_free(DenseShared<M, PTS>& sm, int p0, const float* __restrict__ x,
+                                                 int x_stride, const float* __restrict__ scale,
+                                                 const float* __restrict__ refs, int H, int n,
+                                                 int* __restrict__ idx_out, float* __restrict__ dist_out)
+{
+    using S = DenseShared<M, PTS>;
+    constexpr int P = S::kPer;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int sub = lane % S::kLanes, grp = lane / S::kLanes;
+    const int chunks = (H + 31) >> 5;
+    float next[M];
+    auto fetch = [&](int chunk) {
+        const int j = chunk * 32 + lane;
+#pragma unroll
+        for (int m = 0; m < M; ++m) next[m] = j < H ? __ldg(refs + (size_t)m * H + j) : 0.0f;
+    };
+    if (warp < chunks) fetch(warp);
+    float xr[P][M], best[P];
+    int bj[P];
+#pragma unroll
+    for (int c = 0; c < P; ++c) {
+        const int i = p0 + sub + S::kLanes * c;
+        best[c] = INFINITY;
+        bj[c] = -1;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const float v = i < n ? x[(size_t)m * x_stride + i] : 0.0f;
+            xr[c][m] = scale ? v * scale[m] : v;
+        }
+    }
+    for (int ch = warp; ch < chunks; ch += kDenseWarps) {
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < M; ++m) sm.dir[warp][lane][m] = next[m];
+        __syncwarp();
+        if (ch + kDenseWarps < chunks) fetch(ch + kDenseWarps);
+        const int cnt = min(32, H - ch * 32);
+#pragma unroll 2
+        for (int k = grp; k < cnt; k += S::kGroups) {
+            float r[S::kM4];
+#pragma unroll
+            for (int v = 0; v < S::kM4; v += 4) {
+                const float4 d = *reinterpret_cast<const float4*>(&sm.dir[warp][k][v]);
+                r[v] = d.x;
+                r[v + 1] = d.y;
+                r[v + 2] = d.z;
+                r[v + 3] = d.w;
+            }
+#pragma unroll
+            for (int c = 0; c < P; ++c) {
+                float dot = 0.0f, d2 = 0.0f;
+#pragma unroll
+                for (int m = 0; m < M; ++m) dot = fmaf(xr[c][m], r[m], dot);
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const float res = fmaf(-dot, r[m], xr[c][m]);
+                    d2 = fmaf(res, res, d2);
+                }
+                if (d2 < best[c]) {  // ascending directions: the first of equal ones stays
+                    best[c] = d2;
+                    bj[c] = ch * 32 + k;
+                }
+            }
+        }
+    }
+    // (distance, index) minima over the groups and the warps; none found is +inf and -1
+    unsigned long long (*found)[PTS] = reinterpret_cast<unsigned long long (*)[PTS]>(&sm.tile[0][0]);
+    static_assert(sizeof(sm.tile) >= sizeof(unsigned long long) * kDenseWarps * PTS, "minima fit the tiles' maxima");
+#pragma unroll
+    for (int c = 0; c < P; ++c) {
+        unsigned long long key = ((unsigned long long)__float_as_uint(best[c]) << 32) | (unsigned)bj[c];
+#pragma unroll
+        for (int o = S::kLanes; o < 32; o <<= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xFFFFFFFFu, key, o);
+            key = other < key ? other : key;
+        }
+        if (grp == 0) found[warp][sub + S::kLanes * c] = key;
+    }
+    __syncthreads();
+    if (tid < PTS && p0 + tid < n) {
+        unsigned long long key = found[0][tid];
+#pragma unroll
+        for (int w = 1; w < kDenseWarps; ++w) key = found[w][tid] < key ? found[w][tid] : key;
+        idx_out[p0 + tid] = (int)(unsigned)(key & 0xFFFFFFFFull);
+        dist_out[p0 + tid] = sqrtf(__uint_as_float((unsigned)(key >> 32)));
+    }
+}
+
+// kUnit: the host knows that the directions are of unit length (runs and batches;
+// a single search finds the deviation on the device).
+template <int M, int PTS, bool kUnit>
 __device__ __forceinline__ void dense_block(DenseShared<M, PTS>& sm, int p0, const float* __restrict__ x, int x_stride,
                                             const float* __restrict__ scale, const float* __restrict__ refs, int H,
                                             int n, float delta, int* __restrict__ idx_out, float* __restrict__ dist_out)
 {
+    if (!kUnit && !(delta <= kAssocMaxDelta)) {  // the same for the whole launch, or instance
+        dense_block_free<M, PTS>(sm, p0, x, x_stride, scale, refs, H, n, idx_out, dist_out);
+        return;
+    }
     using S = DenseShared<M, PTS>;
     constexpr int P = S::kPer;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -71,14 +170,17 @@ __device__ __forceinline__ void dense_block(DenseShared<M, PTS>& sm, int p0, con
     if (tid < PTS) {
         const int i = p0 + tid;
         float xx = 0.0f;
+        bool finite = true;
 #pragma unroll
         for (int m = 0; m < M; ++m) {
             float v = i < n ? x[(size_t)m * x_stride + i] : 0.0f;
             if (scale) v = v * scale[m];
             sm.x[tid][m] = v;
+            finite &= isfinite(v) != 0;
             xx = fmaf(v, v, xx);
         }
-        sm.margin[tid] = assoc_margin(M, xx, delta);
+        // a coordinate that is not finite leaves NaN distances only: no candidates
+        sm.margin[tid] = finite ? assoc_margin(M, xx, delta) : -1.0f;
     }
     __syncthreads();
     float xr[P][M];
@@ -142,10 +244,11 @@ __device__ __forceinline__ void dense_block(DenseShared<M, PTS>& sm, int p0, con
         }
         __syncthreads();
         const float thr = sm.thr[q];
+        const bool some = !(sm.margin[q] < 0.0f);
         uint32_t todo = 0u;
         for (int t = part, i = 0; t < tiles; t += kParts, ++i) {
             const float tm = sm.tile[t][q];
-            todo |= (tm * tm >= thr ? 1u : 0u) << i;
+            todo |= (some && tm * tm >= thr ? 1u : 0u) << i;
         }
         sm.todo[part][q] = todo;
         __syncthreads();
@@ -200,7 +303,7 @@ __device__ __forceinline__ void dense_block(DenseShared<M, PTS>& sm, int p0, con
     }
 }
 
-template <int M, int PTS>
+template <int M, int PTS, bool kUnit>
 __global__ void __launch_bounds__(kDenseThreads)
 assoc_dense(const float* __restrict__ x, int x_stride, const float* __restrict__ scale, const float* __restrict__ refs,
             int H, const int* __restrict__ d_n, float delta, const float* __restrict__ d_delta, int* __restrict__ idx_out,
@@ -209,12 +312,12 @@ assoc_dense(const float* __restrict__ x, int x_stride, const float* __restrict__
     extern __shared__ __align__(16) unsigned char dense_raw[];
     const int n = *d_n, p0 = blockIdx.x * PTS;
     if (p0 >= n) return;
-    dense_block<M, PTS>(*reinterpret_cast<DenseShared<M, PTS>*>(dense_raw), p0, x, x_stride, scale, refs, H, n,
+    dense_block<M, PTS, kUnit>(*reinterpret_cast<DenseShared<M, PTS>*>(dense_raw), p0, x, x_stride, scale, refs, H, n,
                       d_delta ? *d_delta : delta, idx_out, dist_out);
 }
 
 // Every instance of a bucket of M objectives (blockIdx.y).
-template <int M, int PTS>
+template <int M, int PTS, bool kUnit>
 __global__ void __launch_bounds__(kDenseThreads)
 fused_assoc_dense(const BatchInst* __restrict__ insts, const int* __restrict__ ids)
 {
@@ -222,7 +325,7 @@ fused_assoc_dense(const BatchInst* __restrict__ insts, const int* __restrict__ i
     const BatchInst& I = insts[ids[blockIdx.y]];
     const int n = I.sizes[3], p0 = blockIdx.x * PTS;
     if (p0 >= n) return;
-    dense_block<M, PTS>(*reinterpret_cast<DenseShared<M, PTS>*>(dense_raw), p0, I.nds_objs, I.n_max, I.rcp_b, I.t_dirs_orig,
+    dense_block<M, PTS, kUnit>(*reinterpret_cast<DenseShared<M, PTS>*>(dense_raw), p0, I.nds_objs, I.n_max, I.rcp_b, I.t_dirs_orig,
                       I.H, n, I.t_delta, I.assoc_idx, I.assoc_dist);
 }
 
@@ -234,51 +337,91 @@ cudaError_t dense_smem(K kernel, size_t bytes)
                              : cudaSuccess;
 }
 
-template <int M, int PTS>
+template <int M, int PTS, bool kUnit>
 int launch_dense(const float* x, int x_stride, const float* scale, const float* refs, int H, const int* d_n, int n_cap,
                  float delta, const float* d_delta, int* idx, float* dist, cudaStream_t stream)
 {
     constexpr size_t smem = sizeof(DenseShared<M, PTS>);
-    MOEA_CUDA_TRY(dense_smem(assoc_dense<M, PTS>, smem));
-    assoc_dense<M, PTS><<<ceil_div(n_cap, PTS), kDenseThreads, smem, stream>>>(x, x_stride, scale, refs, H, d_n, delta,
-                                                                               d_delta, idx, dist);
+    MOEA_CUDA_TRY((dense_smem(assoc_dense<M, PTS, kUnit>, smem)));
+    assoc_dense<M, PTS, kUnit><<<ceil_div(n_cap, PTS), kDenseThreads, smem, stream>>>(x, x_stride, scale, refs, H, d_n,
+                                                                                      delta, d_delta, idx, dist);
     MOEA_CUDA_TRY(cudaGetLastError());
     return MOEA_OK;
 }
 
-// Points from which every SM has a CTA of 64.
-constexpr int kDenseWideFrom = 148 * 64;
+// Points from which CTAs of 64 are used: half of the SMs have a second one then
+// (M=3 / 8 with 30,000 directions, CTAs of 32 and of 64: 12,500 points 126 / 171
+// and 227 / 281 us, 16,000 points 155 / 175 and 298 / 282).
+constexpr int kDenseWideFrom = 148 * 96;
+
+// Where the dense search is the faster one (both with random directions,
+// microseconds, dense / scan).  One objective: every direction is a candidate
+// (64 points, 10,000 directions 153 / 48).  Up to two chunks of directions, or few
+// beside the points, most warps have no tile (60,000 points, M=16: 33 directions
+// 44 / 16, 300 60 / 46, 1,000 93 / 115).  Two objectives: neighbouring directions
+// fall within the margin (500 points: 4,000 29 / 44, 8,000 58 / 47; 16,000
+// points: 2,000 33 / 44, 4,000 63 / 51).  Many directions and few points leave SMs
+// without a block of points (M=5, 64 points: 10,000 38 / 50, 16,000 55 / 54,
+// 100,000 290 / 100; 4,000 points: 20,000 68 / 87, 100,000 302 / 279), from twelve
+// objectives on and with directions of any length a little earlier (M=16, 64
+// points: 8,000 110 / 105, 10,000 136 / 107).
+inline bool dense_search_wins(int M, int n, int H)
+{
+    if (M == 1 || H <= 64 || (M >= 12 ? 64ll : 128ll) * H <= n) return false;
+    if (M == 2) return H <= (n < 148 * 64 ? 4096 : 2048);
+    return H <= (M >= 12 ? 8192 : 12288) || (long long)H <= 6ll * n;
+}
 
 }  // namespace
 
-int run_assoc_dense(const float* x, int x_stride, const float* scale, const float* refs, int M, const int* d_n,
-                    int n_cap, int H, float delta, const float* d_delta, int* idx, float* dist, cudaStream_t stream)
+template <bool kUnit>
+static int run_assoc_dense(const float* x, int x_stride, const float* scale, const float* refs, int M, const int* d_n,
+                           int n_cap, int H, float delta, const float* d_delta, int* idx, float* dist,
+                           cudaStream_t stream)
 {
-    if (n_cap <= 0) return MOEA_OK;
     const bool wide = n_cap >= kDenseWideFrom;
     switch (M) {
-#define MOEA_DENSE_CASE(K)                                                                                        \
-    case K:                                                                                                       \
-        return wide ? launch_dense<K, 64>(x, x_stride, scale, refs, H, d_n, n_cap, delta, d_delta, idx, dist, stream) \
-                   : launch_dense<K, 32>(x, x_stride, scale, refs, H, d_n, n_cap, delta, d_delta, idx, dist, stream);
-    MOEA_DENSE_CASE(1) MOEA_DENSE_CASE(2) MOEA_DENSE_CASE(3) MOEA_DENSE_CASE(4)
-    MOEA_DENSE_CASE(5) MOEA_DENSE_CASE(6) MOEA_DENSE_CASE(7) MOEA_DENSE_CASE(8)
-    MOEA_DENSE_CASE(9) MOEA_DENSE_CASE(10) MOEA_DENSE_CASE(11) MOEA_DENSE_CASE(12)
-    MOEA_DENSE_CASE(13) MOEA_DENSE_CASE(14) MOEA_DENSE_CASE(15) MOEA_DENSE_CASE(16)
+#define MOEA_DENSE_CASE(K)                                                                                         \
+    case K:                                                                                                        \
+        return wide ? launch_dense<K, 64, kUnit>(x, x_stride, scale, refs, H, d_n, n_cap, delta, d_delta, idx, dist, \
+                                                 stream)                                                           \
+                    : launch_dense<K, 32, kUnit>(x, x_stride, scale, refs, H, d_n, n_cap, delta, d_delta, idx, dist, \
+                                                 stream);
+    MOEA_DENSE_CASE(2) MOEA_DENSE_CASE(3) MOEA_DENSE_CASE(4) MOEA_DENSE_CASE(5) MOEA_DENSE_CASE(6)
+    MOEA_DENSE_CASE(7) MOEA_DENSE_CASE(8) MOEA_DENSE_CASE(9) MOEA_DENSE_CASE(10) MOEA_DENSE_CASE(11)
+    MOEA_DENSE_CASE(12) MOEA_DENSE_CASE(13) MOEA_DENSE_CASE(14) MOEA_DENSE_CASE(15) MOEA_DENSE_CASE(16)
 #undef MOEA_DENSE_CASE
     default: return set_error(MOEA_ERR_UNSUPPORTED, "associate: M=%d", M);
     }
 }
 
+int run_assoc_search(const float* x, int x_stride, const float* scale, const float* refs, int M, const int* d_n, int n_cap,
+                     int H, float delta, const float* d_delta, unsigned long long* best, int sms, int* idx, float* dist,
+                     cudaStream_t stream)
+{
+    if (n_cap <= 0) return MOEA_OK;
+    if (dense_search_wins(M, n_cap, H))
+        return !d_delta && delta <= kAssocMaxDelta
+                   ? run_assoc_dense<true>(x, x_stride, scale, refs, M, d_n, n_cap, H, delta, nullptr, idx, dist, stream)
+                   : run_assoc_dense<false>(x, x_stride, scale, refs, M, d_n, n_cap, H, delta, d_delta, idx, dist, stream);
+    return run_assoc_scan(x, x_stride, scale, refs, M, d_n, n_cap, H, delta, d_delta, best, sms, idx, dist, stream);
+}
+
+template <int M, bool kUnit>
+static int launch_fused_dense(const BatchInst* d_inst, const FusedBucket& b, cudaStream_t s)
+{
+    constexpr size_t smem = sizeof(DenseShared<M, 64>);
+    MOEA_CUDA_TRY((dense_smem(fused_assoc_dense<M, 64, kUnit>, smem)));
+    fused_assoc_dense<M, 64, kUnit><<<dim3(ceil_div(b.max_n, 64), b.count), kDenseThreads, smem, s>>>(d_inst, b.d_ids);
+    MOEA_CUDA_TRY(cudaGetLastError());
+    return MOEA_OK;
+}
+
 int fused_associate_dense(const BatchInst* d_inst, const FusedBucket& b, cudaStream_t s)
 {
     switch (b.M) {
-#define MOEA_DENSE_CASE(K)                                                                                         \
-    case K:                                                                                                        \
-        MOEA_CUDA_TRY(dense_smem(fused_assoc_dense<K, 64>, sizeof(DenseShared<K, 64>)));                             \
-        fused_assoc_dense<K, 64><<<dim3(ceil_div(b.max_n, 64), b.count), kDenseThreads, sizeof(DenseShared<K, 64>), s>>>( \
-            d_inst, b.d_ids);                                                                                      \
-        break;
+#define MOEA_DENSE_CASE(K) \
+    case K: return b.unit ? launch_fused_dense<K, true>(d_inst, b, s) : launch_fused_dense<K, false>(d_inst, b, s);
     MOEA_DENSE_CASE(1) MOEA_DENSE_CASE(2) MOEA_DENSE_CASE(3) MOEA_DENSE_CASE(4)
     MOEA_DENSE_CASE(5) MOEA_DENSE_CASE(6) MOEA_DENSE_CASE(7) MOEA_DENSE_CASE(8)
     MOEA_DENSE_CASE(9) MOEA_DENSE_CASE(10) MOEA_DENSE_CASE(11) MOEA_DENSE_CASE(12)
@@ -286,8 +429,6 @@ int fused_associate_dense(const BatchInst* d_inst, const FusedBucket& b, cudaStr
 #undef MOEA_DENSE_CASE
     default: return set_error(MOEA_ERR_UNSUPPORTED, "fused associate: M=%d", b.M);
     }
-    MOEA_CUDA_TRY(cudaGetLastError());
-    return MOEA_OK;
 }
 
 }  // namespace moea

@@ -182,6 +182,9 @@ __device__ __forceinline__ void copy_units4(float4* __restrict__ dst, const floa
     for (; u < units; u += lanes) dst[u] = __ldg(src + u);
 }
 
+// Directions that deviate further from unit length leave no margin: every one is a candidate.
+constexpr float kAssocMaxDelta = 1e-3f;
+
 // Margin of the dot^2 candidate filter of the association for a point with
 // |x|^2 = xx.  For directions with | |r|^2 - 1 | <= delta, the reference's
 // FP32 distance (association.cu:139-170) differs from xx - dot^2 by at most
@@ -193,7 +196,7 @@ __device__ __forceinline__ float assoc_margin(int M, float xx, float delta)
 {
     const float kEps = 5.9604645e-08f;  // 2^-24
     float margin = xx * ((16.0f * M + 64.0f) * kEps + 2.5f * delta) + 1e-35f;
-    if (!isfinite(xx) || !(delta <= 1e-3f)) margin = INFINITY;
+    if (!isfinite(xx) || !(delta <= kAssocMaxDelta)) margin = INFINITY;
     return margin;
 }
 
@@ -299,6 +302,7 @@ struct FusedBucket {
     int M = 0, count = 0, max_n = 0, tile_blocks = 0;
     int shape = 0;                 // dominator positions per row CTA (fused_tile_blocks)
     int max_H = 0;                 // most directions of an instance
+    bool unit = true;              // the directions of every instance are of unit length (kAssocMaxDelta)
     int* d_ids = nullptr;          // (count) instance indices
     int* d_tile_prefix = nullptr;  // (count + 1) first tile block of each instance
 };

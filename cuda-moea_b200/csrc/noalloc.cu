@@ -9,7 +9,8 @@
 // device in the middle of the generation's stream-ordered work, and processes
 // that cap device memory after start-up.
 //
-// Scratch per device: one count word and one delta word, fully written by
+// Scratch per device, statically sized: kStaticMaxPoints packed minima
+// (8 bytes each, 512 KiB), one count word and one delta word, all written by
 // kernels before they are read.
 //
 // The scratch is shared by every call on a device: two calls whose work
@@ -26,19 +27,23 @@
 namespace moea {
 
 int run_associate_scan_scratch(const float* x, const float* refs, int M, const int* d_n, int n_cap,
-                               int H, int* idx, float* dist, float* delta, cudaStream_t stream);
+                               int H, int* idx, float* dist, unsigned long long* best, float* delta, int sms,
+                               cudaStream_t stream);
 
 namespace {
 
 constexpr int kStaticMaxPoints = 65536;
 constexpr int kMaxDevices = 64;
 
+static __device__ __align__(256) unsigned long long g_best[kStaticMaxPoints];
 static __device__ __align__(256) int g_count[1];
 static __device__ __align__(256) float g_delta[1];
 
 struct StaticScratch {
+    unsigned long long* best = nullptr;
     int* count = nullptr;
     float* delta = nullptr;
+    int sms = 0;
 };
 
 StaticScratch g_scratch[kMaxDevices];
@@ -57,8 +62,10 @@ int scratch_for_current_device(StaticScratch& out, int& device)
         std::lock_guard<std::mutex> lock(g_setup);
         if (!g_ready[device].load(std::memory_order_relaxed)) {
             StaticScratch s;
-            cudaError_t e = cudaGetSymbolAddress((void**)&s.count, g_count);
+            cudaError_t e = cudaGetSymbolAddress((void**)&s.best, g_best);
+            if (e == cudaSuccess) e = cudaGetSymbolAddress((void**)&s.count, g_count);
             if (e == cudaSuccess) e = cudaGetSymbolAddress((void**)&s.delta, g_delta);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, device);
             if (e != cudaSuccess) {
                 cudaGetLastError();
                 return set_error(MOEA_ERR_CUDA, "associate_static: cudaGetSymbolAddress failed: %s",
@@ -92,5 +99,5 @@ extern "C" moea_status moea_associate_static(const float* d_x, const float* d_re
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     set_count_kernel<<<1, 1, 0, st>>>(s.count, n);
     MOEA_CUDA_TRY(cudaGetLastError());
-    return run_associate_scan_scratch(d_x, d_refs, M, s.count, n, H, d_idx, d_dist, s.delta, st);
+    return run_associate_scan_scratch(d_x, d_refs, M, s.count, n, H, d_idx, d_dist, s.best, s.delta, s.sms, st);
 }

@@ -882,21 +882,27 @@ constexpr int kTreeMaxDepth = kDirTreeMaxDepth;
 // (large problems) or the dense one is cheaper than a warp per point over the
 // tree.
 constexpr int kTreeMaxObjectives = 5;
-// Whether the dense search is the faster one at or below that many objectives.
-// The tree takes 2-3 ns per point whatever the directions when points fill the
-// device and a few microseconds when they do not; the dense search H (M + 1)
-// instructions per point.  Up to three objectives the tree prunes well, so the
-// dense search wins with many points and few directions only (N=32768: 1,891
-// directions 78 -> 33 us, 4,005 78 -> 53, 8,128 even; N=4096, 4,005 directions
-// 20 -> 23 us).  At four and five it wins up to about 8,192 directions (M=5:
-// N=3002, 2,380 directions 49 -> 20 us; N=8192, 5,985 directions 100 -> 49).
+// Whether a search over every direction is the faster one at or below that many
+// objectives.  The tree takes 2-3 ns per point whatever the directions when
+// points fill the device and a few microseconds when they do not; the dense
+// search H (M + 1) instructions per point.  Up to three objectives the tree
+// prunes well, so the dense search wins with many points and few directions only
+// (N=32768: 1,891 directions 78 -> 33 us, 4,005 78 -> 53, 8,128 even; N=4096,
+// 4,005 directions 20 -> 23 us).  At four and five it wins up to about 8,192
+// directions (M=5: N=3002, 2,380 directions 49 -> 20 us; N=8192, 5,985 directions
+// 100 -> 49).
 inline bool dense_preferred(int M, int n_cap, int H)
 {
     return M <= 3 ? 16ll * H <= n_cap : H <= 8192;
 }
+// Directions that are not of unit length leave the tree nothing to skip (20
+// generations of N=4096 with 9,000 such directions of three objectives: 24.9 ms,
+// 3.5 with every direction visited), so they always take the other search.
 // In a batch the instances fill the device together (85 instances a launch:
-// M=3 295 -> 150 us, M=5 783 -> 216 us).
-inline bool dense_preferred_batch(int max_h) { return max_h <= 8192; }
+// M=3 295 -> 150 us, M=5 783 -> 216 us).  One and two objectives: as in the dense
+// search's own rule (20 generations of 64 instances of two objectives: 8,000
+// directions 2.2 ms with the tree, 3.4 dense; 3,000 2.18 and 2.33; 300 even).
+inline bool dense_preferred_batch(int M, int max_h) { return M == 1 ? false : max_h <= (M == 2 ? 2048 : 8192); }
 
 struct TreeArgs {
     const float* dirs;    // (M, H) in tree order
@@ -1668,7 +1674,8 @@ int run_associate(Workspace& ws, const float* x, int x_stride, const float* scal
     if (mode == MOEA_ASSOC_TREE) {
         if (!direction_tree_ready(ws, refs, M, H))
             return set_error(MOEA_ERR_STATE, "associate: no cone tree prepared for these directions");
-        if (ws.tree_depth <= kTreeMaxDepth && M <= kTreeMaxObjectives && !dense_preferred(M, n_cap, H)) {
+        if (ws.tree_depth <= kTreeMaxDepth && M <= kTreeMaxObjectives && ws.tree_delta <= kAssocMaxDelta &&
+            !dense_preferred(M, n_cap, H)) {
             const TreeArgs t{ws.tree_dirs, ws.tree_order, ws.tree_center, ws.tree_cos, ws.tree_sin,
                              ws.tree_link, H, ws.tree_nodes, ws.tree_delta};
             const int blocks = ceil_div(n_cap, kTreeWarps);
@@ -1687,20 +1694,22 @@ int run_associate(Workspace& ws, const float* x, int x_stride, const float* scal
         // than the kernel's stack -- the dense search
         if (tensor_preferred(M, n_cap, H) && tensor_directions_ready(ws, refs, M, H))
             return run_associate_tensor(ws, x, x_stride, scale, refs, M, d_n, n_cap, H, idx, dist, stream);
-        return run_assoc_dense(x, x_stride, scale, refs, M, d_n, n_cap, H, ws.tree_delta, nullptr, idx, dist, stream);
+        return run_assoc_search(x, x_stride, scale, refs, M, d_n, n_cap, H, ws.tree_delta, nullptr, ws.assoc_best, ws.sm_count,
+                                idx, dist, stream);
     }
     MOEA_TRY(run_dir_delta(refs, M, H, ws.dir_delta, stream));
-    return run_assoc_dense(x, x_stride, scale, refs, M, d_n, n_cap, H, 0.0f, ws.dir_delta, idx, dist, stream);
+    return run_assoc_search(x, x_stride, scale, refs, M, d_n, n_cap, H, 0.0f, ws.dir_delta, ws.assoc_best, ws.sm_count, idx,
+                            dist, stream);
 }
 
 // The full-scan association with caller-provided scratch instead of a
-// workspace: delta (1 float), d_n (device count).  Used by the allocation-free
-// entry point (noalloc.cu).
+// workspace: best (n_cap packed minima), delta (1 float), d_n (device count).
+// Used by the allocation-free entry point (noalloc.cu).
 int run_associate_scan_scratch(const float* x, const float* refs, int M, const int* d_n, int n_cap, int H, int* idx,
-                               float* dist, float* delta, cudaStream_t stream)
+                               float* dist, unsigned long long* best, float* delta, int sms, cudaStream_t stream)
 {
     MOEA_TRY(run_dir_delta(refs, M, H, delta, stream));
-    return run_assoc_dense(x, n_cap, nullptr, refs, M, d_n, n_cap, H, 0.0f, delta, idx, dist, stream);
+    return run_assoc_search(x, n_cap, nullptr, refs, M, d_n, n_cap, H, 0.0f, delta, best, sms, idx, dist, stream);
 }
 
 int run_niching(Workspace& ws, uint64_t seed, const int* nds_gidx, const float* dist,
@@ -1846,7 +1855,7 @@ int fused_select(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s)
 #define MOEA_FP_CASE(K)                                                                              \
         case K:                                                                                      \
             fused_prep<K><<<b.count, kFusedThreads, 0, s>>>(d_inst, b.d_ids);                        \
-            if (K <= kTreeMaxObjectives && !dense_preferred_batch(b.max_H))                          \
+            if (K <= kTreeMaxObjectives && b.unit && !dense_preferred_batch(K, b.max_H))             \
                 fused_assoc<K><<<dim3(ceil_div(b.max_n, kTreeWarps), b.count), kTreeWarps * 32, 0,    \
                                  s>>>(d_inst, b.d_ids);                                              \
             else                                                                                     \
