@@ -1123,6 +1123,127 @@ __device__ unsigned long long counted_arrive(unsigned long long* word, unsigned 
     }
 }
 
+// Highest unassigned dominator of a row in its words 0 .. sw (-1: none), found
+// by G lanes of a warp (l their rank, the same result in each): 256 words a
+// step, in chunks of four from the top, those without unassigned points not
+// read at all.  Every lane of the warp calls it, a group without a row with
+// sw = -1.
+template <int G>
+__device__ __forceinline__ int scan_row_group(const uint32_t* __restrict__ row, const uint32_t* U, int sw, int l)
+{
+    constexpr int kLoads = 64 / G;  // 16-byte chunks a lane has in flight
+    const uint4* row4 = reinterpret_cast<const uint4*>(row);
+    const uint4* U4 = reinterpret_cast<const uint4*>(U);
+    int found = -1;
+    int top = sw >= 0 ? sw >> 2 : -1;  // highest chunk not yet read
+    while (__any_sync(0xFFFFFFFFu, top >= 0)) {
+        uint4 v[kLoads];
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) {
+            const int c = top - l - G * i;
+            v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (c < 0) continue;
+            uint4 u = U4[c];
+            if (4 * c + 3 > sw) {  // words above the start are probed, or not of this row
+                u.w = 0u;
+                if (4 * c + 2 > sw) u.z = 0u;
+                if (4 * c + 1 > sw) u.y = 0u;
+            }
+            if (u.x | u.y | u.z | u.w) {
+                const uint4 r = __ldg(row4 + c);
+                v[i] = make_uint4(r.x & u.x, r.y & u.y, r.z & u.z, r.w & u.w);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) {
+            if (found >= 0 || !(v[i].x | v[i].y | v[i].z | v[i].w)) continue;
+            const int w = v[i].w ? 3 : v[i].z ? 2 : v[i].y ? 1 : 0;
+            const uint32_t bb = v[i].w ? v[i].w : v[i].z ? v[i].z : v[i].y ? v[i].y : v[i].x;
+            found = (4 * (top - l - G * i) + w) * 32 + (31 - __clz(bb));
+        }
+#pragma unroll
+        for (int o = G / 2; o; o >>= 1) found = max(found, __shfl_xor_sync(0xFFFFFFFFu, found, o));
+        top = found >= 0 ? -1 : top - 64;
+    }
+    return found;
+}
+
+// Thin fronts by one CTA.  A front of a few points costs the grid a barrier
+// (about 3 us with its round trips through L2), one CTA three block barriers and
+// a row read.  When the first kThinAfter fronts hold at most thin_total points,
+// CTA 0 goes on alone with every point's blocker in its shared memory (five
+// generations of DTLZ4, M=2: N=1024 6.7 -> 3.7 ms, N=4096 24.9 -> 20.3; sorts of
+// 2000 and 8000 points along a chain 2.5 -> 1.3 and 7.4 -> 4.3 ms).  Larger
+// populations have thicker fronts at the same total, whose rows one CTA reads
+// more slowly: M=2 with 34 points a front, N=2048, 18.7 ms by the grid and 21.3.
+// A call, so that the grid's loop keeps its registers.
+constexpr int kSoloPoints = 8192;
+constexpr int kThinAfter = 8;
+__device__ __forceinline__ int thin_total(int nf) { return nf <= 2048 ? 160 : nf <= 4096 ? 96 : 64; }
+static_assert(kSoloPoints * (sizeof(int) + sizeof(unsigned short)) <= kWinChunks * kPeelThreads * sizeof(uint4),
+              "blockers and queue fit the windows' shared memory");
+
+// Fronts k, k + 1, ... of nf points: U without the fronts before, which hold
+// `total` points.  mem: the windows' shared memory.  Ends with the counters as
+// nds_peel_owned.
+__device__ __noinline__ void peel_solo(const uint32_t* __restrict__ rows, int W, int nf, int target, bool feasible_only,
+                                          int feasible, const int* __restrict__ blocker0, int* __restrict__ front_sorted,
+                                          uint32_t* U, void* mem, int k, int total, int* counters)
+{
+    __shared__ int s_queued[2], s_free[2];
+    int* blk = reinterpret_cast<int*>(mem);  // unassigned dominator a point waits for, -1: assigned
+    unsigned short* queue = reinterpret_cast<unsigned short*>(blk + kSoloPoints);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    constexpr int kWarps = kPeelThreads / 32;
+    for (int q = t; q < nf; q += kPeelThreads) blk[q] = ((U[q >> 5] >> (q & 31)) & 1u) ? blocker0[q] : -1;
+    if (t < 2) s_queued[t] = s_free[t] = 0;
+    __syncthreads();
+    for (;; ++k) {
+        const int par = k & 1;
+        for (int q = t; q < nf; q += kPeelThreads) {
+            const int b = blk[q];
+            if (b >= 0 && !((U[b >> 5] >> (b & 31)) & 1u)) queue[atomicAdd(&s_queued[par], 1)] = (unsigned short)q;
+        }
+        __syncthreads();
+        const int qn = s_queued[par];
+        if (t == 0) s_queued[par ^ 1] = s_free[par ^ 1] = 0;  // last read before this barrier
+        // up to one row per warp by all its lanes, else four by eight lanes each
+        const int width = qn <= kWarps ? 32 : 8;
+        for (int e0 = 0; e0 < qn; e0 += kWarps * (32 / width)) {
+            const int e = e0 + warp + kWarps * (lane / width);
+            const bool act = e < qn;
+            const int q = act ? queue[e] : 0;
+            const int sw = act ? blk[q] >> 5 : -1;
+            const uint32_t* row = rows + (size_t)q * W;
+            const int found = width == 32 ? scan_row_group<32>(row, U, sw, lane) : scan_row_group<8>(row, U, sw, lane & 7);
+            if (act && (lane & (width - 1)) == 0) {
+                blk[q] = found;
+                if (found < 0) {
+                    front_sorted[q] = k;
+                    atomicAdd(&s_free[par], 1);
+                }
+            }
+        }
+        __syncthreads();
+        const int ck = s_free[par];
+        for (int e = t; e < qn; e += kPeelThreads) {
+            const int q = queue[e];
+            if (blk[q] < 0) atomicAnd(U + (q >> 5), ~(1u << (q & 31)));
+        }
+        __syncthreads();
+        total += ck;
+        if (total >= target || ck == 0 || (feasible_only && total >= feasible)) {
+            if (t == 0) {
+                counters[2] = k;
+                counters[3] = total;
+                counters[12] = k;
+                if (ck == 0 && total < (feasible_only ? feasible : target)) atomicExch(counters + 6, kDevPeelInconsistent);
+            }
+            return;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kPeelThreads, 1)
 nds_peel_owned(const uint32_t* __restrict__ rows, int W, int n, int target, const int* __restrict__ blocker0,
                int* __restrict__ front_sorted, uint32_t* __restrict__ fmask, int* counters)
@@ -1333,6 +1454,14 @@ nds_peel_owned(const uint32_t* __restrict__ rows, int W, int n, int target, cons
                     atomicExch(counters + 6, kDevPeelInconsistent);
             }
             cp_async_wait_all();
+            return;
+        }
+        if (k == kThinAfter - 1 && total <= thin_total(nf) && nf <= kSoloPoints) {  // the same in every CTA
+            cp_async_wait_all();
+            __syncthreads();  // no window is in use any more
+            if (blockIdx.x == 0)
+                peel_solo(rows, W, nf, target, feasible_only, feasible, blocker0, front_sorted, U, s_win, k + 1, total,
+                          counters);
             return;
         }
         ++k;
@@ -1897,51 +2026,6 @@ fused_tiles_one(const BatchInst* __restrict__ insts, const int* __restrict__ ids
 
 constexpr int kFusedPeelThreads = 1024;
 constexpr int kWalkHops = 64;  // waiting points followed from one member before the pass over all points
-
-// Highest unassigned dominator of a row in its words 0 .. sw (-1: none), found
-// by G lanes of a warp (l their rank, the same result in each): 256 words a
-// step, in chunks of four from the top, those without unassigned points not
-// read at all.  Every lane of the warp calls it, a group without a row with
-// sw = -1.
-template <int G>
-__device__ __forceinline__ int scan_row_group(const uint32_t* __restrict__ row, const uint32_t* U, int sw, int l)
-{
-    constexpr int kLoads = 64 / G;  // 16-byte chunks a lane has in flight
-    const uint4* row4 = reinterpret_cast<const uint4*>(row);
-    const uint4* U4 = reinterpret_cast<const uint4*>(U);
-    int found = -1;
-    int top = sw >= 0 ? sw >> 2 : -1;  // highest chunk not yet read
-    while (__any_sync(0xFFFFFFFFu, top >= 0)) {
-        uint4 v[kLoads];
-#pragma unroll
-        for (int i = 0; i < kLoads; ++i) {
-            const int c = top - l - G * i;
-            v[i] = make_uint4(0u, 0u, 0u, 0u);
-            if (c < 0) continue;
-            uint4 u = U4[c];
-            if (4 * c + 3 > sw) {  // words above the start are probed, or not of this row
-                u.w = 0u;
-                if (4 * c + 2 > sw) u.z = 0u;
-                if (4 * c + 1 > sw) u.y = 0u;
-            }
-            if (u.x | u.y | u.z | u.w) {
-                const uint4 r = __ldg(row4 + c);
-                v[i] = make_uint4(r.x & u.x, r.y & u.y, r.z & u.z, r.w & u.w);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kLoads; ++i) {
-            if (found >= 0 || !(v[i].x | v[i].y | v[i].z | v[i].w)) continue;
-            const int w = v[i].w ? 3 : v[i].z ? 2 : v[i].y ? 1 : 0;
-            const uint32_t bb = v[i].w ? v[i].w : v[i].z ? v[i].z : v[i].y ? v[i].y : v[i].x;
-            found = (4 * (top - l - G * i) + w) * 32 + (31 - __clz(bb));
-        }
-#pragma unroll
-        for (int o = G / 2; o; o >>= 1) found = max(found, __shfl_xor_sync(0xFFFFFFFFu, found, o));
-        top = found >= 0 ? -1 : top - 64;
-    }
-    return found;
-}
 
 // Peel of one instance per CTA in shared memory.  Every unassigned point waits
 // for one unassigned dominator, its blocker, and the points that wait for the
