@@ -234,8 +234,10 @@ int run_variation_pass(int passes, const float* parents, const int* pidx, const 
         const bool vec = (D & 3) == 0 && ((uintptr_t)parents & 15) == 0 && ((uintptr_t)off & 15) == 0 &&
                          ((uintptr_t)bounds & 15) == 0;
         if (vec && D >= kRowCrossoverD && (n_off & 1) == 0 && count < (1ll << 31)) {
-            // 32 blocks per SM in flight, rows split into blocks of 256 groups
-            const int gx = std::min(ceil_div(D / 4, 256), 64);
+            // 32 blocks per SM in flight, rows split into blocks of 256 groups: up
+            // to 64 a row, or as many as fill the device with few pairs (one pair
+            // of 2^20 variables 29 us with 64, @@ now)
+            const int gx = std::min(ceil_div(D / 4, 256), std::max(64, 148 * 32 / (n_off / 2 > 0 ? n_off / 2 : 1)));
             const dim3 grid(gx, std::max(1, std::min(n_off / 2, 148 * 32 / gx)));
             if (sbx_prob >= 1.0f && copy_prob <= 0.0f)
                 crossover_rows<true><<<grid, 256, 0, stream>>>(parents, pidx, bounds, off, n_off / 2, D, sbx_eta0, sbx_eta1,

@@ -81,6 +81,20 @@ __device__ __forceinline__ void stage_directions(float (&s)[M][kDirStage], const
     __syncthreads();
 }
 
+// The largest cosine of the warp's lanes, the smallest direction index on ties.
+__device__ __forceinline__ void warp_best_direction(float& best, int& bj)
+{
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const float ob = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+        const int oj = __shfl_xor_sync(0xFFFFFFFFu, bj, o);
+        if (ob > best || (ob == best && oj >= 0 && (bj < 0 || oj < bj))) {
+            best = ob;
+            bj = oj;
+        }
+    }
+}
+
 // The direction of largest cosine of the warp's point x: lane l takes the
 // directions l, l + 32, ... with the same FMA order over m as a sequential
 // scan, keeps the first maximum it meets, and the warp reduces to the largest
@@ -108,21 +122,48 @@ __device__ __forceinline__ void nearest_direction(float (&s)[M][kDirStage], cons
             }
         }
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        const float ob = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-        const int oj = __shfl_xor_sync(0xFFFFFFFFu, bj, o);
-        if (ob > best || (ob == best && oj >= 0 && (bj < 0 || oj < bj))) {
-            best = ob;
-            bj = oj;
-        }
-    }
+    warp_best_direction(best, bj);
     *best_out = best;
     *bj_out = bj;
 }
 
-// A warp per point.
+// nearest_direction with the directions read from device memory by each warp.
 template <int M>
+__device__ __forceinline__ void nearest_direction_direct(const float (&x)[M], float inv_norm,
+                                                         const float* __restrict__ refs, int K, float* best_out,
+                                                         int* bj_out)
+{
+    float best = -CUDART_INF_F;
+    int bj = -1;
+    for (int j = threadIdx.x & 31; j < K; j += 32) {
+        float dot = 0.f;
+#pragma unroll
+        for (int m = 0; m < M; ++m) dot = fmaf(x[m], __ldg(refs + (size_t)m * K + j), dot);
+        const float c = dot * inv_norm;
+        if (c > best) {
+            best = c;
+            bj = j;
+        }
+    }
+    warp_best_direction(best, bj);
+    *best_out = best;
+    *bj_out = bj;
+}
+
+// Whether the warps read the directions themselves.  Staging hides the cold lines
+// of a few CTAs; with thousands of them the directions stay in L1 and the
+// staging is extra work (microseconds, staged / direct: M=3, K=3000, 2000 points
+// 13.7 / 16.7, 20,000 39.6 / 35.6, 60,000 107 / 88; M=8, 20,000 points 79 / 79,
+// 60,000 223 / 193; M=16, 60,000 points, K=91 44 / 34, K=3000 481 / 522).
+inline bool partition_direct(int M, int n, int K)
+{
+    if (M <= 2) return n > 4096;
+    if (K <= 128) return n >= 16384;
+    return K <= 8192 && (M <= 3 ? n >= 16384 : M <= 8 && n >= 40960);
+}
+
+// A warp per point.
+template <int M, bool kStaged>
 __global__ void __launch_bounds__(256)
 partition_kernel(const float* __restrict__ t, int t_stride, int n, const float* __restrict__ refs,
                  int K, const int* __restrict__ d_active, int n_active_host, int n_parent,
@@ -130,7 +171,7 @@ partition_kernel(const float* __restrict__ t, int t_stride, int n, const float* 
 {
     const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
-    __shared__ float s_dir[M][kDirStage];
+    if (!kStaged && i >= n) return;  // uniform over the warp
     float x[M];
     float sqr = 0.f;
 #pragma unroll
@@ -142,7 +183,12 @@ partition_kernel(const float* __restrict__ t, int t_stride, int n, const float* 
     const float inv_norm = rsqrtf(sqr + 1e-12f);
     float best;
     int bj;
-    nearest_direction<M>(s_dir, x, inv_norm, refs, K, &best, &bj);
+    if constexpr (kStaged) {
+        __shared__ float s_dir[M][kDirStage];
+        nearest_direction<M>(s_dir, x, inv_norm, refs, K, &best, &bj);
+    } else {
+        nearest_direction_direct<M>(x, inv_norm, refs, K, &best, &bj);
+    }
     if (lane != 0 || i >= n) return;
     theta[i] = (best > -CUDART_INF_F) ? acosf(fminf(fmaxf(best, 0.f), 1.f)) : CUDART_INF_F;
     const int n_active = d_active ? *d_active : n_active_host;
@@ -686,8 +732,13 @@ int run_rvea_partition(const float* t, int t_stride, int n, const float* refs, i
                        const int* d_active, int n_active, int n_parent, float* theta, int* idx,
                        cudaStream_t s)
 {
-    MOEA_DISPATCH_M(M, (partition_kernel<MM><<<ceil_div(n, 8), 256, 0, s>>>(
-                           t, t_stride, n, refs, K, d_active, n_active, n_parent, theta, idx)));
+    if (partition_direct(M, n, K)) {
+        MOEA_DISPATCH_M(M, (partition_kernel<MM, false><<<ceil_div(n, 8), 256, 0, s>>>(
+                               t, t_stride, n, refs, K, d_active, n_active, n_parent, theta, idx)));
+    } else {
+        MOEA_DISPATCH_M(M, (partition_kernel<MM, true><<<ceil_div(n, 8), 256, 0, s>>>(
+                               t, t_stride, n, refs, K, d_active, n_active, n_parent, theta, idx)));
+    }
     MOEA_CUDA_TRY(cudaGetLastError());
     return MOEA_OK;
 }
