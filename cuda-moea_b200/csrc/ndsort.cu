@@ -254,10 +254,10 @@ constexpr int kTieSmemSort = 4096;    // longer runs: bitonic in shared memory u
 // Runs of equal keys in class 0 into lexicographic order: every member of a run
 // of at most kTieShort counts the members before it; longer runs are copied
 // and listed for nds_tie_fix_long.  Every lane of the warp calls, with active
-// false past the last point.  The lanes of a run step through it together, and
-// no lane leaves a comparison early: lanes that each followed their own loops
-// ran one after another (5000 points of 243 vectors of five objectives: 258 us,
-// 20 now; points without ties 3-4 us either way).
+// false past the last point.  The lanes of the warp step through their runs
+// together, and no lane leaves a comparison early: lanes that each followed their
+// own loops ran one after another (5000 points of 243 vectors of five objectives:
+// 258 us, 16 now; points without ties 3-4 us either way).
 __device__ __forceinline__ void tie_rank(int pos, bool active, const SplitPop& pop, int M,
                                          const uint64_t* __restrict__ skey, const int* __restrict__ perm_in,
                                          int* __restrict__ perm_out, int* __restrict__ long_runs,
@@ -287,15 +287,18 @@ __device__ __forceinline__ void tie_rank(int pos, bool active, const SplitPop& p
     }
     const int steps = __reduce_max_sync(0xFFFFFFFFu, members);
     for (int i = 0; i < steps; ++i) {
-        const int other = i < members ? perm_in[a + i] : pt;
-        bool less = false, equal = true;
+        if (i < members) {
+            const int other = perm_in[a + i];
+            bool less = false, equal = true;
 #pragma unroll 4
-        for (int m = 1; m < M; ++m) {
-            const uint32_t ka = float_order_key(pop.obj(m, other)), kb = float_order_key(pop.obj(m, pt));
-            less |= equal && ka < kb;
-            equal &= ka == kb;
+            for (int m = 1; m < M; ++m) {
+                const uint32_t ka = float_order_key(pop.obj(m, other)), kb = float_order_key(pop.obj(m, pt));
+                less |= equal && ka < kb;
+                equal &= ka == kb;
+            }
+            to += (less || (equal && other < pt)) ? 1 : 0;
         }
-        to += (less || (equal && other < pt)) ? 1 : 0;
+        __syncwarp();
     }
     if (active) perm_out[to] = pt;
 }
@@ -1456,7 +1459,7 @@ nds_peel_owned(const uint32_t* __restrict__ rows, int W, int n, int target, cons
             cp_async_wait_all();
             return;
         }
-        if (k == kThinAfter - 1 && total <= thin_total(nf) && nf <= kSoloPoints) {  // the same in every CTA
+        if (__builtin_expect(k == kThinAfter - 1, 0) && total <= thin_total(nf) && nf <= kSoloPoints) {  // the same in every CTA
             cp_async_wait_all();
             __syncthreads();  // no window is in use any more
             if (blockIdx.x == 0)

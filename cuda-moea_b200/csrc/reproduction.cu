@@ -236,7 +236,7 @@ int run_variation_pass(int passes, const float* parents, const int* pidx, const 
         if (vec && D >= kRowCrossoverD && (n_off & 1) == 0 && count < (1ll << 31)) {
             // 32 blocks per SM in flight, rows split into blocks of 256 groups: up
             // to 64 a row, or as many as fill the device with few pairs (one pair
-            // of 2^20 variables 29 us with 64, @@ now)
+            // of 2^20 variables with its mating and mutation 29 us with 64, 21 now)
             const int gx = std::min(ceil_div(D / 4, 256), std::max(64, 148 * 32 / (n_off / 2 > 0 ? n_off / 2 : 1)));
             const dim3 grid(gx, std::max(1, std::min(n_off / 2, 148 * 32 / gx)));
             if (sbx_prob >= 1.0f && copy_prob <= 0.0f)
