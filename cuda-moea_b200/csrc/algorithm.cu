@@ -1312,6 +1312,7 @@ struct moea_batch {
     int setup_fused(const std::vector<int>* schedule = nullptr)
     {
         if (!fused_possible()) return MOEA_OK;
+        MOEA_TRY(fused_offspring_configure());
         MOEA_TRY(fused_ndsort_configure());
         MOEA_TRY(fused_select_configure());
         const int count = (int)inst.size();

@@ -323,6 +323,7 @@ int fused_tile_blocks(int M, int n, int shape);  // tile CTAs of one instance in
 constexpr int kTileShapes = 2;
 // Kernel attributes (shared memory opt-in) of the fused stages, set once per
 // device before any capture.
+int fused_offspring_configure();
 int fused_ndsort_configure();
 int fused_select_configure();
 

@@ -139,12 +139,22 @@ int run_offspring(OffspringArgs A, cudaStream_t stream)
     return MOEA_OK;
 }
 
+// The shared-memory limit of fused_offspring for the longest rows that a fused
+// batch holds (256 g-terms behind kMaxObjectives - 1 position variables).  The
+// limit belongs to the function: set by each launch for its own rows, a smaller
+// launch on another thread could lower it under a larger one.
+int fused_offspring_configure()
+{
+    constexpr int kPairs = kOffThreads / kFusedGroup;
+    MOEA_CUDA_TRY(cudaFuncSetAttribute(fused_offspring, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(float) * kPairs * offspring_stride(256 + kMaxObjectives - 1)));
+    return MOEA_OK;
+}
+
 int fused_reproduce(const BatchInst* d_inst, const FusedGroup& g, cudaStream_t s)
 {
     constexpr int kPairs = kOffThreads / kFusedGroup;
     const size_t smem = sizeof(float) * kPairs * offspring_stride(g.max_D);
-    if (smem > 48 * 1024)
-        MOEA_CUDA_TRY(cudaFuncSetAttribute(fused_offspring, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     fused_offspring<<<dim3(ceil_div((g.max_N + 1) / 2, kPairs), g.count), kOffThreads, smem, s>>>(d_inst, g.d_ids);
     MOEA_CUDA_TRY(cudaGetLastError());
     return MOEA_OK;
