@@ -31,6 +31,7 @@
 
 #include "internal.cuh"
 #include "niche_select.cuh"
+#include "per_device.h"
 
 namespace cg = cooperative_groups;
 
@@ -615,24 +616,15 @@ bool nich_select_solo(int n_mix, int H) { return n_mix <= kNcSlice && H <= 2 * k
 
 int niching_cluster_capacity() { return kNcCtas * kNcSlice; }
 
-// Whether the cluster kernel can run on the current device (attributes are
-// set once per process; a device that cannot co-schedule the cluster keeps
-// the library sort).
-bool niching_cluster_ready()
+namespace {
+
+// Sets the attributes of the selection kernels on the current device; false when
+// it cannot co-schedule their cluster.
+bool configure_niching_cluster()
 {
-    static int state = -1;  // -1 unknown, 0 no, 1 yes
-    if (state >= 0) return state == 1;
-    state = 0;
-    if (cudaFuncSetAttribute(nich_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(nich_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(NcShared)) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kNcCtas);
     cfg.blockDim = dim3(kNcThreads);
-    cfg.dynamicSmemBytes = sizeof(NcShared);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = kNcCtas;
@@ -641,26 +633,42 @@ bool niching_cluster_ready()
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, (void*)nich_cluster, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    if (clusters < 1) return false;
-    if (cudaFuncSetAttribute(nich_select<NicheCluster>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(nich_select<NicheCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(NcSelectShared)) != cudaSuccess ||
-        cudaFuncSetAttribute(nich_select<NicheSolo>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(NcSelectShared)) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
+    cudaError_t e = cudaFuncSetAttribute(nich_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(nich_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NcShared));
+    cfg.dynamicSmemBytes = sizeof(NcShared);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, (void*)nich_cluster, &cfg);
+    if (e == cudaSuccess && clusters < 1) return false;
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(nich_select<NicheCluster>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(nich_select<NicheCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(NcSelectShared));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(nich_select<NicheSolo>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(NcSelectShared));
     cfg.dynamicSmemBytes = sizeof(NcSelectShared);
-    if (cudaOccupancyMaxActiveClusters(&clusters, (void*)nich_select<NicheCluster>, &cfg) != cudaSuccess) {
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, (void*)nich_select<NicheCluster>, &cfg);
+    if (e != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    state = clusters >= 1 ? 1 : 0;
-    return state == 1;
+    return clusters >= 1;
+}
+
+}  // namespace
+
+// Whether the cluster kernels can run on the current device; one that cannot
+// co-schedule the cluster keeps the library sort.
+bool niching_cluster_ready()
+{
+    static PerDevice answers;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return answers.get(device, configure_niching_cluster);
 }
 
 int launch_niching_cluster(const int* idx, const float* dist, const int* sizes, const int* rho, int H,

@@ -21,6 +21,7 @@
 #include "internal.cuh"
 #include "niche_select.cuh"
 #include "dirtree.h"
+#include "per_device.h"
 
 namespace cg = cooperative_groups;
 
@@ -699,33 +700,41 @@ int prep_ctas(int n)
 
 constexpr int kPrepCapacity = kPrepCtas * kPrepTiles * kPrepThreads;
 
-// Whether the device can place the sixteen-CTA cluster (once per process).
+// Allows nsga3_prep its sixteen-CTA cluster on the current device; false when the
+// device cannot place it.
+template <int M>
+bool configure_prep()
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kPrepCtas);
+    cfg.blockDim = dim3(kPrepThreads);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kPrepCtas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    cudaError_t e = cudaFuncSetAttribute(nsga3_prep<M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, (void*)nsga3_prep<M>, &cfg);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return clusters >= 1;
+}
+
 template <int M>
 bool prep_ready()
 {
-    static const bool ok = [] {
-        if (cudaFuncSetAttribute(nsga3_prep<M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(kPrepCtas);
-        cfg.blockDim = dim3(kPrepThreads);
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = kPrepCtas;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, (void*)nsga3_prep<M>, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        return clusters >= 1;
-    }();
-    return ok;
+    static PerDevice answers;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return answers.get(device, configure_prep<M>);
 }
 
 template <int M>
