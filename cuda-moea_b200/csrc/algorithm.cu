@@ -821,9 +821,19 @@ struct moea_algorithm {
             const int parity = (P == 0) ? 0 : 1;
             if (!graph[parity]) {
                 cudaGraph_t g = nullptr;
-                MOEA_CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-                const int st = whole ? generation_body() : select_body();
-                cudaError_t ce = cudaStreamEndCapture(stream, &g);
+                const cudaError_t begun = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+                if (begun != cudaSuccess) cudaGetLastError();
+                if (whole && begun != cudaSuccess)
+                    return set_error(MOEA_ERR_CUDA, "graph capture of a generation: %s", cudaGetErrorString(begun));
+                // a callback problem may run on a stream that cannot be
+                // captured (the legacy default stream): its selection is then
+                // launched directly
+                int st = MOEA_ERR_CUDA;
+                cudaError_t ce = begun;
+                if (begun == cudaSuccess) {
+                    st = whole ? generation_body() : select_body();
+                    ce = cudaStreamEndCapture(stream, &g);
+                }
                 if (st == MOEA_OK && ce == cudaSuccess) {
                     size_t count = 0;
                     if (cudaGraphGetNodes(g, nullptr, &count) == cudaSuccess && count > 0) {
