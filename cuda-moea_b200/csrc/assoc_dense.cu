@@ -12,8 +12,9 @@
 // the directions of the tiles whose largest dot^2 reaches the point's threshold
 // -- one or two tiles of 32 for most points, a warp per point, a lane per
 // direction.  The minimum of (d2, index) over them is the reference's argmin
-// with its tie rule.  Points whose margin is infinite (non-finite, or
-// directions far from unit length) re-score every tile.
+// with its tie rule.  Points whose squared length overflows re-score every tile,
+// points with a coordinate that is not finite none; directions far from unit
+// length take one pass over every distance (dense_block_free).
 //
 // A CTA holds 32 or 64 points; its eight warps take the tiles in turn, each
 // through its own 32-direction buffer in shared memory, so the first pass has

@@ -1,7 +1,7 @@
 // Niche selection of the last front by direction buckets, and the ordered
-// survivor list, in one kernel: device code shared by the cluster kernel of
-// the staged path (niching_cluster.cu) and the one-CTA kernel of the fused
-// path (nsga3.cu).
+// survivor list, in one kernel: device code shared by the staged path
+// (niching_cluster.cu: one CTA or a cluster of sixteen) and the batches (nsga3.cu:
+// a cluster of two per instance).
 //
 // The reference selects with three stable sorts of the last front's members
 // (niching.cu:96-178); the random words of the second and third hash the

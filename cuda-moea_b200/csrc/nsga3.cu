@@ -482,7 +482,7 @@ norm_finalize(const float* __restrict__ nds, int nds_stride, const float* __rest
 // selection in one cluster: what run_extract, run_ideal and the two launches
 // of the normalisation do, with one pass over the fronts and two cluster
 // barriers instead of five launches.  CTA c holds a contiguous segment of the
-// points, thread t of its tile j the point c S + 1024-aligned tile + t; the
+// points, thread t of its tile j the segment's point j kPrepThreads + t; the
 // class counts, the minima and the extreme-point candidates pass through the
 // cluster's shared memory, and CTA 0 solves for the intercepts.  Bound by the
 // latency of its two barriers and of the solve.  Measured with the launches
@@ -804,7 +804,7 @@ int dispatch_norm(Workspace& ws, const SplitPop& pop, const int* gidx, const int
 // ---------------------------------------------------------------------------
 // The searches share one rule: the reference's argmin lies among the directions
 // whose dot^2 comes within a rounding margin of the largest (assoc_margin).
-// assoc_dense.cu visits every direction; the cone tree below skips most of a
+// assoc_dense.cu and assoc_scan.cu visit every direction; the cone tree below skips most of a
 // large set; assoc_tc.cu forms the dots on the tensor cores.
 
 // delta = max_j | |r_j|^2 - 1 | in FP64, rounded up to FP32: one 8-CTA cluster

@@ -97,7 +97,7 @@ def normalize(ws: Workspace, objs: torch.Tensor, ideal: torch.Tensor):
     return f, rcp, ext
 
 
-ASSOC_TREE = 0    # cone-tree search (default)
+ASSOC_TREE = 0    # the fastest search for the sizes: cone tree, tensor cores or every direction (default)
 ASSOC_SCAN = 1    # every direction visited
 ASSOC_TENSOR = 2  # dots on the tensor cores, exact FP32 re-score of the candidates
 

@@ -117,10 +117,16 @@ moea_status moea_normalize(moea_workspace* ws, float* d_objs, const float* d_ide
                            int n, float* d_rcp_b, int* d_extreme, void* stream);
 
 /* Association modes; all give the reference's exact argmin. */
-#define MOEA_ASSOC_TREE 0    /* cone tree over the directions, one warp per point, subtrees
-                                pruned by a conservative bound on dot^2 (default); above 5
-                                objectives the tensor-core search of MOEA_ASSOC_TENSOR when
-                                points x directions >= 2^24, else the scan */
+#define MOEA_ASSOC_TREE 0    /* the fastest search for the sizes (default).  Up to 5 objectives a
+                                cone tree over the directions, one warp per point, subtrees
+                                pruned by a conservative bound on dot^2; every direction visited
+                                instead, as MOEA_ASSOC_SCAN, where the tree prunes little (4 and
+                                5 objectives up to 8192 directions, fewer directions than a
+                                sixteenth of the points, directions not of unit length).  Above
+                                5 objectives the tensor-core search of MOEA_ASSOC_TENSOR when
+                                points x directions >= 2^24, else every direction visited.
+                                moea_nsga3_select builds no tree: MOEA_ASSOC_TENSOR from 4
+                                objectives and 2^24 pairs on, else MOEA_ASSOC_SCAN */
 #define MOEA_ASSOC_SCAN 1    /* every direction visited, FP32 re-score of the dot^2 candidates */
 #define MOEA_ASSOC_TENSOR 2  /* precision form: the point x direction dots on the tensor cores
                                 (split TF32 operands, FP32 accumulation), FP32 re-score of every
