@@ -39,17 +39,26 @@ namespace moea {
 namespace {
 
 constexpr int kNcCtas = 16;
+constexpr int kNcSlice = 4096;       // members per CTA
+// Threads per CTA: the sorts alone 512 (100 members 23 us, with 1024 26; the call
+// 45 and 54), the selection by buckets, and so the sorts behind it, 1024.
+constexpr int kNcSortThreads = 512;
 constexpr int kNcThreads = 1024;
-constexpr int kNcWarps = kNcThreads / 32;
-constexpr int kNcSlice = 4096;                        // members per CTA
-constexpr int kNcSteps = kNcSlice / kNcWarps / 32;    // 32-member steps per warp segment
-constexpr int kNcPerThread = kNcSlice / kNcThreads;   // members per thread in the run scan
 
+template <int THREADS>
+struct NcCfg {
+    static constexpr int kWarps = THREADS / 32;
+    static constexpr int kSteps = kNcSlice / kWarps / 32;  // 32-member steps per warp segment
+    static constexpr int kPerThread = kNcSlice / THREADS;  // members per thread in the run scan
+};
+
+template <int THREADS>
 struct NcShared {
+    static constexpr int kWarps = NcCfg<THREADS>::kWarps;
     uint64_t key[2][kNcSlice];
     int val[2][kNcSlice];
     int run[kNcSlice];          // global position where the member's direction run starts
-    int cnt[kNcWarps][256];     // per-warp digit counts, then their prefix over warps
+    int cnt[kWarps][256];     // per-warp digit counts, then their prefix over warps
     int dcount[256];            // this CTA's digit totals (read by the other CTAs)
     int dtotal[256];
     int dbefore[256];
@@ -59,8 +68,8 @@ struct NcShared {
     int plan[8];                // cluster mode: shifts of the digits that differ somewhere
     uint64_t red_or, red_and;   // OR / AND of this CTA's keys (read by the other CTAs)
     uint64_t diff;              // bits that differ in some pair of keys
-    uint64_t wred[kNcWarps][2];
-    int wmax[kNcWarps];
+    uint64_t wred[kWarps][2];
+    int wmax[kWarps];
     int last_head;              // highest run head in this CTA's slice, or -1 (read by the others)
     int carry;
 };
@@ -103,19 +112,21 @@ __device__ __forceinline__ T* nc_map(cg::cluster_group& cluster, T* p, int r)
 }
 
 // One stable pass over key bits [shift, shift + 8): buffer cur -> cur ^ 1.
-template <bool kSolo>
-__device__ void nc_pass(NcShared& sm, cg::cluster_group& cluster, int c, int cur, int len, int S, int shift)
+template <int THREADS, bool kSolo>
+__device__ void nc_pass(NcShared<THREADS>& sm, cg::cluster_group& cluster, int c, int cur, int len, int S, int shift)
 {
+    constexpr int kWarps = NcCfg<THREADS>::kWarps;
+    constexpr int kSteps = NcCfg<THREADS>::kSteps;
     constexpr int kCtas = kSolo ? 1 : kNcCtas;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < kNcWarps * 256; i += kNcThreads) (&sm.cnt[0][0])[i] = 0;
+    for (int i = tid; i < kWarps * 256; i += THREADS) (&sm.cnt[0][0])[i] = 0;
     __syncthreads();
     // per-warp contiguous segments, a multiple of 32 members each
-    const int seg = (((len + kNcWarps - 1) / kNcWarps) + 31) & ~31;
+    const int seg = (((len + kWarps - 1) / kWarps) + 31) & ~31;
     const int b0 = warp * seg, b1 = min(len, b0 + seg);
-    int rk[kNcSteps], dg[kNcSteps];
+    int rk[kSteps], dg[kSteps];
 #pragma unroll
-    for (int j = 0; j < kNcSteps; ++j) {
+    for (int j = 0; j < kSteps; ++j) {
         if (b0 + 32 * j >= b1) break;  // warp-uniform: the segment has ended
         const int e = b0 + 32 * j + lane;
         const bool valid = e < b1;
@@ -136,7 +147,7 @@ __device__ void nc_pass(NcShared& sm, cg::cluster_group& cluster, int c, int cur
     if (tid < 256) {
         int run = 0;
 #pragma unroll
-        for (int w = 0; w < kNcWarps; ++w) {
+        for (int w = 0; w < kWarps; ++w) {
             const int x = sm.cnt[w][tid];
             sm.cnt[w][tid] = run;
             run += x;
@@ -177,7 +188,7 @@ __device__ void nc_pass(NcShared& sm, cg::cluster_group& cluster, int c, int cur
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kNcSteps; ++j) {
+    for (int j = 0; j < kSteps; ++j) {
         if (b0 + 32 * j >= b1) break;
         const int e = b0 + 32 * j + lane;
         if (e < b1) {
@@ -185,7 +196,7 @@ __device__ void nc_pass(NcShared& sm, cg::cluster_group& cluster, int c, int cur
             const int pos = sm.dbase[d] + sm.cnt[warp][d] + rk[j];
             const int dest = pos / S;
             const int slot = pos - dest * S;
-            NcShared* ds = nc_map<kSolo>(cluster, &sm, dest);
+            NcShared<THREADS>* ds = nc_map<kSolo>(cluster, &sm, dest);
             ds->key[cur ^ 1][slot] = sm.key[cur][e];
             ds->val[cur ^ 1][slot] = sm.val[cur][e];
         }
@@ -195,13 +206,14 @@ __device__ void nc_pass(NcShared& sm, cg::cluster_group& cluster, int c, int cur
 
 // Stable sort of the nl keys (with their values) held in buffer cur; returns
 // the buffer that holds the result.
-template <bool kSolo>
-__device__ int nc_sort(NcShared& sm, cg::cluster_group& cluster, int c, int cur, int len, int S)
+template <int THREADS, bool kSolo>
+__device__ int nc_sort(NcShared<THREADS>& sm, cg::cluster_group& cluster, int c, int cur, int len, int S)
 {
+    constexpr int kWarps = NcCfg<THREADS>::kWarps;
     constexpr int kCtas = kSolo ? 1 : kNcCtas;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint64_t o = 0, a = ~0ull;
-    for (int e = tid; e < len; e += kNcThreads) {
+    for (int e = tid; e < len; e += THREADS) {
         o |= sm.key[cur][e];
         a &= sm.key[cur][e];
     }
@@ -216,7 +228,7 @@ __device__ int nc_sort(NcShared& sm, cg::cluster_group& cluster, int c, int cur,
     }
     __syncthreads();
     if (tid == 0) {
-        for (int w = 1; w < kNcWarps; ++w) {
+        for (int w = 1; w < kWarps; ++w) {
             o |= sm.wred[w][0];
             a &= sm.wred[w][1];
         }
@@ -227,7 +239,7 @@ __device__ int nc_sort(NcShared& sm, cg::cluster_group& cluster, int c, int cur,
     if (tid == 0) {
         uint64_t go = 0, ga = ~0ull;
         for (int r = 0; r < kCtas; ++r) {
-            const NcShared* rs = nc_map<kSolo>(cluster, &sm, r);
+            const NcShared<THREADS>* rs = nc_map<kSolo>(cluster, &sm, r);
             go |= rs->red_or;
             ga &= rs->red_and;
         }
@@ -237,7 +249,7 @@ __device__ int nc_sort(NcShared& sm, cg::cluster_group& cluster, int c, int cur,
     const uint64_t diff = sm.diff;
     for (int d = 0; d < 8; ++d) {
         if (((diff >> (8 * d)) & 0xFFu) == 0) continue;  // the same digit in every key
-        nc_pass<kSolo>(sm, cluster, c, cur, len, S, 8 * d);
+        nc_pass<THREADS, kSolo>(sm, cluster, c, cur, len, S, 8 * d);
         cur ^= 1;
     }
     return cur;
@@ -248,12 +260,15 @@ __device__ int nc_sort(NcShared& sm, cg::cluster_group& cluster, int c, int cur,
 // or counted locally before pass 0), scatters, and pushes each member's next
 // digit into the destination's hist[(i + 1) % 3]; hist[(i + 2) % 3], read by
 // pass i - 1 before its barrier, is cleared meanwhile.
-__device__ void nc_pass_push(NcShared& sm, cg::cluster_group& cluster, int c, int cur, int len, int S, int i,
+template <int THREADS>
+__device__ void nc_pass_push(NcShared<THREADS>& sm, cg::cluster_group& cluster, int c, int cur, int len, int S, int i,
                              int shift, int next_shift)
 {
+    constexpr int kWarps = NcCfg<THREADS>::kWarps;
+    constexpr int kSteps = NcCfg<THREADS>::kSteps;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int hb = i % 3, hn = (i + 1) % 3, hz = (i + 2) % 3;
-    for (int k = tid; k < kNcWarps * 256; k += kNcThreads) (&sm.cnt[0][0])[k] = 0;
+    for (int k = tid; k < kWarps * 256; k += THREADS) (&sm.cnt[0][0])[k] = 0;
     if (tid < 256) sm.hist[hz][tid] = 0;
     // every CTA's count of each digit, and of the same digit in lower CTAs
     if (tid < 256) {
@@ -268,11 +283,11 @@ __device__ void nc_pass_push(NcShared& sm, cg::cluster_group& cluster, int c, in
         sm.dbefore[tid] = before;
     }
     __syncthreads();
-    const int seg = (((len + kNcWarps - 1) / kNcWarps) + 31) & ~31;
+    const int seg = (((len + kWarps - 1) / kWarps) + 31) & ~31;
     const int b0 = warp * seg, b1 = min(len, b0 + seg);
-    int rk[kNcSteps], dg[kNcSteps];
+    int rk[kSteps], dg[kSteps];
 #pragma unroll
-    for (int j = 0; j < kNcSteps; ++j) {
+    for (int j = 0; j < kSteps; ++j) {
         if (b0 + 32 * j >= b1) break;  // warp-uniform: the segment has ended
         const int e = b0 + 32 * j + lane;
         const bool valid = e < b1;
@@ -293,7 +308,7 @@ __device__ void nc_pass_push(NcShared& sm, cg::cluster_group& cluster, int c, in
     if (tid < 256) {
         int run = 0;
 #pragma unroll
-        for (int w = 0; w < kNcWarps; ++w) {
+        for (int w = 0; w < kWarps; ++w) {
             const int x = sm.cnt[w][tid];
             sm.cnt[w][tid] = run;
             run += x;
@@ -319,7 +334,7 @@ __device__ void nc_pass_push(NcShared& sm, cg::cluster_group& cluster, int c, in
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kNcSteps; ++j) {
+    for (int j = 0; j < kSteps; ++j) {
         if (b0 + 32 * j >= b1) break;
         const int e = b0 + 32 * j + lane;
         if (e < b1) {
@@ -327,7 +342,7 @@ __device__ void nc_pass_push(NcShared& sm, cg::cluster_group& cluster, int c, in
             const int pos = sm.dbase[d] + sm.cnt[warp][d] + rk[j];
             const int dest = pos / S;
             const int slot = pos - dest * S;
-            NcShared* ds = cluster.map_shared_rank(&sm, dest);
+            NcShared<THREADS>* ds = cluster.map_shared_rank(&sm, dest);
             const uint64_t k = sm.key[cur][e];
             ds->key[cur ^ 1][slot] = k;
             ds->val[cur ^ 1][slot] = sm.val[cur][e];
@@ -338,10 +353,11 @@ __device__ void nc_pass_push(NcShared& sm, cg::cluster_group& cluster, int c, in
 }
 
 // Local counts of the digit at `shift` into hist[h] (warp-aggregated).
-__device__ void nc_count(NcShared& sm, int cur, int len, int shift, int h)
+template <int THREADS>
+__device__ void nc_count(NcShared<THREADS>& sm, int cur, int len, int shift, int h)
 {
     const int tid = threadIdx.x, lane = tid & 31;
-    for (int e0 = tid - lane; e0 < len; e0 += kNcThreads) {
+    for (int e0 = tid - lane; e0 < len; e0 += THREADS) {
         const int e = e0 + lane;
         const int d = (e < len) ? (int)((sm.key[cur][e] >> shift) & 0xFFu) : 0;
         const unsigned peers = match_digit(d, e < len);
@@ -349,8 +365,10 @@ __device__ void nc_count(NcShared& sm, int cur, int len, int shift, int h)
     }
 }
 
-__device__ int nc_sort_cluster(NcShared& sm, cg::cluster_group& cluster, int c, int cur, int len, int S)
+template <int THREADS>
+__device__ int nc_sort_cluster(NcShared<THREADS>& sm, cg::cluster_group& cluster, int c, int cur, int len, int S)
 {
+    constexpr int kWarps = NcCfg<THREADS>::kWarps;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid < 256) {
         sm.hist[0][tid] = 0;
@@ -358,7 +376,7 @@ __device__ int nc_sort_cluster(NcShared& sm, cg::cluster_group& cluster, int c, 
     }
     __syncthreads();
     uint64_t o = 0, a = ~0ull;
-    for (int e = tid; e < len; e += kNcThreads) {
+    for (int e = tid; e < len; e += THREADS) {
         o |= sm.key[cur][e];
         a &= sm.key[cur][e];
     }
@@ -375,7 +393,7 @@ __device__ int nc_sort_cluster(NcShared& sm, cg::cluster_group& cluster, int c, 
     nc_count(sm, cur, len, 0, 0);
     __syncthreads();
     if (tid == 0) {
-        for (int w = 1; w < kNcWarps; ++w) {
+        for (int w = 1; w < kWarps; ++w) {
             o |= sm.wred[w][0];
             a &= sm.wred[w][1];
         }
@@ -386,7 +404,7 @@ __device__ int nc_sort_cluster(NcShared& sm, cg::cluster_group& cluster, int c, 
     if (tid == 0) {
         uint64_t go = 0, ga = ~0ull;
         for (int r = 0; r < kNcCtas; ++r) {
-            const NcShared* rs = cluster.map_shared_rank(&sm, r);
+            const NcShared<THREADS>* rs = cluster.map_shared_rank(&sm, r);
             go |= rs->red_or;
             ga &= rs->red_and;
         }
@@ -418,17 +436,19 @@ __device__ int nc_sort_cluster(NcShared& sm, cg::cluster_group& cluster, int c, 
 
 // run[e] = global position where the direction run of member e starts
 // (heads: a different direction than the member before).
-template <bool kSolo>
-__device__ void nc_runs(NcShared& sm, cg::cluster_group& cluster, int c, int cur, int len, int S, int lo)
+template <int THREADS, bool kSolo>
+__device__ void nc_runs(NcShared<THREADS>& sm, cg::cluster_group& cluster, int c, int cur, int len, int S, int lo)
 {
+    constexpr int kWarps = NcCfg<THREADS>::kWarps;
+    constexpr int kPerThread = NcCfg<THREADS>::kPerThread;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t prev_dir = 0;
     if (c > 0 && len > 0) prev_dir = (uint32_t)(nc_map<kSolo>(cluster, &sm, c - 1)->key[cur][S - 1] >> 32);
-    const int e0 = tid * kNcPerThread;
-    int h[kNcPerThread];
+    const int e0 = tid * kPerThread;
+    int h[kPerThread];
     int m = -1;
 #pragma unroll
-    for (int i = 0; i < kNcPerThread; ++i) {
+    for (int i = 0; i < kPerThread; ++i) {
         const int e = e0 + i;
         int head = -1;
         if (e < len) {
@@ -450,7 +470,7 @@ __device__ void nc_runs(NcShared& sm, cg::cluster_group& cluster, int c, int cur
     __syncthreads();
     if (tid == 0) {
         int best = -1;
-        for (int w = 0; w < kNcWarps; ++w) best = max(best, sm.wmax[w]);
+        for (int w = 0; w < kWarps; ++w) best = max(best, sm.wmax[w]);
         sm.last_head = best;
     }
     int wprefix = -1;
@@ -467,23 +487,23 @@ __device__ void nc_runs(NcShared& sm, cg::cluster_group& cluster, int c, int cur
     __syncthreads();
     const int start = max(sm.carry, base);
 #pragma unroll
-    for (int i = 0; i < kNcPerThread; ++i) {
+    for (int i = 0; i < kPerThread; ++i) {
         const int e = e0 + i;
         if (e < len) sm.run[e] = max(start, h[i]);
     }
     nc_sync<kSolo>(cluster);  // last_head was read everywhere before the CTAs move on
 }
 
-template <bool kSolo>
-__device__ __forceinline__ int nc_sort_any(NcShared& sm, cg::cluster_group& cluster, int c, int cur, int len,
+template <int THREADS, bool kSolo>
+__device__ __forceinline__ int nc_sort_any(NcShared<THREADS>& sm, cg::cluster_group& cluster, int c, int cur, int len,
                                            int S)
 {
-    if constexpr (kSolo) return nc_sort<true>(sm, cluster, c, cur, len, S);
+    if constexpr (kSolo) return nc_sort<THREADS, true>(sm, cluster, c, cur, len, S);
     else return nc_sort_cluster(sm, cluster, c, cur, len, S);
 }
 
-template <bool kSolo>
-__device__ void nc_niching(NcShared& sm, cg::cluster_group& cluster, int c, const int* __restrict__ idx,
+template <int THREADS, bool kSolo>
+__device__ void nc_niching(NcShared<THREADS>& sm, cg::cluster_group& cluster, int c, const int* __restrict__ idx,
                            const float* __restrict__ dist, int np, int nl, int nrem,
                            const int* __restrict__ rho, int H, uint64_t seed,
                            unsigned long long* __restrict__ offset, const int* __restrict__ nds_gidx,
@@ -496,17 +516,17 @@ __device__ void nc_niching(NcShared& sm, cg::cluster_group& cluster, int c, cons
     const int len = max(0, min(S, nl - lo));
 
     // stage 1: (direction, distance bits)
-    for (int e = tid; e < len; e += kNcThreads) {
+    for (int e = tid; e < len; e += THREADS) {
         const int t = lo + e;
         sm.key[0][e] = ((uint64_t)(uint32_t)idx[np + t] << 32) | __float_as_uint(dist[np + t]);
         sm.val[0][e] = t;
     }
     __syncthreads();
-    int cur = nc_sort_any<kSolo>(sm, cluster, c, 0, len, S);
-    nc_runs<kSolo>(sm, cluster, c, cur, len, S, lo);
+    int cur = nc_sort_any<THREADS, kSolo>(sm, cluster, c, 0, len, S);
+    nc_runs<THREADS, kSolo>(sm, cluster, c, cur, len, S, lo);
 
     // stage 2: (direction, 0 for the closest member of an empty niche, else a random odd word)
-    for (int e = tid; e < len; e += kNcThreads) {
+    for (int e = tid; e < len; e += THREADS) {
         const int t = lo + e;
         const uint32_t ref = (uint32_t)(sm.key[cur][e] >> 32);
         const int r_i = (int)ref;
@@ -518,10 +538,10 @@ __device__ void nc_niching(NcShared& sm, cg::cluster_group& cluster, int c, cons
     }
     __syncthreads();
     // the direction runs keep their positions: only their members move
-    cur = nc_sort_any<kSolo>(sm, cluster, c, cur, len, S);
+    cur = nc_sort_any<THREADS, kSolo>(sm, cluster, c, cur, len, S);
 
     // stage 3: (niche count + rank in the niche, random word)
-    for (int e = tid; e < len; e += kNcThreads) {
+    for (int e = tid; e < len; e += THREADS) {
         const int t = lo + e;
         const uint32_t ref = (uint32_t)(sm.key[cur][e] >> 32);
         const int r_i = (int)ref;
@@ -531,22 +551,22 @@ __device__ void nc_niching(NcShared& sm, cg::cluster_group& cluster, int c, cons
         sm.key[cur][e] = ((uint64_t)(uint32_t)(rho_r + rank) << 32) | rnd;
     }
     __syncthreads();
-    cur = nc_sort_any<kSolo>(sm, cluster, c, cur, len, S);
+    cur = nc_sort_any<THREADS, kSolo>(sm, cluster, c, cur, len, S);
 
-    for (int e = tid; e < len; e += kNcThreads) {
+    for (int e = tid; e < len; e += THREADS) {
         const int t = lo + e;
         if (t < nrem) selected[np + t] = nds_gidx[np + sm.val[cur][e]];
     }
     if (c == 0 && tid == 0) *offset = off + 2ull * (unsigned long long)nl;
 }
 
-__global__ void __launch_bounds__(kNcThreads, 1)
+__global__ void __launch_bounds__(kNcSortThreads, 1)
 nich_cluster(const int* __restrict__ idx, const float* __restrict__ dist, const int* __restrict__ sizes,
              const int* __restrict__ rho, int H, uint64_t seed, unsigned long long* __restrict__ offset,
              const int* __restrict__ nds_gidx, int* __restrict__ selected, int* __restrict__ status)
 {
     extern __shared__ __align__(16) unsigned char nc_raw[];
-    NcShared& sm = *reinterpret_cast<NcShared*>(nc_raw);
+    NcShared<kNcSortThreads>& sm = *reinterpret_cast<NcShared<kNcSortThreads>*>(nc_raw);
     cg::cluster_group cluster = cg::this_cluster();
     const int c = (int)cluster.block_rank();
     const int np = sizes[0], nl = sizes[1], nrem = sizes[2];
@@ -559,18 +579,21 @@ nich_cluster(const int* __restrict__ idx, const float* __restrict__ dist, const 
     if (nl <= kNcSlice) {
         // one CTA holds the whole front: CTA barriers instead of cluster
         // barriers; the other CTAs leave at once and share nothing
-        if (c == 0) nc_niching<true>(sm, cluster, 0, idx, dist, np, nl, nrem, rho, H, seed, offset, nds_gidx,
+        if (c == 0) nc_niching<kNcSortThreads, true>(sm, cluster, 0, idx, dist, np, nl, nrem, rho, H, seed, offset, nds_gidx,
                                      selected);
         return;
     }
-    nc_niching<false>(sm, cluster, c, idx, dist, np, nl, nrem, rho, H, seed, offset, nds_gidx, selected);
+    nc_niching<kNcSortThreads, false>(sm, cluster, c, idx, dist, np, nl, nrem, rho, H, seed, offset, nds_gidx, selected);
 }
+
+using NcSortShared = NcShared<kNcSortThreads>;
 
 // Niche selection and the ascending survivor list of one generation: the
 // direction buckets of niche_select.cuh, else the three sorts above.
+constexpr int kNcItems = NcCfg<kNcThreads>::kPerThread;  // last-front members per thread
 union NcSelectShared {
-    NcShared sorts;
-    NicheShared<kNcThreads, kNcPerThread> buckets;
+    NcShared<kNcThreads> sorts;
+    NicheShared<kNcThreads, kNcItems> buckets;
 };
 
 template <class G>
@@ -590,21 +613,21 @@ nich_select(const int* __restrict__ idx, const float* __restrict__ dist, const i
         return;
     }
     const unsigned long long off = *offset;
-    if (niche_buckets<kNcThreads, kNcPerThread>(grp, sm.buckets, S, idx, dist, nds_gidx, np, nl, nrem, H, seed, off, n_mix)) {
+    if (niche_buckets<kNcThreads, kNcItems>(grp, sm.buckets, S, idx, dist, nds_gidx, np, nl, nrem, H, seed, off, n_mix)) {
         if (c == 0 && threadIdx.x == 0) *offset = off + 2ull * (unsigned long long)nl;
     } else {
         cg::cluster_group cluster = cg::this_cluster();
         if (G::kMany && nl > kNcSlice)
-            nc_niching<false>(sm.sorts, cluster, c, idx, dist, np, nl, nrem, S.rho, H, seed, offset, nds_gidx, selected);
+            nc_niching<kNcThreads, false>(sm.sorts, cluster, c, idx, dist, np, nl, nrem, S.rho, H, seed, offset, nds_gidx, selected);
         else if (c == 0)
-            nc_niching<true>(sm.sorts, cluster, 0, idx, dist, np, nl, nrem, S.rho, H, seed, offset, nds_gidx, selected);
+            nc_niching<kNcThreads, true>(sm.sorts, cluster, 0, idx, dist, np, nl, nrem, S.rho, H, seed, offset, nds_gidx, selected);
         grp.sync();  // the selection is complete
         const int take = min(nrem, nl);
         for (int i = c * kNcThreads + (int)threadIdx.x; i < take; i += grp.count() * kNcThreads)
             niche_mark(S.mask, __ldcg(selected + np + i));
         grp.sync();
     }
-    niche_survivors<kNcThreads, kNcPerThread>(grp, sm.buckets, S.mask, n_mix, survivors, N);
+    niche_survivors<kNcThreads, kNcItems>(grp, sm.buckets, S.mask, n_mix, survivors, N);
 }
 
 // One CTA for the merged populations whose last front it can hold and few
@@ -635,9 +658,11 @@ bool configure_niching_cluster()
     int clusters = 0;
     cudaError_t e = cudaFuncSetAttribute(nich_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(nich_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NcShared));
-    cfg.dynamicSmemBytes = sizeof(NcShared);
+        e = cudaFuncSetAttribute(nich_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NcSortShared));
+    cfg.blockDim = dim3(kNcSortThreads);
+    cfg.dynamicSmemBytes = sizeof(NcSortShared);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, (void*)nich_cluster, &cfg);
+    cfg.blockDim = dim3(kNcThreads);
     if (e == cudaSuccess && clusters < 1) return false;
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(nich_select<NicheCluster>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -677,8 +702,8 @@ int launch_niching_cluster(const int* idx, const float* dist, const int* sizes, 
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kNcCtas);
-    cfg.blockDim = dim3(kNcThreads);
-    cfg.dynamicSmemBytes = sizeof(NcShared);
+    cfg.blockDim = dim3(kNcSortThreads);
+    cfg.dynamicSmemBytes = sizeof(NcSortShared);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
